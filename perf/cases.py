@@ -1,0 +1,477 @@
+"""The workloads this engine's speed is measured on.
+
+Each case is one call (or, for the sharder, one build) through the public entry
+points of ``gcgpu`` on device-resident inputs, the way a program that keeps its
+graph on the GPU uses them. ``listed()`` gives the fixed cases, ``draw(rng)`` more
+of the same ranges, ``prepare`` what a program holds before the call, ``run`` one
+call, ``work`` the bytes and operations it cannot do without and ``exact`` its
+answer in 64-bit arithmetic by plain torch.
+
+Inputs are R-MAT graphs (a/b/c/d = 0.57/0.19/0.19/0.05; a vertex count that is no
+power of two folds the ids) and Erdos-Renyi graphs, made on the device from the
+seed.
+"""
+import ctypes
+import math
+import os
+import sys
+
+import numpy as np
+import torch
+
+_PKG = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "graphchi-cpp_b200")
+if _PKG not in sys.path:
+    sys.path.insert(0, _PKG)
+
+TELEPORT, DAMPING = 0.15, 0.85
+MODEL = os.path.join(_PKG, "gcgpu", "warm_start_rmat.npz")
+
+
+def _gcgpu():
+    import gcgpu
+    return gcgpu
+
+
+def listed():
+    return [
+        # PageRank as the reference's app runs it by default: 4 iterations (the initial
+        # one and 3 sweeps) of a small graph; a call of a few kernels, all latency
+        {"name": "pagerank_4iter_rmat16", "kind": "pagerank", "model": "rmat", "n": 1 << 16, "m": 16 << 16,
+         "sweeps": 3, "tol": 0.0},
+        # PageRank to convergence on a small uniform graph that is no power of two
+        {"name": "pagerank_tol_er300k", "kind": "pagerank", "model": "er", "n": 300000, "m": 2400000,
+         "sweeps": 1000, "tol": 1e-8},
+        # PageRank to convergence on the largest graph: the headline solve
+        {"name": "pagerank_tol_rmat24", "kind": "pagerank", "model": "rmat", "n": 1 << 24, "m": 16 << 24,
+         "sweeps": 1000, "tol": 1e-8},
+        # the vertex-API program with the reference's visit order, 4 iterations, bit-exact
+        {"name": "gauss_seidel_rmat20", "kind": "gauss_seidel", "n": 1 << 20, "m": 16 << 20, "sweeps": 3},
+        # the sharder on a small edge list (both CSRs), and on a large one cut into 64
+        # vertex intervals (in-edges only, what PageRank needs)
+        {"name": "build_rmat16", "kind": "build", "n": 1 << 16, "m": 16 << 16, "symmetrise": False,
+         "out_csr": True, "nshards": 1},
+        {"name": "build_rmat22", "kind": "build", "n": 1 << 22, "m": 16 << 22, "symmetrise": False,
+         "out_csr": False, "nshards": 64},
+        # connected components of a large undirected graph
+        {"name": "components_rmat24", "kind": "components", "n": 1 << 24, "m": 16 << 24, "symmetrise": True},
+        # triangle counts (total, per vertex, degree ranking) of an undirected graph
+        {"name": "triangles_rmat20", "kind": "triangles", "n": 1 << 20, "m": 16 << 20},
+        # personalised PageRank of a ragged number of sources at once, to convergence
+        {"name": "ppr100_rmat20", "kind": "ppr", "n": 1 << 20, "m": 16 << 20, "sources": 100, "tol": 1e-8},
+        # many graphs of uneven size (10k-300k vertices, both models) in one launch
+        {"name": "batch64", "kind": "batch", "graphs": 64, "lo": 10000, "hi": 300000, "tol": 1e-8},
+        # learned initial ranks: degree features and the network's inference
+        {"name": "warm_start_rmat22", "kind": "warm_start", "n": 1 << 22, "m": 16 << 22},
+        # the network's training direction: loss gradient over a set of samples
+        {"name": "mlp_gradient_1m", "kind": "mlp_gradient", "samples": 1000000},
+    ]
+
+
+def _log_uniform(rng, lo, hi):
+    return int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))
+
+
+def draw(rng):
+    """A case of the ranges that the listed ones stand for: sizes log-uniform, odd as they fall."""
+    kind = rng.choice(["pagerank", "pagerank", "pagerank", "gauss_seidel", "build", "build", "components",
+                       "triangles", "ppr", "batch", "warm_start", "mlp_gradient"])
+    c = {"kind": kind}
+    if kind == "batch":
+        c["graphs"] = _log_uniform(rng, 2, 64)
+        c["lo"] = 10000
+        c["hi"] = _log_uniform(rng, 20000, 300000)
+        c["tol"] = rng.choice([1e-6, 1e-8])
+        return c
+    if kind == "mlp_gradient":
+        c["samples"] = _log_uniform(rng, 4096, 1000000)
+        return c
+    hi = {"pagerank": 1 << 24, "gauss_seidel": 1 << 20, "build": 1 << 22, "components": 1 << 24,
+          "triangles": 1 << 20, "ppr": 1 << 20, "warm_start": 1 << 22}[kind]
+    n = _log_uniform(rng, 1 << 16 if kind in ("pagerank", "build") else 1 << 14, hi)
+    c["n"] = n
+    c["m"] = int(n * rng.uniform(4.0, 16.0))
+    if kind == "pagerank":
+        c["model"] = rng.choice(["rmat", "rmat", "er"])
+        c["sweeps"], c["tol"] = rng.choice([(3, 0.0), (1000, 1e-6), (1000, 1e-8)])
+    elif kind == "gauss_seidel":
+        c["sweeps"] = rng.choice([1, 3, 5])
+    elif kind == "build":
+        c["symmetrise"] = rng.random() < 0.3
+        if c["symmetrise"]:
+            c["m"] //= 2
+        c["out_csr"] = rng.random() < 0.5
+        c["nshards"] = rng.choice([1, 4, 64])
+    elif kind == "components":
+        c["symmetrise"] = rng.random() < 0.5
+    elif kind == "ppr":
+        c["sources"] = _log_uniform(rng, 2, 100)
+        c["tol"] = rng.choice([1e-6, 1e-8])
+    return c
+
+
+# ---- inputs ------------------------------------------------------------------
+
+def _generator(seed):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(int(seed))
+    return g
+
+
+def _edges(model, n, m, seed):
+    """m seeded edges over n vertices as two int32 device tensors."""
+    gen = _generator(seed)
+    src = torch.empty(m, dtype=torch.int32, device="cuda")
+    dst = torch.empty(m, dtype=torch.int32, device="cuda")
+    if model == "er":
+        src.random_(0, n, generator=gen)
+        dst.random_(0, n, generator=gen)
+        return src, dst
+    a, b, c = 0.57, 0.19, 0.19
+    bits = max(1, (n - 1).bit_length())
+    step = 1 << 25
+    for at in range(0, m, step):
+        k = min(step, m - at)
+        s = torch.zeros(k, dtype=torch.int32, device="cuda")
+        d = torch.zeros(k, dtype=torch.int32, device="cuda")
+        r = torch.empty(k, dtype=torch.float32, device="cuda")
+        for _ in range(bits):
+            r.uniform_(generator=gen)
+            down = r >= a + b
+            right = ((r >= a) & ~down) | (r >= a + b + c)
+            s.mul_(2).add_(down)
+            d.mul_(2).add_(right)
+        if n != 1 << bits:
+            s.remainder_(n)
+            d.remainder_(n)
+        src[at:at + k] = s
+        dst[at:at + k] = d
+    return src, dst
+
+
+def _batch_specs(case, seed):
+    """(model, vertices, edges, seed) of every graph of a batch: sizes by the case, edges by the seed."""
+    rng = np.random.default_rng([case["graphs"], case["lo"], case["hi"]])
+    ns = np.exp(rng.uniform(math.log(case["lo"]), math.log(case["hi"]), case["graphs"])).astype(int)
+    return [("er" if i % 2 == 0 else "rmat", int(n), 8 * int(n), seed * 1000 + i) for i, n in enumerate(ns)]
+
+
+def _model_arrays():
+    z = np.load(MODEL)
+    return z["params"], z["norm"]
+
+
+def _mlp_samples(case, seed):
+    """Samples with the normalisation's mean and spread, and their targets."""
+    _, norm = _model_arrays()
+    norm = torch.from_numpy(norm).cuda()
+    gen = _generator(seed)
+    x = torch.randn(case["samples"], 8, generator=gen, device="cuda") / norm[8:] + norm[:8]
+    t = torch.randn(case["samples"], generator=gen, device="cuda") + 1.0
+    return x.contiguous(), t
+
+
+def _ppr_sources(case, seed):
+    return np.random.default_rng(seed).integers(0, case["n"], case["sources"]).astype(np.uint32)
+
+
+def prepare(case, seed):
+    gcgpu = _gcgpu()
+    kind = case["kind"]
+    if kind == "build":
+        lib = ctypes.CDLL(gcgpu.LIB_PATH)  # the C ABI's copies into device arrays
+        for f in (lib.gcg_graph_csr, lib.gcg_graph_degrees):
+            f.restype = ctypes.c_int
+        n, cap = case["n"], case["m"] * (2 if case["symmetrise"] else 1)
+        src, dst = _edges("rmat", n, case["m"], seed)
+        state = {"case": case, "lib": lib, "src": src, "dst": dst,
+                 "degrees": torch.empty((n, 2), dtype=torch.int32, device="cuda")}
+        for side in ("in", "out") if case["out_csr"] else ("in",):  # room for every edge; repeats leave the end 0
+            state[side + "_rowptr"] = torch.empty(n + 1, dtype=torch.int32, device="cuda")
+            state[side + "_col"] = torch.zeros(cap, dtype=torch.int32, device="cuda")
+        return state
+    if kind == "batch":
+        graphs = []
+        for model, n, m, s in _batch_specs(case, seed):
+            src, dst = _edges(model, n, m, s)
+            graphs.append(gcgpu.Graph.from_edges(src, dst, num_vertices=n, dedup=True, out_csr=False))
+        batch = gcgpu.Batch(graphs)
+        for g in graphs:
+            g.free()
+        return {"case": case, "batch": batch,
+                "out": torch.empty(int(batch.offsets[-1]), dtype=torch.float32, device="cuda")}
+    if kind == "mlp_gradient":
+        x, t = _mlp_samples(case, seed)
+        return {"case": case, "mlp": gcgpu.Mlp.load(MODEL), "x": x, "t": t}
+    n = case["n"]
+    src, dst = _edges(case.get("model", "rmat"), n, case["m"], seed)
+    both = kind == "triangles" or bool(case.get("symmetrise"))
+    graph = gcgpu.Graph.from_edges(src, dst, num_vertices=n, dedup=True, symmetrise=both,
+                                   out_csr=kind == "components" and not both)
+    state = {"case": case, "graph": graph}
+    if kind in ("pagerank", "gauss_seidel", "warm_start"):
+        state["out"] = torch.empty(n, dtype=torch.float32, device="cuda")
+    if kind == "components":
+        state["out"] = torch.empty(n, dtype=torch.int32, device="cuda")
+    if kind == "triangles":
+        state["per_rank"] = torch.empty(n, dtype=torch.int32, device="cuda")
+        state["vertexmap"] = torch.empty(n, dtype=torch.int32, device="cuda")
+    if kind == "ppr":
+        state["sources"] = _ppr_sources(case, seed)
+        state["out"] = torch.empty((n, case["sources"]), dtype=torch.float32, device="cuda")
+    if kind == "warm_start":
+        state["mlp"] = gcgpu.Mlp.load(MODEL)
+    return state
+
+
+def _check(status):
+    if status != 0:
+        raise RuntimeError(_gcgpu().last_error())
+
+
+def _address(tensor):
+    return ctypes.c_void_p(tensor.data_ptr())
+
+
+def run(state):
+    gcgpu = _gcgpu()
+    case = state["case"]
+    kind = case["kind"]
+    if kind == "pagerank":
+        state["graph"].pagerank(max_sweeps=case["sweeps"], tol=case["tol"], teleport=TELEPORT, damping=DAMPING,
+                                out=state["out"])
+        return {"ranks": state["out"]}
+    if kind == "gauss_seidel":
+        state["graph"].pagerank(mode=gcgpu.PR_GS_EXACT, max_sweeps=case["sweeps"], out=state["out"])
+        return {"values": state["out"]}
+    if kind == "build":
+        lib = state["lib"]
+        with gcgpu.Graph.from_edges(state["src"], state["dst"], num_vertices=case["n"], dedup=True,
+                                    symmetrise=case["symmetrise"], nshards=case["nshards"],
+                                    out_csr=case["out_csr"]) as g:
+            for side, which in (("in", gcgpu.CSR_IN), ("out", gcgpu.CSR_OUT)):
+                if side + "_col" in state:
+                    _check(lib.gcg_graph_csr(g.handle, which, _address(state[side + "_rowptr"]),
+                                             _address(state[side + "_col"])))
+            _check(lib.gcg_graph_degrees(g.handle, _address(state["degrees"])))
+            out = {"edges": g.num_edges, "intervals": g.intervals().astype(np.int64)}
+        for name in ("in_rowptr", "in_col", "out_rowptr", "out_col", "degrees"):
+            if name in state:
+                out[name] = state[name]
+        return out
+    if kind == "components":
+        state["graph"].connected_components(out=state["out"])
+        return {"labels": state["out"]}
+    if kind == "triangles":
+        total, per_rank, vertexmap, _ = state["graph"].triangle_count(state["per_rank"], state["vertexmap"])
+        return {"total": total, "per_rank": per_rank, "vertexmap": vertexmap}
+    if kind == "ppr":
+        state["graph"].ppr_batched(state["sources"], max_sweeps=1000, tol=case["tol"], teleport=TELEPORT,
+                                   damping=DAMPING, out=state["out"])
+        return {"ranks": state["out"]}
+    if kind == "batch":
+        state["batch"].pagerank(max_sweeps=1000, tol=case["tol"], teleport=TELEPORT, damping=DAMPING,
+                                out=state["out"])
+        return {"ranks": state["out"]}
+    if kind == "warm_start":
+        state["graph"].warm_start_rank(state["mlp"], teleport=TELEPORT, damping=DAMPING, out=state["out"])
+        return {"ranks": state["out"]}
+    grad, loss = state["mlp"].gradient(state["x"], state["t"])
+    return {"gradient": grad, "loss": np.float32(loss)}
+
+
+# ---- the least a call has to do ------------------------------------------------
+
+def _sweeps(case):
+    """Sweeps of a solve: the fixed count, or what it takes to the tolerance (measured: the
+    rank that R-MAT's vertices without out-edges lose decays slowly, uniform graphs mix fast)."""
+    if not case.get("tol"):
+        return case["sweeps"]
+    slow = case.get("model", "rmat") == "rmat"
+    return (80 if slow else 18) * (1.0 if case["tol"] <= 1e-8 else 0.72)
+
+
+def work(case):
+    """A sweep reads every edge's source once, and the vertex values once, and writes them
+    once: 4 E + 8 V bytes, 2 E operations. Everything else reads its input once and writes
+    its output once."""
+    kind = case["kind"]
+    if kind == "mlp_gradient":
+        return {"bytes": 36.0 * case["samples"], "flops": 6.0 * (8 * 64 + 64 * 64 + 64) * case["samples"]}
+    if kind == "batch":
+        mean = (case["hi"] - case["lo"]) / math.log(case["hi"] / case["lo"])
+        nv = mean * case["graphs"]
+        k = sum(_sweeps({"model": m, "tol": case["tol"]}) for m in ("er", "rmat")) / 2
+        return {"bytes": k * 40.0 * nv, "flops": k * 16.0 * nv}
+    n, m = case["n"], case["m"]
+    if kind in ("pagerank", "gauss_seidel"):
+        k = _sweeps(case)
+        return {"bytes": k * (4.0 * m + 8.0 * n), "flops": k * 2.0 * m}
+    if kind == "ppr":  # a source without out-edges (44 % of them) is done after two sweeps
+        k, live = _sweeps(case), 0.56 * case["sources"]
+        return {"bytes": k * (4.0 * m + 8.0 * n * live), "flops": k * 2.0 * m * live}
+    if kind == "build":
+        e = 2.0 * m if case["symmetrise"] else 1.0 * m
+        return {"bytes": 8.0 * m + (2 if case["out_csr"] else 1) * 4.0 * (e + n) + 8.0 * n, "flops": 0.0}
+    if kind == "components":
+        return {"bytes": 4.0 * m * 2 + 8.0 * n, "flops": 0.0}
+    if kind == "triangles":
+        return {"bytes": 4.0 * m * 2 + 12.0 * n, "flops": 0.0}
+    return {"bytes": 4.0 * m + 12.0 * n, "flops": 2.0 * (8 * 64 + 64 * 64 + 64) * n}  # warm_start
+
+
+# ---- the answers in 64 bits ----------------------------------------------------
+
+def _adjacency(model, n, m, seed):
+    """Simple directed graph of the edges: (in-rowptr, in-col, destination of each edge, in- and out-degree)."""
+    src, dst = _edges(model, n, m, seed)
+    keys = dst.long() * n + src.long()
+    keys = keys[src != dst]
+    del src, dst
+    keys = torch.unique(keys)
+    row, col = keys // n, keys % n
+    del keys
+    indeg = torch.bincount(row, minlength=n)
+    outdeg = torch.bincount(col, minlength=n)
+    rowptr = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    rowptr[1:] = torch.cumsum(indeg, 0)
+    return rowptr, col, row, indeg, outdeg
+
+
+def _gather_matrix(rowptr, col, n):
+    """A with (A x)[v] = sum of x over v's in-neighbours."""
+    ones = torch.ones(col.numel(), dtype=torch.float64, device="cuda")
+    return torch.sparse_csr_tensor(rowptr.int(), col.int(), ones, size=(n, n))
+
+
+def _exact_jacobi(model, n, m, seed, sweeps, tol):
+    rowptr, col, _, _, outdeg = _adjacency(model, n, m, seed)
+    a = _gather_matrix(rowptr, col, n)
+    share = torch.where(outdeg > 0, 1.0 / outdeg.clamp(min=1).double(), 0.0)
+    r = torch.ones(n, dtype=torch.float64, device="cuda")
+    for _ in range(sweeps):
+        new = TELEPORT + DAMPING * (a @ (r * share))
+        res = float((new - r).abs().sum() / new.abs().sum())
+        r = new
+        if tol and res <= tol:
+            break
+    return r
+
+
+def _exact_ppr(case, seed):
+    n, k = case["n"], case["sources"]
+    rowptr, col, _, _, outdeg = _adjacency("rmat", n, case["m"], seed)
+    a = _gather_matrix(rowptr, col, n)
+    share = torch.where(outdeg > 0, 1.0 / outdeg.clamp(min=1).double(), 0.0)[:, None]
+    out = torch.zeros((n, k), dtype=torch.float64, device="cuda")
+    live = torch.arange(k, device="cuda")
+    src = torch.from_numpy(_ppr_sources(case, seed).astype(np.int64)).cuda()
+    r = torch.zeros((n, k), dtype=torch.float64, device="cuda")
+    r[src, live] = 1.0
+    for _ in range(1000):
+        new = DAMPING * (a @ (r * share))
+        new[src, torch.arange(src.numel(), device="cuda")] += TELEPORT
+        res = (new - r).abs().sum(0) / new.abs().sum(0)
+        done = res <= case["tol"]
+        out[:, live[done]] = new[:, done]
+        live, src, r = live[~done], src[~done], new[:, ~done].contiguous()
+        if live.numel() == 0:
+            break
+    out[:, live] = r
+    return out
+
+
+def _exact_gauss_seidel(case, seed):
+    """Sweeps in id order: x = (teleport + damping (L x + U x_old)) / outdeg with L the edges
+    from smaller ids, solved by repeating x -> f(x) until nothing moves."""
+    n = case["n"]
+    rowptr, col, row, _, outdeg = _adjacency("rmat", n, case["m"], seed)
+    lower = col < row
+
+    def part(keep):
+        rp = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+        rp[1:] = torch.cumsum(torch.bincount(row[keep], minlength=n), 0)
+        return _gather_matrix(rp, col[keep], n)
+
+    low, up = part(lower), part(~lower)
+    od = outdeg.clamp(min=1).double()
+    x = torch.where(outdeg > 0, 1.0 / od, TELEPORT)
+    for _ in range(case["sweeps"]):
+        base = TELEPORT + DAMPING * (up @ x)
+        for _ in range(2000):
+            new = (base + DAMPING * (low @ x)) / od
+            moved = float(((new - x).abs() / new).max())
+            x = new
+            if moved <= 1e-15:
+                break
+    return x * od
+
+
+def _bf16(x):
+    return x.float().bfloat16().double()
+
+
+def _network(x):
+    """The shipped network's layers on raw features x: what the gradient needs of them."""
+    params, norm = (torch.from_numpy(v).cuda().double() for v in _model_arrays())
+    w1, b1, w2, b2, w3, b3 = torch.split(params, [512, 64, 4096, 64, 64, 1])
+    w1, w2, w3 = _bf16(w1).view(64, 8), _bf16(w2).view(64, 64), _bf16(w3)
+    xn = _bf16((x.double() - norm[:8]) * norm[8:])
+    a1 = xn @ w1.T + b1
+    h1 = _bf16(a1.clamp(min=0))
+    a2 = h1 @ w2.T + b2
+    h2 = a2.clamp(min=0)
+    return h2 @ w3 + b3, xn, a1, h1, a2, h2, w2, w3
+
+
+def _exact_gradient(case, seed):
+    x, t = _mlp_samples(case, seed)
+    n = x.shape[0]
+    y, xn, a1, h1, a2, h2, w2, w3 = _network(x)
+    err = y - t.double()
+    dy = 2.0 * err / n
+    d2 = dy[:, None] * w3 * (a2 > 0)
+    d1 = (d2 @ w2) * (a1 > 0)
+    grad = torch.cat([(d1.T @ xn).reshape(-1), d1.sum(0), (d2.T @ h1).reshape(-1), d2.sum(0), h2.T @ dy,
+                      dy.sum()[None]])
+    return {"gradient": grad, "loss": (err * err).mean()}
+
+
+def _exact_warm_start(case, seed):
+    n = case["n"]
+    rowptr, col, _, indeg, outdeg = _adjacency("rmat", n, case["m"], seed)
+    a = _gather_matrix(rowptr, col, n)
+    di, do = indeg.double(), outdeg.double()
+    f = torch.zeros((n, 8), dtype=torch.float64, device="cuda")
+    f[:, 0], f[:, 1] = torch.log1p(di), torch.log1p(do)
+    f[:, 2] = (a @ torch.log1p(di)) / di.clamp(min=1)
+    biggest = torch.segment_reduce(di[col], "max", lengths=indeg, initial=0.0)
+    f[:, 3] = torch.log1p(biggest)
+    f[:, 4] = torch.log1p(a @ di)
+    f[:, 5] = torch.where(do > 0, 1.0 / do.clamp(min=1), 0.0)
+    bits = max(1, (n - 1).bit_length())
+    v = torch.arange(n, device="cuda")
+    f[:, 6], f[:, 7] = (v >> (bits - 1)) & 1, (v >> (bits - 2)) & 1
+    y = torch.cat([_network(part)[0] for part in torch.split(f.float(), 1 << 19)])
+    z, d = indeg == 0, outdeg == 0
+    p = TELEPORT * torch.exp(y)
+    num = TELEPORT * (n - (1 - DAMPING) * z.sum() - DAMPING * (z & d).sum())
+    den = (1 - DAMPING) * p[~z].sum() + DAMPING * p[~z & d].sum()
+    return torch.where(z, TELEPORT, p * (num / den))
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind == "pagerank":
+        return {"ranks": _exact_jacobi(case["model"], case["n"], case["m"], seed, case["sweeps"], case["tol"])}
+    if kind == "gauss_seidel":
+        return {"values": _exact_gauss_seidel(case, seed)}
+    if kind == "ppr":
+        return {"ranks": _exact_ppr(case, seed)}
+    if kind == "batch":
+        parts = [_exact_jacobi(model, n, m, s, 1000, case["tol"]) for model, n, m, s in _batch_specs(case, seed)]
+        return {"ranks": torch.cat(parts)}
+    if kind == "warm_start":
+        return {"ranks": _exact_warm_start(case, seed)}
+    if kind == "mlp_gradient":
+        return _exact_gradient(case, seed)
+    return None  # whole numbers
