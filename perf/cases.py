@@ -283,11 +283,11 @@ def run(state):
 
 def _sweeps(case):
     """Sweeps of a solve: the fixed count, or what it takes to the tolerance (measured: the
-    rank that R-MAT's vertices without out-edges lose decays slowly, uniform graphs mix fast)."""
+    rank that vertices without out-edges lose decays slowly, also where they are few)."""
     if not case.get("tol"):
         return case["sweeps"]
     slow = case.get("model", "rmat") == "rmat"
-    return (80 if slow else 18) * (1.0 if case["tol"] <= 1e-8 else 0.72)
+    return (80 if slow else 64) * (1.0 if case["tol"] <= 1e-8 else 0.72)
 
 
 def work(case):
