@@ -41,6 +41,16 @@ bool is_device_ptr(const void *p) {
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+bool is_local_device_ptr(const void *p) {
+    cudaPointerAttributes a;
+    int dev = 0;
+    if (!p || cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == dev;
+}
+
 int copy_in(void *dst_dev, const void *src_user, size_t bytes, cudaStream_t s) {
     if (bytes == 0) return GCG_OK;
     GCG_CUDA(cudaMemcpyAsync(dst_dev, src_user, bytes, cudaMemcpyDefault, s));

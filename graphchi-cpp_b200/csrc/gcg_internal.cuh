@@ -126,6 +126,8 @@ struct tbuf {
 /* Pointer classification: device-resident buffers are used in place; anything
  * else is treated as host memory and staged through a device copy. */
 bool is_device_ptr(const void *p);
+/* memory of the current device, which kernels may write in place */
+bool is_local_device_ptr(const void *p);
 
 /* Copy count elements between a user pointer (host or device) and device memory. */
 int copy_in(void *dst_dev, const void *src_user, size_t bytes, cudaStream_t s);

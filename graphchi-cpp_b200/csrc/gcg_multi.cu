@@ -336,11 +336,8 @@ __global__ void __launch_bounds__(EDGE_THREADS, 1) k_multi_pagerank(MultiArgs m)
                 const uint32_t g = find_graph(s_pref, m.ng, x);
                 sp = a.split[m.gr[g].ss + (x - s_pref[g])];
             }
-            if (valid && (sp.z - sp.y) <= LONG_SPAN) {
-                float s = __ldcg(a.tail_part + sp.y);
-                for (uint32_t c = sp.y + 1; c <= sp.z; ++c) s += __ldcg(a.head_part + c);
-                a.nzsum[sp.x] = s;
-            }
+            if (valid && (sp.z - sp.y) <= LONG_SPAN)
+                a.nzsum[sp.x] = short_row_sum<true>(a.tail_part, a.head_part, sp.y, sp.z);
         }
         if (!grid_sync(m, gen)) return;
 

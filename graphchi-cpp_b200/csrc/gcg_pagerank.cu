@@ -232,11 +232,7 @@ __global__ void __launch_bounds__(256) k_pr_fix(SweepArgs a) {
         const uint32_t k = wb + lane;
         if (k < a.nsplit) {
             const uint4 sp = a.split[k];
-            if (sp.z - sp.y <= LONG_SPAN) {
-                float s = a.tail_part[sp.y];
-                for (uint32_t c = sp.y + 1; c <= sp.z; ++c) s += a.head_part[c];
-                a.nzsum[sp.x] = s;
-            }
+            if (sp.z - sp.y <= LONG_SPAN) a.nzsum[sp.x] = short_row_sum<false>(a.tail_part, a.head_part, sp.y, sp.z);
         }
     }
 }
@@ -788,23 +784,17 @@ static int edge_grid(uint32_t hub_bytes) {
     return num_sms() * per_sm;
 }
 
-static int pagerank_jacobi(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg_pr_stats *stats) {
-    GCG_TRY(ensure_chunk_plan(g));
-    cudaStream_t s = g->stream;
-    const ChunkPlan &pl = *g->cplan;
-    const uint32_t nv = g->nv;
-    const int max_sweeps = p->max_sweeps;
+/* blocks of the vertex kernel */
+static int vertex_grid(const ChunkPlan &pl) { return (int)grid1d(std::max<uint64_t>(pl.nnz, pl.nzero), 16); }
 
-    const uint32_t hub_bytes = std::min(pl.hub, pl.tune_hub) * 4u;
-    const uint64_t run = std::max(1u, pl.tune_run);
-    const int ge = std::max(1, (int)std::min<uint64_t>((uint64_t)edge_grid(hub_bytes), (pl.nchunks + 32 * run - 1) / (32 * run)));
-    const int gv = (int)grid1d(std::max<uint64_t>(pl.nnz, pl.nzero), 16);
-    /* the sweep workspace lives with the graph: allocated on the first call,
-     * reused by later calls (no allocation on the repeated-solve path) */
+/* the sweep workspace lives with the graph: allocated on the first call,
+ * reused by later calls (no allocation on the repeated-solve path) */
+static int ensure_pr_work(gcg_graph *g, int max_sweeps) {
+    const ChunkPlan &pl = *g->cplan;
     PrWork &w = g->cplan->work;
-    /* each contrib buffer starts on a 512-byte boundary (vector loads of the hub,
-     * texture alignment) */
-    const size_t cstride = ((size_t)nv + 127) & ~(size_t)127;
+    const uint32_t nv = g->nv;
+    const int gv = vertex_grid(pl);
+    const size_t cstride = pr_contrib_stride(nv);
     if (!w.r.get()) {
         GCG_TRY(w.r.alloc((size_t)nv));
         GCG_TRY(w.rnz.alloc((size_t)2 * std::max<uint32_t>(pl.nnz, 1)));
@@ -837,6 +827,56 @@ static int pagerank_jacobi(gcg_graph *g, const gcg_pr_params *p, float *out_rank
         }
     }
     if (w.dres.n < 2 * (size_t)max_sweeps + 1) GCG_TRY(w.dres.alloc(2 * (size_t)max_sweeps + 1));
+    return GCG_OK;
+}
+
+int pr_norm_const(gcg_graph *g, const gcg_pr_params *p, double *norm) {
+    if (p->source == GCG_NO_SOURCE) {
+        *norm = (double)g->cplan->nzero * fabs((double)(float)p->teleport);
+    } else { /* only the source keeps a teleport value, if it has no in-edges */
+        uint32_t sdeg = 0;
+        GCG_CUDA(cudaMemcpy(&sdeg, g->indeg.get() + p->source, 4, cudaMemcpyDeviceToHost));
+        *norm = sdeg == 0 ? fabs((double)(float)p->teleport) : 0.0;
+    }
+    return GCG_OK;
+}
+
+int pr_copy_logs(gcg_graph *g, const gcg_pr_params *p, int sweeps, const double *res, const double *delta) {
+    if (sweeps <= 0) return GCG_OK;
+    cudaStream_t s = g->stream;
+    if (p->residuals) GCG_TRY(copy_out(p->residuals, res, (size_t)sweeps * sizeof(double), s));
+    if (p->delta_log) GCG_TRY(copy_out(p->delta_log, delta, (size_t)sweeps * sizeof(double), s));
+    if (p->work_log) { /* every vertex updated and every in-edge gathered per sweep */
+        std::vector<uint64_t> wl(2 * (size_t)sweeps);
+        for (int i = 0; i < sweeps; ++i) {
+            wl[2 * i] = (uint64_t)g->nv * (uint64_t)(i + 1);
+            wl[2 * i + 1] = g->ne * (uint64_t)(i + 1);
+        }
+        GCG_TRY(copy_out(p->work_log, wl.data(), wl.size() * sizeof(uint64_t), s));
+    }
+    if (p->residuals || p->delta_log || p->work_log) GCG_CUDA(cudaStreamSynchronize(s));
+    return GCG_OK;
+}
+
+static int pagerank_jacobi(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg_pr_stats *stats) {
+    GCG_TRY(ensure_chunk_plan(g));
+    GCG_TRY(ensure_pr_work(g, p->max_sweeps));
+    if (resident_applies(g, p)) {
+        bool ran = false;
+        const int st = pagerank_resident(g, p, out_rank, stats, &ran);
+        if (ran || st != GCG_OK) return st;
+    }
+    cudaStream_t s = g->stream;
+    const ChunkPlan &pl = *g->cplan;
+    const uint32_t nv = g->nv;
+    const int max_sweeps = p->max_sweeps;
+
+    const uint32_t hub_bytes = std::min(pl.hub, pl.tune_hub) * 4u;
+    const uint64_t run = std::max(1u, pl.tune_run);
+    const int ge = std::max(1, (int)std::min<uint64_t>((uint64_t)edge_grid(hub_bytes), (pl.nchunks + 32 * run - 1) / (32 * run)));
+    const int gv = vertex_grid(pl);
+    PrWork &w = g->cplan->work;
+    const size_t cstride = pr_contrib_stride(nv);
     dbuf<float> &r = w.r, &c = w.c, &nzsum = w.nzsum, &parts = w.parts, &rnz = w.rnz;
     dbuf<double2> &bres = w.bres;
     dbuf<uint32_t> &ctl = w.ctl; /* ticket, done, sweeps_done */
@@ -896,15 +936,9 @@ static int pagerank_jacobi(gcg_graph *g, const gcg_pr_params *p, float *out_rank
     a.teleport = p->teleport;
     a.damping = p->damping;
     a.tol = p->tol;
-    /* |r'| of the constant vertices, added to the norm once they are no longer visited */
     a.source = p->source;
-    if (p->source == GCG_NO_SOURCE) {
-        a.norm_const = (double)pl.nzero * fabs((double)(float)p->teleport);
-    } else { /* only the source keeps a teleport value, if it has no in-edges */
-        uint32_t sdeg = 0;
-        GCG_CUDA(cudaMemcpy(&sdeg, g->indeg.get() + p->source, 4, cudaMemcpyDeviceToHost));
-        a.norm_const = sdeg == 0 ? fabs((double)(float)p->teleport) : 0.0;
-    }
+    /* |r'| of the constant vertices, added to the norm once they are no longer visited */
+    GCG_TRY(pr_norm_const(g, p, &a.norm_const));
     /* + a block per FIX_WARPS long rows */
     const int fg = (int)grid1d(std::max<uint32_t>(pl.nsplit, 1), 32) + (int)((pl.nlong + FIX_WARPS - 1) / FIX_WARPS);
 
@@ -1050,18 +1084,7 @@ static int pagerank_jacobi(gcg_graph *g, const gcg_pr_params *p, float *out_rank
     }
     double last_res = 0.0;
     GCG_CUDA(cudaMemcpy(&last_res, a.last_res, sizeof(double), cudaMemcpyDeviceToHost));
-    if (p->residuals && sweeps > 0) GCG_TRY(copy_out(p->residuals, dres.get(), (size_t)sweeps * sizeof(double), s));
-    if (p->delta_log && sweeps > 0)
-        GCG_TRY(copy_out(p->delta_log, dres.get() + max_sweeps + 1, (size_t)sweeps * sizeof(double), s));
-    if (p->work_log && sweeps > 0) { /* every vertex updated and every in-edge gathered per sweep */
-        std::vector<uint64_t> wl(2 * (size_t)sweeps);
-        for (int i = 0; i < sweeps; ++i) {
-            wl[2 * i] = (uint64_t)nv * (uint64_t)(i + 1);
-            wl[2 * i + 1] = g->ne * (uint64_t)(i + 1);
-        }
-        GCG_TRY(copy_out(p->work_log, wl.data(), wl.size() * sizeof(uint64_t), s));
-        GCG_CUDA(cudaStreamSynchronize(s));
-    }
+    GCG_TRY(pr_copy_logs(g, p, sweeps, dres.get(), dres.get() + max_sweeps + 1));
     if (sweeps > 0) {
         const float t = (float)p->teleport; /* teleport + damping * 0 */
         k_pr_scatter<<<grid1d(nv, 8), 256, 0, s>>>(pl.nnz, pl.nzero, pl.nz_rows.get(), pl.zero_rows.get(),
@@ -1113,6 +1136,7 @@ int gcg_pagerank_set_config(gcg_graph *g, uint32_t hub_entries, uint32_t chunk_r
     GCG_TRY(ensure_chunk_plan(g));
     g->cplan->tune_hub = hub_entries;
     g->cplan->tune_run = chunk_run;
+    g->cplan->configured = true;
     return GCG_OK;
 }
 
@@ -1121,6 +1145,7 @@ int gcg_pagerank_set_tiers(gcg_graph *g, uint32_t tiers) {
     if (tiers < 1 || tiers > (uint32_t)MAX_TIERS) return fail(GCG_ERR_INVALID, "gcg_pagerank_set_tiers: tiers must be 1..4");
     GCG_TRY(ensure_chunk_plan(g));
     g->cplan->tune_tiers = tiers;
+    g->cplan->configured = true;
     return GCG_OK;
 }
 
@@ -1144,6 +1169,7 @@ int gcg_pagerank_autotune(gcg_graph *g, int sweeps, uint32_t *hub_entries, uint3
     if (sweeps < 1) return fail(GCG_ERR_INVALID, "gcg_pagerank_autotune: sweeps must be >= 1");
     GCG_TRY(ensure_chunk_plan(g));
     ChunkPlan &pl = *g->cplan;
+    pl.configured = true;
     std::vector<uint32_t> hubs;
     for (uint32_t h : {0u, 16384u, 32768u, HUB_DEFAULT, HUB_MAX})
         if (h <= pl.hub && std::find(hubs.begin(), hubs.end(), h) == hubs.end()) hubs.push_back(h);

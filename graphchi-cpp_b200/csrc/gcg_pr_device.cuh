@@ -284,13 +284,31 @@ constexpr uint32_t HUB_MAX = 49152; /* 192 KB of shared memory */
 constexpr uint32_t HUB_DEFAULT = 41724;
 constexpr uint32_t RUN_DEFAULT = 1; /* with texture gathers, 0.4 % faster than runs of 2 */
 
+/* One CTA's part of the one-launch solve: chunks [c0, c1), the rows that begin in
+ * them [r0, r1) and their entries of the split list [s0, s1); cross: the last row
+ * runs on into the chunks of CTAs up to blast. */
+struct ResRange {
+    uint32_t c0, c1, r0, r1, s0, s1, cross, blast;
+};
+/* what that solve reports, in pinned host memory */
+struct ResStatus {
+    int sweeps, done, err, reserved;
+    double residual;
+};
+
 /* Sweep workspace of one graph, reused across calls. */
 struct PrWork {
     dbuf<float> r, c, nzsum, parts, rnz;
     dbuf<double2> bres;
     dbuf<uint32_t> ctl;
     dbuf<double> dres;
-    int *h_flags = nullptr; /* pinned: done flags copied back per chunk of sweeps */
+    int *h_flags = nullptr; /* pinned: done flags copied back per chunk of sweeps, or the ResStatus */
+    /* the one-launch solve (gcg_pr_resident.cu), set up on its first use */
+    uint32_t res_ctas = 0, res_hub = 0;
+    dbuf<ResRange> res_rg;
+    dbuf<uint32_t> res_ctl; /* barrier count, error flag, a flag per CTA */
+    dbuf<double2> res_bres;
+    cudaEvent_t ev[2] = {nullptr, nullptr};
     /* texture objects over the two contribution buffers (0: not available, the
      * edge kernel then gathers with plain loads) */
     unsigned long long tex[2] = {0, 0};
@@ -298,6 +316,8 @@ struct PrWork {
         if (h_flags) host_free(h_flags);
         for (unsigned long long t : tex)
             if (t) cudaDestroyTextureObject((cudaTextureObject_t)t);
+        for (cudaEvent_t e : ev)
+            if (e) cudaEventDestroy(e);
     }
 };
 
@@ -312,24 +332,50 @@ constexpr uint32_t LONG_SPAN = 8;
 constexpr int LONG_GROUPS = 8;
 
 template <bool COHERENT>
-__device__ __forceinline__ float long_row_group(const float *head_part, uint32_t cs, uint32_t ce, int grp,
-                                                uint32_t lane) {
-    float s = 0.0f;
-    for (uint32_t c = cs + 1 + 32u * (uint32_t)grp + lane; c <= ce; c += 32u * LONG_GROUPS)
-        s += COHERENT ? __ldcg(head_part + c) : head_part[c];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    return s;
+__device__ __forceinline__ float ld_part(const float *p) {
+    return COHERENT ? __ldcg(p) : *p;
 }
 
-/* the whole long-row sum by one warp (every lane returns it) */
+/* the whole long-row sum by one warp (every lane returns it). Each lane runs its
+ * chains of all groups side by side, so LONG_GROUPS loads are in flight; the
+ * chains, trees and the order of the groups are those defined above. */
 template <bool COHERENT>
 __device__ __forceinline__ float long_row_sum_warp(const float *head_part, uint32_t cs, uint32_t ce,
                                                    uint32_t lane) {
+    float s[LONG_GROUPS];
+#pragma unroll
+    for (int g = 0; g < LONG_GROUPS; ++g) s[g] = 0.0f;
+    for (uint64_t c0 = (uint64_t)cs + 1 + lane; c0 <= ce; c0 += 32u * LONG_GROUPS) {
+        float v[LONG_GROUPS];
+#pragma unroll
+        for (int g = 0; g < LONG_GROUPS; ++g) v[g] = c0 + 32u * g <= ce ? ld_part<COHERENT>(head_part + c0 + 32u * g) : 0.0f;
+#pragma unroll
+        for (int g = 0; g < LONG_GROUPS; ++g)
+            if (c0 + 32u * g <= ce) s[g] += v[g];
+    }
     float t = 0.0f;
-#pragma unroll 1
-    for (int grp = 0; grp < LONG_GROUPS; ++grp) t += long_row_group<COHERENT>(head_part, cs, ce, grp, lane);
+#pragma unroll
+    for (int g = 0; g < LONG_GROUPS; ++g) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[g] += __shfl_xor_sync(0xFFFFFFFFu, s[g], o);
+        t += s[g];
+    }
     return t;
+}
+
+/* a row of at most LONG_SPAN chunks after its first: tail part, then the head
+ * parts in chunk order; all parts are loaded before the first is added */
+template <bool COHERENT>
+__device__ __forceinline__ float short_row_sum(const float *tail_part, const float *head_part, uint32_t cs,
+                                               uint32_t ce) {
+    float v[LONG_SPAN];
+    float s = ld_part<COHERENT>(tail_part + cs);
+#pragma unroll
+    for (uint32_t k = 0; k < LONG_SPAN; ++k) v[k] = cs + 1 + k <= ce ? ld_part<COHERENT>(head_part + cs + 1 + k) : 0.0f;
+#pragma unroll
+    for (uint32_t k = 0; k < LONG_SPAN; ++k)
+        if (cs + 1 + k <= ce) s += v[k];
+    return s;
 }
 
 /* Source tiers of the edge phase. The sources (relabelled by out-degree) are cut
@@ -378,6 +424,7 @@ struct ChunkPlan {
     /* launch configuration of the edge kernel (gcg_pagerank_autotune):
      * shared-memory hub entries (capped at hub) and chunks per warp run */
     uint32_t tune_hub = HUB_DEFAULT, tune_run = RUN_DEFAULT;
+    bool configured = false; /* set by hand or by the autotuner: the kernels it configures run */
     /* sources relabelled within each interval (each interval keeps its id range) */
     bool per_interval = false;
 };
@@ -387,6 +434,21 @@ int ensure_chunk_plan(gcg_graph *g);
 /* builds (or keeps) the plan's source tiers for ntiers tiers of width ids */
 int ensure_tier_plan(gcg_graph *g, int ntiers, uint32_t width);
 int pr_init_state(gcg_graph *g, float init, const float *init_dev, float *r, float *c, float *rnz);
+
+/* each of the two contribution buffers starts on a 512-byte boundary (vector
+ * loads of the hub, texture alignment) */
+inline size_t pr_contrib_stride(uint32_t nv) { return ((size_t)nv + 127) & ~(size_t)127; }
+/* |r'| of the vertices without in-edges, which later sweeps do not visit */
+int pr_norm_const(gcg_graph *g, const gcg_pr_params *p, double *norm);
+/* the caller's residual, delta and work logs of a finished solve */
+int pr_copy_logs(gcg_graph *g, const gcg_pr_params *p, int sweeps, const double *res, const double *delta);
+
+/* the whole solve in one cooperative launch (gcg_pr_resident.cu); *ran = false
+ * with GCG_OK when this device cannot hold it */
+constexpr uint64_t RESIDENT_MAX_EDGES = 1ull << 25;
+constexpr uint32_t RESIDENT_MAX_VERTICES = 1u << 22;
+bool resident_applies(const gcg_graph *g, const gcg_pr_params *p);
+int pagerank_resident(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg_pr_stats *stats, bool *ran);
 
 /* separate round-to-nearest multiply and add (no FMA contraction), as the
  * reference computes (float)(teleport + damping * (double)sum) */
