@@ -252,23 +252,20 @@ __global__ void __launch_bounds__(EDGE_THREADS, 1) k_multi_pagerank(MultiArgs m)
                         cur = g;
                     }
                     const uint32_t cs0 = s_cs[g] - s_pref[g]; /* chunk = cs0 + position */
-                    uint32_t col[EPL], flags = 0, nvalid = 0, base = 0;
+                    uint32_t col[EPL], meta = 0, base = 0;
                     uint32_t pos = x + warp;
-                    if (pos < send) load_chunk(a, cs0 + pos, lane, pol_stream, col, flags, nvalid, base, a.ne);
+                    if (pos < send) load_chunk(a, cs0 + pos, lane, pol_stream, col, meta, base);
                     while (pos < send) {
                         float val[EPL];
 #pragma unroll
                         for (int j = 0; j < EPL; ++j) {
                             const uint32_t d = col[j] - hb;
-                            float v = 0.0f;
-                            if ((uint32_t)j < nvalid)
-                                v = d < hn ? s_hub[d] : ld_cg_keep_f32(a.c_old + col[j], pol_keep);
-                            val[j] = v;
+                            val[j] = d < hn ? s_hub[d] : ld_cg_keep_f32(a.c_old + col[j], pol_keep);
                         }
-                        const uint32_t cch = cs0 + pos, cf = flags, cn = nvalid, cb = base;
+                        const uint32_t cch = cs0 + pos, cm = meta, cb = base;
                         pos += EDGE_THREADS / 32;
-                        if (pos < send) load_chunk(a, cs0 + pos, lane, pol_stream, col, flags, nvalid, base, a.ne);
-                        reduce_chunk(a, cch, lane, val, cf, cn, cb, a.ne);
+                        if (pos < send) load_chunk(a, cs0 + pos, lane, pol_stream, col, meta, base);
+                        reduce_chunk(a, cch, lane, val, cm, cb, a.ne);
                     }
                     x = send;
                 }
@@ -296,21 +293,21 @@ __global__ void __launch_bounds__(EDGE_THREADS, 1) k_multi_pagerank(MultiArgs m)
             /* A graph's last chunk may end in filler edges: they form the row of
              * the graph's padding vertex (its own head, never read), so chunks
              * are reduced up to the union's end like the single-graph kernel's */
-            uint32_t col[EPL], flags = 0, nvalid = 0, base = 0, ch = 0;
+            uint32_t col[EPL], meta = 0, base = 0, ch = 0;
             auto load_item = [&](uint32_t it) {
                 const uint32_t g = find_graph(s_pref, m.ng, it);
                 ch = s_cs[g] + (it - s_pref[g]);
-                load_chunk(a, ch, lane, pol_stream, col, flags, nvalid, base, a.ne);
+                load_chunk(a, ch, lane, pol_stream, col, meta, base);
             };
             if (item < item_end) load_item(item);
             while (item < item_end) {
                 float val[EPL];
-                gather_chunk<true>(a, col, nvalid, s_hub, pol_keep, val);
-                const uint32_t cch = ch, cf = flags, cn = nvalid, cb = base;
+                gather_chunk<true>(a, col, s_hub, pol_keep, val);
+                const uint32_t cch = ch, cm = meta, cb = base;
                 ++item;
                 if (item >= item_end) next_run(item, item_end);
                 if (item < item_end) load_item(item);
-                reduce_chunk(a, cch, lane, val, cf, cn, cb, a.ne);
+                reduce_chunk(a, cch, lane, val, cm, cb, a.ne);
             }
         }
         if (!grid_sync(m, gen)) return;
@@ -802,7 +799,7 @@ static int batch_pagerank(gcg_batch *b, const gcg_pr_params *p, float *out, int3
     memset(&m, 0, sizeof(m));
     a.col = pl.col_r.get();
     a.outdeg = u->outdeg.get();
-    a.heads = (const uint8_t *)pl.head_bits.get();
+    a.meta = pl.lane_meta.get();
     a.chunk_nz = pl.chunk_nz.get();
     a.nz_rows = pl.nz_rows.get();
     a.zero_rows = pl.zero_rows.get();

@@ -11,8 +11,7 @@
  *                two 128-bit column loads per lane (streamed: no L1 allocation,
  *                L2 evict-first), eight independent gathers of contrib[src]
  *                (L2 evict-last, so the contrib vector stays resident while the
- *                columns stream past), row starts read from a 1-bit-per-edge
- *                head bitmap, in-lane segment sums, and a warp segmented scan
+ *                columns stream past), row starts read from a word per lane, in-lane segment sums, and a warp segmented scan
  *                (shuffles) to join rows across lanes. Rows inside the chunk get
  *                their sum written; a row crossing chunk boundaries leaves one
  *                partial per chunk.
@@ -79,6 +78,27 @@ __global__ void k_head_bits(const uint32_t *__restrict__ nz_start, uint32_t nnz,
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
         uint32_t p = nz_start[i];
         atomicOr(bits + (p >> 5), 1u << (p & 31u));
+    }
+}
+
+/* the lanes' words of every chunk from the row-start bits: one warp per chunk */
+__global__ void k_lane_meta(const uint8_t *__restrict__ heads, uint64_t ne, uint32_t nchunks,
+                            uint16_t *__restrict__ meta) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t w0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t c = w0; c < nchunks; c += nw) {
+        const uint32_t f = heads[c * (CH / 8) + lane];
+        uint32_t incl = (uint32_t)__popc(f);
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            if (lane >= (uint32_t)d) incl += y;
+        }
+        uint32_t high = incl - (uint32_t)__popc(f);
+        if (lane == 0) /* the bits cover a spare word past the last chunk */
+            high = (c + 1) * CH >= ne || (heads[(c + 1) * (CH / 8)] & 1u) ? 1u : 0u;
+        meta[meta_slot(c, lane)] = (uint16_t)(f | (high << 8));
     }
 }
 
@@ -158,12 +178,12 @@ __global__ void __launch_bounds__(EDGE_THREADS, 1) k_pr_edges(SweepArgs a) {
     for (uint32_t i = hub4 + threadIdx.x; i < a.hub; i += blockDim.x) s_hub[i] = __ldcg(a.c_old + i);
 
     /* Warp w takes runs of a.run consecutive chunks: runs w, w + nwarps, ...
-     * Software pipeline: while a chunk's gathers are in flight, the next chunk's
-     * columns, head flags and row base are already being loaded. */
+     * Software pipeline: the next chunk's columns, row starts and row base are
+     * loaded before a chunk's gathers are issued. */
     const uint64_t R = a.run, nch = a.nchunks;
     uint64_t q = gwarp, ch = q * R, end = ch + R < nch ? ch + R : nch;
-    uint32_t col[EPL], flags = 0, nvalid = 0, base = 0;
-    if (ch < end) load_chunk(a, (uint32_t)ch, lane, pol_stream, col, flags, nvalid, base, a.ne);
+    uint32_t col[EPL], meta = 0, base = 0;
+    if (ch < end) load_chunk(a, (uint32_t)ch, lane, pol_stream, col, meta, base);
     if (hub4) { /* bounded wait for the hub copy */
         bool ok = false;
         for (long long spin = 0; !ok && spin < MBAR_SPIN; ++spin) ok = mbar_try_wait(&s_bar, 0u);
@@ -178,26 +198,38 @@ __global__ void __launch_bounds__(EDGE_THREADS, 1) k_pr_edges(SweepArgs a) {
         return;
     }
     while (ch < end) {
-        float val[EPL];
-        if (TEX) {
+        const uint32_t cur = (uint32_t)ch, cur_meta = meta, cur_base = base;
+        uint32_t cc[EPL];
 #pragma unroll
-            for (int j = 0; j < EPL; ++j) {
-                const uint32_t x = col[j];
-                float v = 0.0f;
-                if ((uint32_t)j < nvalid) v = x < a.hub ? s_hub[x] : tex1Dfetch<float>(a.tex_old, (int)x);
-                val[j] = v;
-            }
-        } else {
-            gather_chunk(a, col, nvalid, s_hub, pol_keep, val);
-        }
-        const uint32_t cur = (uint32_t)ch, cur_flags = flags, cur_nvalid = nvalid, cur_base = base;
+        for (int j = 0; j < EPL; ++j) cc[j] = col[j];
         if (++ch >= end) {
             q += nwarps;
             ch = q * R;
             end = ch + R < nch ? ch + R : nch;
         }
-        if (ch < end) load_chunk(a, (uint32_t)ch, lane, pol_stream, col, flags, nvalid, base, a.ne);
-        reduce_chunk(a, cur, lane, val, cur_flags, cur_nvalid, cur_base, a.ne);
+        /* on its way before the gathers: behind them it would wait for their queue */
+        if (ch < end) load_chunk(a, (uint32_t)ch, lane, pol_stream, col, meta, base);
+        float val[EPL];
+        if (TEX) {
+            /* Each edge is a branch of its own (past the end of the edges nothing is
+             * gathered), so a warp's fetches go out one by one between its shared-memory
+             * reads. As one predicated burst of eight they fill the texture queue, warps
+             * stall on it (7.3 of 16.7 stall cycles per issue) and the L1's requests to L2
+             * fall from 84 to 76 % of their rate: 668 instead of 621 us at R-MAT scale 24,
+             * 140 instead of 127 us at scale 22. */
+            const uint64_t e = (uint64_t)cur * CH + (uint64_t)EPL * lane;
+            const uint32_t nvalid = e < a.ne ? (uint32_t)((a.ne - e) < EPL ? (a.ne - e) : EPL) : 0u;
+#pragma unroll
+            for (int j = 0; j < EPL; ++j) {
+                const uint32_t x = cc[j];
+                float v = 0.0f;
+                if ((uint32_t)j < nvalid) v = x < a.hub ? s_hub[x] : tex1Dfetch<float>(a.tex_old, (int)x);
+                val[j] = v;
+            }
+        } else {
+            gather_chunk(a, cc, s_hub, pol_keep, val);
+        }
+        reduce_chunk(a, cur, lane, val, cur_meta, cur_base, a.ne);
     }
 }
 
@@ -548,17 +580,19 @@ int pr_init_state(gcg_graph *g, float init, const float *init_dev, float *r, flo
 }
 
 /* Row structure of an edge array grouped by row (nrows non-empty rows starting
- * at edge positions nz_start[], ne edges): the 1-bit-per-edge row-start bitmap,
+ * at edge positions nz_start[], ne edges): each lane's row starts (lane_meta),
  * each 256-edge chunk's starting row, the rows crossing chunk boundaries and,
  * among them, those spanning more than LONG_SPAN chunks. */
 static int build_segments(const uint32_t *nz_start, uint32_t nrows, uint64_t ne, cudaStream_t s, uint32_t &nchunks,
-                          dbuf<uint32_t> &head_bits, dbuf<uint32_t> &chunk_nz, dbuf<uint4> &split,
+                          dbuf<uint16_t> &lane_meta, dbuf<uint32_t> &chunk_nz, dbuf<uint4> &split,
                           dbuf<uint32_t> &long_split, uint32_t &nsplit, uint32_t &nlong) {
     nchunks = (uint32_t)((ne + CH - 1) / CH);
     nsplit = nlong = 0;
     /* head bitmap covers whole chunks plus one spare word (read of the next chunk's first bit) */
     const uint64_t words = ((uint64_t)nchunks * CH) / 32 + 8;
-    GCG_TRY(head_bits.alloc(words));
+    tbuf<uint32_t> head_bits;
+    GCG_TRY(head_bits.alloc(words, s));
+    GCG_TRY(lane_meta.alloc(std::max<uint64_t>((uint64_t)nchunks * 32, 1)));
     GCG_TRY(chunk_nz.alloc(std::max<uint32_t>(nchunks, 1)));
     GCG_CUDA(cudaMemsetAsync(head_bits.get(), 0, words * 4, s));
     if (!nrows) return split.alloc(1);
@@ -567,6 +601,8 @@ static int build_segments(const uint32_t *nz_start, uint32_t nrows, uint64_t ne,
     GCG_TRY(pos.alloc(nrows, s));
     GCG_TRY(total.alloc(1, s));
     k_head_bits<<<grid1d(nrows), 256, 0, s>>>(nz_start, nrows, head_bits.get());
+    k_lane_meta<<<grid1d((uint64_t)nchunks * 32, 32), 256, 0, s>>>((const uint8_t *)head_bits.get(), ne, nchunks,
+                                                                  lane_meta.get());
     k_chunk_nz<<<grid1d(nchunks), 256, 0, s>>>(nz_start, nrows, nchunks, chunk_nz.get());
     k_split_flags<<<grid1d(nrows), 256, 0, s>>>(nz_start, nrows, ne, flags.get());
     GCG_TRY(scan_u32(flags.get(), pos.get(), nrows, total.get(), s));
@@ -665,7 +701,7 @@ int ensure_chunk_plan(gcg_graph *g) {
     if (p->nzero)
         k_gather_u32<<<grid1d(p->nzero), 256, 0, s>>>(p->nzero, p->zero_rows.get(), p->newid.get(),
                                                      p->zero_cidx.get());
-    if ((st = build_segments(p->nz_start.get(), nnz, ne, s, p->nchunks, p->head_bits, p->chunk_nz, p->split,
+    if ((st = build_segments(p->nz_start.get(), nnz, ne, s, p->nchunks, p->lane_meta, p->chunk_nz, p->split,
                              p->long_split, p->nsplit, p->nlong)))
         return bail(st);
     if (p->nchunks)
@@ -725,7 +761,7 @@ int ensure_tier_plan(gcg_graph *g, int ntiers, uint32_t width) {
                                                    tp.idx.get() + (size_t)k * nnz, start.get());
         }
         t.nrows = nrows;
-        GCG_TRY(build_segments(start.get(), nrows, tne, s, t.nchunks, t.head_bits, t.chunk_nz, t.split, t.long_split,
+        GCG_TRY(build_segments(start.get(), nrows, tne, s, t.nchunks, t.lane_meta, t.chunk_nz, t.split, t.long_split,
                                t.nsplit, t.nlong));
         const uint64_t slots = std::max<uint64_t>((uint64_t)t.nchunks * CH, CH);
         GCG_TRY(t.col.alloc(slots));
@@ -908,7 +944,7 @@ static int pagerank_jacobi(gcg_graph *g, const gcg_pr_params *p, float *out_rank
     a.nz_cidx = pl.nz_cidx.get();
     a.zero_cidx = pl.zero_cidx.get();
     a.outdeg = g->outdeg.get();
-    a.heads = (const uint8_t *)pl.head_bits.get();
+    a.meta = pl.lane_meta.get();
     a.chunk_nz = pl.chunk_nz.get();
     a.nz_rows = pl.nz_rows.get();
     a.zero_rows = pl.zero_rows.get();
@@ -959,7 +995,7 @@ static int pagerank_jacobi(gcg_graph *g, const gcg_pr_params *p, float *out_rank
             SweepArgs &b = at[k];
             b = a;
             b.col = t.col.get();
-            b.heads = (const uint8_t *)t.head_bits.get();
+            b.meta = t.lane_meta.get();
             b.chunk_nz = t.chunk_nz.get();
             b.split = t.split.get();
             b.long_split = t.long_split.get();

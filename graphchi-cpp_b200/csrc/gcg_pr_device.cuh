@@ -74,7 +74,7 @@ constexpr long long MBAR_SPIN = 1ll << 22;
 struct SweepArgs {
     /* graph / plan */
     const uint32_t *col, *outdeg;
-    const uint8_t *heads;
+    const uint16_t *meta; /* row starts, a 16-bit word per lane of a chunk (lane_meta) */
     const uint32_t *chunk_nz, *nz_rows, *zero_rows;
     const uint4 *split;
     const uint32_t *long_split; /* indices into split of the rows spanning more than LONG_SPAN chunks */
@@ -120,24 +120,24 @@ __host__ __device__ __forceinline__ uint64_t chunk_slot(uint64_t e) {
     return (e & ~(uint64_t)(CH - 1)) + (j < 4 ? 4u * l + j : 128u + 4u * l + (j - 4u));
 }
 
-/* columns (streamed), head flags and starting row index of one chunk; ne is
- * the end of the edge range being swept (positions at or beyond it are masked) */
+/* Row starts of a chunk, one 16-bit word per lane: bits 0-7 flag the lane's edges
+ * that begin a row, bits 8-15 count the row starts of the lanes before it (at most
+ * 248; counted once when the plan is built, not by a warp scan per sweep). Lane 0
+ * counts none: its bit 8 says instead that the chunk's last row ends with the chunk.
+ * Words past the last edge hold 0. */
+__host__ __device__ __forceinline__ uint64_t meta_slot(uint64_t chunk, uint32_t lane) { return chunk * 32u + lane; }
+
+/* columns (streamed; slots past the last edge hold 0), row starts and starting row
+ * index of one chunk */
 template <typename A>
 __device__ __forceinline__ void load_chunk(const A &a, uint32_t ch, uint32_t lane, uint64_t pol, uint32_t (&col)[EPL],
-                                           uint32_t &flags, uint32_t &nvalid, uint32_t &base, uint64_t ne) {
+                                           uint32_t &meta, uint32_t &base) {
     const uint64_t c0 = (uint64_t)ch * CH;
-    const uint64_t e = c0 + (uint64_t)EPL * lane;
-    nvalid = e < ne ? (uint32_t)((ne - e) < EPL ? (ne - e) : EPL) : 0u;
     const uint4 x = ld_stream_v4(a.col + c0 + 4u * lane, pol);
     const uint4 y = ld_stream_v4(a.col + c0 + 128u + 4u * lane, pol);
     col[0] = x.x; col[1] = x.y; col[2] = x.z; col[3] = x.w;
     col[4] = y.x; col[5] = y.y; col[6] = y.z; col[7] = y.w;
-    if (nvalid < EPL) {
-#pragma unroll
-        for (int j = 0; j < EPL; ++j)
-            if ((uint32_t)j >= nvalid) col[j] = 0u;
-    }
-    flags = nvalid ? ((uint32_t)a.heads[e >> 3] & ((1u << nvalid) - 1u)) : 0u;
+    meta = a.meta[meta_slot(ch, lane)];
     base = a.chunk_nz[ch];
 }
 
@@ -164,17 +164,13 @@ __device__ __forceinline__ void load_hub(const A &a, float *s_hub) {
  * L2/HBM (kept in L2). COHERENT selects loads that see writes made earlier in
  * the same launch. */
 template <bool COHERENT = false, typename A>
-__device__ __forceinline__ void gather_chunk(const A &a, const uint32_t (&col)[EPL], uint32_t nvalid,
-                                             const float *s_hub, uint64_t pol_keep, float (&val)[EPL]) {
+__device__ __forceinline__ void gather_chunk(const A &a, const uint32_t (&col)[EPL], const float *s_hub,
+                                             uint64_t pol_keep, float (&val)[EPL]) {
 #pragma unroll
     for (int j = 0; j < EPL; ++j) {
         const uint32_t x = col[j];
-        float v = 0.0f;
-        if ((uint32_t)j < nvalid) {
-            if (x < a.hub) v = s_hub[x];
-            else v = COHERENT ? ld_cg_keep_f32(a.c_old + x, pol_keep) : ld_keep_f32(a.c_old + x, pol_keep);
-        }
-        val[j] = v;
+        if (x < a.hub) val[j] = s_hub[x];
+        else val[j] = COHERENT ? ld_cg_keep_f32(a.c_old + x, pol_keep) : ld_keep_f32(a.c_old + x, pol_keep);
     }
 }
 
@@ -198,80 +194,99 @@ __device__ __forceinline__ Agg3 vshfl_up(Agg3 x, int o) {
  * chunk are written to nzsum; a row that began in an earlier chunk leaves its
  * part in head_part[ch], a row that continues into the next chunk leaves its
  * part in tail_part[ch] (both completed in chunk order by the fix-up pass).
- * ne is the end of the edge range being swept. A supplies heads; R supplies
- * nzsum, head_part and tail_part of value type V. */
-template <typename A, typename R, typename V>
-__device__ __forceinline__ void reduce_chunk_to(const A &a, const R &o, uint32_t ch, uint32_t lane,
-                                                const V (&val)[EPL], uint32_t flags, uint32_t nvalid, uint32_t base,
-                                                uint64_t ne) {
+ * ne is the end of the edge range being swept. R supplies nzsum, head_part and
+ * tail_part of value type V.
+ *
+ * The order of every sum: a lane's edges one after another, the lanes of a row by
+ * doubling steps, the carry from earlier lanes last. The kernels that reduce chunks
+ * issue more instructions here than anywhere else, so the common chunks take short
+ * ways through it: one without a row start is a plain scan, and the stores of rows
+ * that lie inside a lane are tried only when some lane has two row starts. */
+template <typename R, typename V>
+__device__ __forceinline__ void reduce_chunk_to(const R &o, uint32_t ch, uint32_t lane, V (&val)[EPL],
+                                                uint32_t meta, uint32_t base, uint64_t ne) {
     const uint32_t FULL = 0xFFFFFFFFu;
     const uint64_t e0 = (uint64_t)ch * CH;
-    const uint32_t head0 = __shfl_sync(FULL, flags, 0) & 1u;
-    const uint32_t nh_lane = __popc(flags);
-    uint32_t incl = nh_lane;
+    const V zero = vzero(val[0]);
+    uint32_t L = 31u; /* the lane of the chunk's last edge */
+    if (ne - e0 < (uint64_t)CH) { /* the last chunk: what was gathered for its empty slots is dropped */
+        const uint32_t left = (uint32_t)(ne - e0);
+        L = (left - 1u) / EPL;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        uint32_t y = __shfl_up_sync(FULL, incl, d);
-        if (lane >= (uint32_t)d) incl += y;
+        for (int j = 0; j < EPL; ++j)
+            if (EPL * lane + (uint32_t)j >= left) val[j] = zero;
     }
-    const uint32_t H = incl - nh_lane; /* heads in earlier lanes of this chunk */
-    const uint32_t Htot = __shfl_sync(FULL, incl, 31);
-    const uint32_t rowbase = base + (head0 ? 0u : 1u) + H; /* row started by this lane's first head */
+    const uint32_t flags = meta & 0xFFu;
+    const uint32_t hb = __ballot_sync(FULL, flags != 0u);
+    V run = zero;
+    if (hb == 0u) { /* the whole chunk lies inside one row */
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) run = vadd(run, val[j]);
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const V vu = vshfl_up(run, d);
+            if (lane >= (uint32_t)d) run = vadd(vu, run);
+        }
+        if (lane == L) o.head_part[ch] = run;
+        return;
+    }
+    const uint32_t meta0 = __shfl_sync(FULL, meta, 0);
+    const uint32_t head0 = meta0 & 1u;
+    const uint32_t H = lane ? meta >> 8 : 0u; /* heads in earlier lanes of this chunk */
+    const uint32_t row0 = base + (head0 ? 0u : 1u); /* the chunk's first row start */
 
     /* in-lane segments: rows that start and end inside this lane are final */
-    const V zero = vzero(val[0]);
-    V run = zero, pre = zero;
-    uint32_t nh = 0;
+    V pre = zero;
+    if (__any_sync(FULL, (flags & (flags - 1u)) != 0u)) {
+        uint32_t at = row0 + H - 1u;
 #pragma unroll
-    for (int j = 0; j < EPL; ++j) {
-        if ((uint32_t)j < nvalid) {
+        for (int j = 0; j < EPL; ++j) {
             if ((flags >> j) & 1u) {
-                if (nh == 0) pre = run;
-                else o.nzsum[rowbase + nh - 1] = run;
-                ++nh;
+                if (at == row0 + H - 1u) pre = run;
+                else o.nzsum[at] = run;
+                ++at;
+                run = zero;
+            }
+            run = vadd(run, val[j]);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) {
+            if ((flags >> j) & 1u) {
+                pre = run;
                 run = zero;
             }
             run = vadd(run, val[j]);
         }
     }
-    /* warp segmented inclusive scan of (lane has a head, lane tail value) */
-    int finc = nh > 0;
-    V vinc = run;
+    /* warp segmented inclusive scan of the lanes' tail values: a lane adds the lane d
+     * before it when no row starts in the d lanes up to itself */
+    const uint32_t upto = hb & (FULL >> (31u - lane));
+    const uint32_t dist = lane - (31u - (uint32_t)__clz((int)(upto | 1u)));
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        int fu = __shfl_up_sync(FULL, finc, d);
-        V vu = vshfl_up(vinc, d);
-        if (lane >= (uint32_t)d) {
-            if (!finc) vinc = vadd(vu, vinc);
-            finc |= fu;
-        }
+        const V vu = vshfl_up(run, d);
+        if (dist >= (uint32_t)d) run = vadd(vu, run);
     }
-    const V prev = vshfl_up(vinc, 1);
-    const V carry = lane ? prev : zero;
-    if (nh > 0) {
+    const V prev = vshfl_up(run, 1);
+    if (flags) {
         /* the row that ends at this lane's first head */
-        const V sv = vadd(carry, pre);
+        const V sv = vadd(lane ? prev : zero, pre);
         if (H == 0 && !head0) o.head_part[ch] = sv;                /* began in an earlier chunk */
-        else if (!(lane == 0 && head0)) o.nzsum[rowbase - 1] = sv; /* began in an earlier lane */
+        else if (!(lane == 0 && head0)) o.nzsum[row0 + H - 1u] = sv; /* began in an earlier lane */
     }
     /* the chunk's last row */
-    const uint32_t L = (ne - e0 >= (uint64_t)CH) ? 31u : (uint32_t)((ne - 1 - e0) / EPL);
     if (lane == L) {
-        if (Htot == 0) {
-            o.head_part[ch] = vinc; /* the whole chunk lies inside one row */
-        } else {
-            const bool ends_here = (e0 + CH >= ne) || (a.heads[(e0 + CH) >> 3] & 1u);
-            const uint32_t idx = base + (head0 ? 0u : 1u) + Htot - 1;
-            if (ends_here) o.nzsum[idx] = vinc;
-            else o.tail_part[ch] = vinc;
-        }
+        const uint32_t last = row0 + H + __popc(flags) - 1u;
+        if ((meta0 >> 8) & 1u) o.nzsum[last] = run;
+        else o.tail_part[ch] = run;
     }
 }
 
 template <typename A>
-__device__ __forceinline__ void reduce_chunk(const A &a, uint32_t ch, uint32_t lane, const float (&val)[EPL],
-                                             uint32_t flags, uint32_t nvalid, uint32_t base, uint64_t ne) {
-    reduce_chunk_to(a, a, ch, lane, val, flags, nvalid, base, ne);
+__device__ __forceinline__ void reduce_chunk(const A &a, uint32_t ch, uint32_t lane, float (&val)[EPL],
+                                             uint32_t meta, uint32_t base, uint64_t ne) {
+    reduce_chunk_to(a, ch, lane, val, meta, base, ne);
 }
 
 constexpr int EDGE_THREADS = 1024;
@@ -392,7 +407,8 @@ struct EdgeTier {
     uint32_t nchunks = 0, nrows = 0, nsplit = 0, nlong = 0;
     uint32_t first = 0; /* relabelled id of column value 0 */
     uint32_t hub = 0;   /* contributions [first, first + hub) staged in shared memory */
-    dbuf<uint32_t> col, head_bits, chunk_nz, long_split;
+    dbuf<uint32_t> col, chunk_nz, long_split;
+    dbuf<uint16_t> lane_meta;
     dbuf<uint4> split;
     dbuf<float> nzsum, parts;
 };
@@ -413,7 +429,8 @@ struct ChunkPlan {
      * whose relabelling could not keep every graph's id range */
     bool rows_relabelled = true;
     /* nz row i: original vertex id, first edge position in col_r's order */
-    dbuf<uint32_t> nz_rows, nz_start, zero_rows, head_bits, chunk_nz, od_nz;
+    dbuf<uint32_t> nz_rows, nz_start, zero_rows, chunk_nz, od_nz;
+    dbuf<uint16_t> lane_meta; /* row starts by chunk and lane */
     dbuf<uint4> split;
     uint32_t nlong = 0;
     dbuf<uint32_t> long_split; /* split rows spanning more than LONG_SPAN chunks */

@@ -75,7 +75,7 @@ __device__ __forceinline__ uint64_t res_cost(const uint32_t *chunk_nz, uint32_t 
 }
 
 /* the range of each CTA: thread k of one block takes CTA k */
-__global__ void k_res_ranges(const uint32_t *__restrict__ chunk_nz, const uint8_t *__restrict__ heads,
+__global__ void k_res_ranges(const uint32_t *__restrict__ chunk_nz, const uint16_t *__restrict__ meta,
                              const uint4 *__restrict__ split, uint32_t nchunks, uint32_t nnz, uint32_t nsplit,
                              uint32_t ncta, const uint32_t *__restrict__ od_nz,
                              const uint32_t *__restrict__ nz_cidx, ResRange *__restrict__ out,
@@ -103,7 +103,7 @@ __global__ void k_res_ranges(const uint32_t *__restrict__ chunk_nz, const uint8_
     };
     auto first_row = [&](uint32_t c) { /* first row that begins at or after chunk c */
         if (c >= nchunks) return nnz;
-        return chunk_nz[c] + ((heads[((uint64_t)c * CH) >> 3] & 1u) ? 0u : 1u);
+        return chunk_nz[c] + ((meta[meta_slot(c, 0)] & 1u) ? 0u : 1u);
     };
     auto first_split = [&](uint32_t row) {
         uint32_t lo = 0, hi = nsplit;
@@ -212,9 +212,9 @@ __global__ void __launch_bounds__(EDGE_THREADS, 1) k_pr_resident(ResArgs m) {
     if (tid == 0) s_stop = 0;
 
     /* the first chunk's columns do not change: they are loaded ahead of each barrier */
-    uint32_t col[EPL], flags = 0, nvalid = 0, base = 0;
+    uint32_t col[EPL], meta = 0, base = 0;
     const uint32_t first = rg.c0 + warp;
-    if (first < rg.c1) load_chunk(a, first, lane, pol_stream, col, flags, nvalid, base, a.ne);
+    if (first < rg.c1) load_chunk(a, first, lane, pol_stream, col, meta, base);
     uint32_t meets = gridDim.x;
     if (!res_sync(m, meets)) return;
 
@@ -262,14 +262,12 @@ __global__ void __launch_bounds__(EDGE_THREADS, 1) k_pr_resident(ResArgs m) {
 #pragma unroll
             for (int j = 0; j < EPL; ++j) {
                 const uint32_t x = col[j];
-                float v = 0.0f;
-                if ((uint32_t)j < nvalid) v = x < a.hub ? s_hub[x] : ld_contrib(c_old + x);
-                val[j] = v;
+                val[j] = x < a.hub ? s_hub[x] : ld_contrib(c_old + x);
             }
-            const uint32_t cur = ch, cf = flags, cn = nvalid, cb = base;
+            const uint32_t cur = ch, cm = meta, cb = base;
             ch += WARPS;
-            if (ch < rg.c1) load_chunk(a, ch, lane, pol_stream, col, flags, nvalid, base, a.ne);
-            reduce_chunk(a, cur, lane, val, cf, cn, cb, a.ne);
+            if (ch < rg.c1) load_chunk(a, ch, lane, pol_stream, col, meta, base);
+            reduce_chunk(a, cur, lane, val, cm, cb, a.ne);
         }
         /* rows and split rows that need nothing of other CTAs, and the one that does; a
          * thread's first split row is on its way during the wait */
@@ -376,7 +374,7 @@ __global__ void __launch_bounds__(EDGE_THREADS, 1) k_pr_resident(ResArgs m) {
             n += __shfl_down_sync(FULL, n, o);
         }
         if (lane == 0) s_red[warp] = make_double2(d, n);
-        if (first < rg.c1) load_chunk(a, first, lane, pol_stream, col, flags, nvalid, base, a.ne);
+        if (first < rg.c1) load_chunk(a, first, lane, pol_stream, col, meta, base);
         __syncthreads();
         if (warp == 0) {
             const double2 w = s_red[lane];
@@ -451,7 +449,7 @@ int pagerank_resident(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
         GCG_TRY(w.res_bres.alloc(2 * (size_t)ncta));
         for (cudaEvent_t &e : w.ev)
             if (!e) GCG_CUDA(cudaEventCreate(&e));
-        k_res_ranges<<<ncta / 32 + 1, 32, 0, s>>>(pl.chunk_nz.get(), (const uint8_t *)pl.head_bits.get(),
+        k_res_ranges<<<ncta / 32 + 1, 32, 0, s>>>(pl.chunk_nz.get(), pl.lane_meta.get(),
                                                      pl.split.get(), pl.nchunks, pl.nnz, pl.nsplit, ncta,
                                               pl.od_nz.get(), pl.nz_cidx.get(), w.res_rg.get(), w.res_ctl.get());
         GCG_LAUNCH_CHECK();
@@ -480,7 +478,7 @@ int pagerank_resident(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
     SweepArgs &a = m.a;
     a.col = pl.col_r.get();
     a.outdeg = g->outdeg.get();
-    a.heads = (const uint8_t *)pl.head_bits.get();
+    a.meta = pl.lane_meta.get();
     a.chunk_nz = pl.chunk_nz.get();
     a.nz_rows = pl.nz_rows.get();
     a.zero_rows = pl.zero_rows.get();

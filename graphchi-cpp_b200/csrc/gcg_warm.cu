@@ -80,7 +80,7 @@ __host__ __device__ __forceinline__ uint32_t bf16_bits(float x_rounded) {
  * {L(u), L(u), indeg(u)} to its row's (sum, max, sum). */
 struct AggArgs {
     const uint32_t *col; /* relabelled sources */
-    const uint8_t *heads;
+    const uint16_t *meta;
     const uint32_t *chunk_nz;
     uint64_t ne;
     uint32_t nchunks, hub;
@@ -114,21 +114,20 @@ __global__ void __launch_bounds__(EDGE_THREADS, 1) k_warm_agg_edges(AggArgs a, A
     for (uint32_t i = threadIdx.x; i < a.hub; i += blockDim.x) s_vs[i] = a.vstat[i];
     __syncthreads();
     uint32_t ch = gwarp;
-    uint32_t col[EPL], flags = 0, nvalid = 0, base = 0;
-    if (ch < a.nchunks) load_chunk(a, ch, lane, pol_stream, col, flags, nvalid, base, a.ne);
+    uint32_t col[EPL], meta = 0, base = 0;
+    if (ch < a.nchunks) load_chunk(a, ch, lane, pol_stream, col, meta, base);
     for (; ch < a.nchunks; ch += nwarps) {
         Agg3 val[EPL];
 #pragma unroll
         for (int j = 0; j < EPL; ++j) {
             const uint32_t x = col[j];
-            uint2 w = make_uint2(0u, 0u);
-            if ((uint32_t)j < nvalid) w = x < a.hub ? s_vs[x] : ld_keep_u2(a.vstat + x, pol_keep);
+            const uint2 w = x < a.hub ? s_vs[x] : ld_keep_u2(a.vstat + x, pol_keep);
             const float L = __uint_as_float(w.x);
             val[j] = Agg3{L, L, (float)w.y};
         }
-        const uint32_t cf = flags, cn = nvalid, cb = base;
-        if (ch + nwarps < a.nchunks) load_chunk(a, ch + nwarps, lane, pol_stream, col, flags, nvalid, base, a.ne);
-        reduce_chunk_to(a, o, ch, lane, val, cf, cn, cb, a.ne);
+        const uint32_t cm = meta, cb = base;
+        if (ch + nwarps < a.nchunks) load_chunk(a, ch + nwarps, lane, pol_stream, col, meta, base);
+        reduce_chunk_to(o, ch, lane, val, cm, cb, a.ne);
     }
 }
 
@@ -755,7 +754,7 @@ int warm_aggregates(gcg_graph *g, tbuf<Agg3> &agg, cudaStream_t s) {
     if (pl.nchunks) {
         AggArgs a;
         a.col = pl.col_r.get();
-        a.heads = (const uint8_t *)pl.head_bits.get();
+        a.meta = pl.lane_meta.get();
         a.chunk_nz = pl.chunk_nz.get();
         a.ne = g->ne;
         a.nchunks = pl.nchunks;
