@@ -10,9 +10,10 @@
  * (1 + max level of those u, 0 if none) orders the sweep: every level is a set of
  * independent vertices. Within a sweep, levels run in order; each vertex sums
  * sequentially (bit-exact float order), reading new values below its id and old
- * values above it. Levels come from a monotone relaxation over the in-CSR and a
- * radix sort of (level, id); the per-level launches of one sweep are captured
- * once in a CUDA graph and replayed per sweep.
+ * values above it. Levels come from topological rounds over the in-CSR and a radix
+ * sort of (level, id); a sweep is one cooperative launch with a grid barrier between
+ * levels, and the sums of long rows, though sequential by definition, are evaluated
+ * in parallel with the same bits (group_add).
  *
  * The same schedule runs the edge-value program of the app (PagerankProgram,
  * example_apps/pagerank.cpp:73-113, taken when num_vertices * 4 >= membudget):
@@ -103,12 +104,13 @@ __global__ void __launch_bounds__(256) k_gs_round(uint32_t r, const uint32_t *__
 }
 
 /* Vertex classes of a level, by in-degree: a thread sums a row of at most
- * GS_THREAD_MAX in-edges, a warp one of at most GS_WARP_MAX, a block a longer
- * one. Every class adds the in-edges one after another in ascending source
- * order (a float sum is not associative); the cooperating threads only load. */
-/* R-MAT scale 22, per sweep: warp limit 1024: 31.8 ms, 512: 31.1, 256: 29.0, 128: 29.1
- * (scale 24: 88.6 ms for all four) */
-constexpr uint32_t GS_THREAD_MAX = 32, GS_WARP_MAX = 256;
+ * GS_THREAD_MAX in-edges, a warp one of at most GS_WARP_MAX, a group of threads a
+ * longer one. The result is always that of adding the in-edges one after another in
+ * ascending source order (a float sum is not associative). A thread's and a warp's
+ * row have all their loads in flight at once: with 32 in-edges per thread, eight at a
+ * time, and a warp's batches one ahead, their latencies made most of a small level
+ * (scale 14: 8.4 against 6.0 us a level). */
+constexpr uint32_t GS_THREAD_MAX = 8, GS_WARP_MAX = 256;
 constexpr int GS_CLASSES = 4; /* segments per level: thread, warp, block, (unused) */
 
 /* sort key: level, class, vertex id */
@@ -165,18 +167,6 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-/* block class: steps of GS_STEP values, GS_DEPTH of them in flight (per sweep
- * at R-MAT scale 24, 10 sweeps: 1024 x 2 88.6 ms, 1024 x 3 90.1, 1024 x 4 90.7,
- * 2048 x 2 88.0, 2048 x 3 92.7, 512 x 2 116.1, 512 x 3 119.7, 256 x 3 108.2) */
-constexpr uint32_t GS_STEP = 1024, GS_DEPTH = 2;
-
-/* value of in-edge (u -> v): this sweep's for u < v (an earlier level, written
- * by an earlier launch), the previous sweep's otherwise */
-__device__ __forceinline__ float gs_in_value(uint32_t u, uint32_t v, const float *__restrict__ pr_old,
-                                             const float *__restrict__ pr_new) {
-    return u < v ? __ldg(pr_new + u) : __ldg(pr_old + u);
-}
-
 /* The apply of one vertex. In-memory program (EDGE = false), pagerank.cpp:127-136:
  * pr = (float)((0.15 + 0.85 * (double)sum) / outc). Edge-value program (EDGE =
  * true), pagerank.cpp:89-111: pagerank = (float)(0.15 + 0.85 * (double)sum), the
@@ -186,9 +176,9 @@ __device__ __forceinline__ float gs_in_value(uint32_t u, uint32_t v, const float
  * contraction, the same rounding as the reference's separate double multiply
  * and add. */
 template <bool EDGE, bool TRACK>
-__device__ __forceinline__ void gs_apply(uint32_t v, float sum, const uint32_t *__restrict__ outdeg, float *pr_new,
+__device__ __forceinline__ void gs_apply(uint32_t v, float sum, uint32_t outdeg, float *pr_new,
                                          float *val, float *delta, double reset, double damping) {
-    const int outc = (int)outdeg[v];
+    const int outc = (int)outdeg;
     const double t = __dadd_rn(reset, __dmul_rn(damping, (double)sum));
     if (EDGE) pr_new[v] = outc > 0 ? __fdiv_rn(__double2float_rn(t), (float)outc) : 0.0f;
     else pr_new[v] = outc > 0 ? (float)__ddiv_rn(t, (double)outc) : (float)t;
@@ -199,115 +189,407 @@ __device__ __forceinline__ void gs_apply(uint32_t v, float sum, const uint32_t *
     }
 }
 
-/* One level of a sweep: the level's vertices are independent. Blocks
- * [0, nb) take the block-class vertices (one each: the threads copy the
- * in-edge values of a GS_STEP-edge step into shared memory, GS_DEPTH steps in
- * flight, thread 0 adds the step in order); the next blocks take the
- * warp-class vertices (one per warp: 32 values per batch, lane 0 adds them in
- * order from shuffles, the next batch already loading); the rest take the
- * thread-class vertices (eight loads in flight, then eight adds in order).
- * Levels of sweeps queued after `done` was raised return at once. */
-template <bool EDGE, bool TRACK>
-__global__ void __launch_bounds__(256) k_gs_level(const uint32_t *__restrict__ order, uint32_t tb, uint32_t wb,
-                                                  uint32_t bb, uint32_t be, const uint32_t *__restrict__ rowptr,
-                                                  const uint32_t *__restrict__ col,
-                                                  const uint32_t *__restrict__ outdeg,
-                                                  const float *__restrict__ pr_old, float *pr_new, float *val,
-                                                  float *delta, const int *done, double reset, double damping) {
-    if (TRACK && *(volatile const int *)done) return;
-    const uint32_t nb = be - bb, nwb = (bb - wb + 7) / 8;
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    if (blockIdx.x < nb) { /* block class */
-        /* GS_DEPTH steps of GS_STEP in-edge values in flight: every thread copies
-         * GS_STEP / 256 values of a step into shared memory with cp.async (the
-         * source columns read one step ahead), so the loads of the next step
-         * overlap thread 0's in-order adds of the current one */
-        constexpr uint32_t GQ = GS_STEP / 256;
-        __shared__ __align__(16) float s_val[GS_DEPTH][GS_STEP];
-        const uint32_t v = order[bb + blockIdx.x];
-        const uint32_t jb = rowptr[v], je = rowptr[v + 1];
-        const uint32_t nstep = (je - jb + GS_STEP - 1) / GS_STEP;
-        float sum = 0.0f;
-        /* this thread's copies for step b (source columns u), then one commit
-         * group per step, empty past the row's end */
-        auto issue = [&](uint32_t b, const uint32_t (&u)[GQ]) {
+/* ---- exact sums of long rows ------------------------------------------------
+ * A row's value is the float sum of its in-edge values one after another, each add
+ * rounded: a chain of dependent adds. It can be evaluated in parallel, bit for bit,
+ * as long as the running sum stays in one binade: there the sum is a whole number m
+ * of its ulp u, and adding x >= 0 makes it m + round(x / u), to nearest, ties to the
+ * even result. The increment depends on m only through m's parity, and only in a tie,
+ * so each value is a function of the parity (two increments), and such functions
+ * compose associatively: a prefix scan gives every partial sum. With E the binade's
+ * first float (even) and E' the next one (odd), the two increments are
+ * bits(E + x) - bits(E) and bits(E' + x) - bits(E'): one float add each. The first
+ * partial sum that leaves the binade is formed by an ordinary add, and the scan starts
+ * again behind it in the new binade, at most once per doubling of the sum. Sums that
+ * are zero, subnormal or not finite and values that are negative or NaN go one by one.
+ *
+ * A thread adds in ~4.5 cycles a value; a pass takes ~500 cycles for up to 1,024
+ * values, ~1,100 where the sum leaves its binade. R-MAT, per sweep, against one launch
+ * per level and one thread's adds: scale 20 10.6 -> 6.1 ms, scale 22 29.1 -> 15.2 ms
+ * (1,340 levels, 11.3 us each: barrier and value latency ~4, the longest row's sum the
+ * rest). */
+constexpr uint32_t GS_GROUP = 256;                /* threads that take a block-class row */
+constexpr uint32_t GS_STEP = 4 * GS_GROUP;        /* values of a step, four per thread */
+constexpr uint32_t GS_DEPTH = 3;                  /* steps in flight */
+constexpr uint32_t GS_THREADS = 512;              /* one CTA per SM, two groups */
+constexpr uint32_t GS_GROUPS = GS_THREADS / GS_GROUP;
+constexpr uint32_t GS_TAIL = 64;                  /* so few values are added by one thread */
+constexpr uint32_t GS_HEAD = 256;                 /* a row's first values: the sum doubles too often for the scan
+                                                     (scale 20: 128 6.72 ms, 256 6.47, 512 6.50) */
+constexpr uint32_t BINADE = 1u << 23;             /* ulps in a binade */
+constexpr uint32_t INC_MAX = 1u << 24;            /* increments are cut here: past any binade's end */
+
+constexpr uint32_t GS_WARPS = GS_GROUP / 32;
+constexpr uint32_t ODD_VALUES = 0xFFFFFFFFu;      /* in place of a warp's increment */
+
+/* Shared memory of a group. What one pass or thread tells the group alternates between
+ * two places: between two uses of one place lies a barrier that every reader of the
+ * first has passed after reading. */
+struct GsGroup {
+    float val[GS_DEPTH][GS_STEP];
+    uint2 total[2][GS_WARPS]; /* each warp's increment for an even and an odd start */
+    struct {
+        float sum;
+        uint32_t pos;
+    } told[2];
+};
+
+__device__ __forceinline__ void group_sync(uint32_t grp) {
+    asm volatile("bar.sync %0, %1;" ::"r"(grp + 1u), "n"(GS_GROUP) : "memory");
+}
+
+/* s + sv[k] + ... + sv[end - 1], one after another */
+__device__ __forceinline__ float add_in_order(float s, const float *sv, uint32_t k, uint32_t end) {
+    for (; k < end && (k & 3u); ++k) s += sv[k];
+    for (; k + 16 <= end; k += 16) { /* four loads, then the sixteen adds */
+        float4 q[4];
 #pragma unroll
-            for (uint32_t q = 0; q < GQ; ++q)
-                if (b < nstep && jb + b * GS_STEP + q * 256 + tid < je)
-                    cp_async4(&s_val[b % GS_DEPTH][q * 256 + tid], (u[q] < v ? pr_new : pr_old) + u[q]);
-            cp_async_commit();
-        };
-        auto columns = [&](uint32_t b, uint32_t (&u)[GQ]) {
+        for (int i = 0; i < 4; ++i) q[i] = *(const float4 *)(sv + k + 4 * i);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            s += q[i].x;
+            s += q[i].y;
+            s += q[i].z;
+            s += q[i].w;
+        }
+    }
+    for (; k < end; ++k) s += sv[k];
+    return s;
+}
+
+/* sum + sv[0] + ... + sv[n - 1] in this order, by a group; every thread has sum and
+ * gets the result. head: values that one thread adds first. par: which of the two
+ * places are next, bit 0 for total, bit 1 for told. */
+__device__ __forceinline__ float group_add(GsGroup &g, const float *sv, uint32_t n, uint32_t head, uint32_t grp,
+                                           uint32_t tid, float sum, uint32_t &par) {
+    const uint32_t FULL = 0xFFFFFFFFu, lane = tid & 31u, warp = tid >> 5;
+    auto one_thread = [&](uint32_t pos, uint32_t end) {
+        par ^= 2u;
+        auto &told = g.told[par >> 1];
+        if (tid == 0) told.sum = add_in_order(sum, sv, pos, end);
+        group_sync(grp);
+        sum = told.sum;
+    };
+    uint32_t pos = n <= head + GS_TAIL && head ? n : min(head, n);
+    if (pos) one_thread(0, pos);
+    const float4 q = *(const float4 *)(sv + 4u * tid);
+    while (pos < n) {
+        const uint32_t sb = __float_as_uint(sum), E = sb & 0x7F800000u;
+        /* few values; or a negative, zero, subnormal, huge or not finite sum */
+        if (n - pos <= GS_TAIL || sb >= 0x7F000000u || E == 0u) {
+            one_thread(pos, n);
+            return sum;
+        }
+        const float e0 = __uint_as_float(E), e1 = __uint_as_float(E + 1u);
+        float x[4] = {q.x, q.y, q.z, q.w};
+        uint32_t a0[4], a1[4];
+        bool tie = false, odd = false;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t i = 4u * tid + k;
+            if (i < pos || i >= n) x[k] = 0.0f;
+            odd |= !(x[k] >= 0.0f);
+            a0[k] = min(__float_as_uint(__fadd_rn(e0, x[k])) - E, INC_MAX);
+            a1[k] = min(__float_as_uint(__fadd_rn(e1, x[k])) - (E + 1u), INC_MAX);
+            tie |= a0[k] != a1[k];
+        }
+        /* this thread's function (t0, t1) and its warp's (w0, w1). Without a tie both are
+         * whole numbers, and unless the sum leaves the binade among this warp's values
+         * only the total is wanted. */
+        uint32_t t0, t1, w0, w1, p0 = 0u, p1 = 0u;
+        const bool ties = __any_sync(FULL, tie);
+        if (!ties) {
+            t0 = t1 = (a0[0] + a0[1]) + (a0[2] + a0[3]);
+            w0 = w1 = min(__reduce_add_sync(FULL, t0), INC_MAX); /* 128 increments: at most 2^31 */
+        } else {
+            t0 = t1 = 0u;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                t0 += (t0 & 1u) ? a1[k] : a0[k];
+                t1 += (t1 & 1u) ? a0[k] : a1[k];
+            }
+            w0 = t0;
+            w1 = t1;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y0 = __shfl_up_sync(FULL, w0, d), y1 = __shfl_up_sync(FULL, w1, d);
+                if (lane >= (uint32_t)d) { /* first the lower lanes' function, then this one */
+                    const uint32_t n0 = y0 + ((y0 & 1u) ? w1 : w0), n1 = y1 + ((y1 & 1u) ? w0 : w1);
+                    w0 = min(n0, INC_MAX);
+                    w1 = min(n1, INC_MAX);
+                }
+            }
+            p0 = __shfl_up_sync(FULL, w0, 1);
+            p1 = __shfl_up_sync(FULL, w1, 1);
+            if (lane == 0u) p0 = p1 = 0u;
+        }
+        if (__any_sync(FULL, odd)) w0 = w1 = ODD_VALUES;
+        par ^= 1u;
+        uint2 *const total = g.total[par & 1u];
+        if (lane == 31u) total[warp] = make_uint2(w0, w1);
+        group_sync(grp);
+        /* ulps past the binade's first float: now, before this warp, after all warps */
+        uint32_t m = sb - E, before = 0u;
+        bool odd_values = false;
+#pragma unroll
+        for (uint32_t w = 0; w < GS_WARPS; ++w) {
+            const uint2 t = total[w];
+            if (w == warp) before = m;
+            odd_values |= t.x == ODD_VALUES;
+            m = min(m + ((m & 1u) ? t.y : t.x), INC_MAX);
+        }
+        if (odd_values) {
+            one_thread(pos, n);
+            return sum;
+        }
+        if (m < BINADE) { /* the sum stays in its binade: every thread has it */
+            sum = __uint_as_float(E + m);
+            return sum;
+        }
+        par ^= 2u;
+        auto &told = g.told[par >> 1];
+        const uint32_t through = before + ((before & 1u) ? w1 : w0); /* (lane 31's is the warp's) */
+        if (before < BINADE && __shfl_sync(FULL, through, 31) >= BINADE) { /* it leaves it among this warp's values */
+            if (!ties) {
+                uint32_t incl = t0;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const uint32_t y = __shfl_up_sync(FULL, incl, d);
+                    if (lane >= (uint32_t)d) incl += y;
+                }
+                p0 = p1 = incl - t0;
+            }
+            uint32_t at = before + ((before & 1u) ? p1 : p0);
+            if (at < BINADE && at + ((at & 1u) ? t1 : t0) >= BINADE) { /* this thread's */
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t next = at + ((at & 1u) ? a1[k] : a0[k]);
+                    if (at < BINADE && next >= BINADE) {
+                        told.sum = __fadd_rn(__uint_as_float(E + at), x[k]);
+                        told.pos = 4u * tid + k + 1u;
+                    }
+                    at = next;
+                }
+            }
+        }
+        group_sync(grp);
+        sum = told.sum;
+        pos = told.pos;
+    }
+    return sum;
+}
+
+struct GsArgs {
+    const uint32_t *order, *off; /* off: GS_CLASSES entries per level */
+    uint32_t nlev;
+    const uint32_t *rowptr, *col, *outdeg;
+    const float *pr_old;
+    float *pr_new, *val, *delta;
+    const int *done;
+    uint32_t *bar; /* arrivals at the grid barrier, counted up over the call */
+    uint32_t meets; /* arrivals before this sweep */
+    int *err;
+    double reset, damping;
+};
+
+/* polls of the grid barrier: seconds */
+constexpr long long GS_SPIN = 1ll << 23;
+
+/* the grid barrier in two halves, so that what follows need not wait for static loads:
+ * every CTA arrives; then waits, false when the (bounded) wait ran out here or in
+ * another CTA */
+__device__ __forceinline__ void gs_arrive(const GsArgs &a) {
+    __syncthreads();
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+}
+__device__ __forceinline__ bool gs_wait(const GsArgs &a, uint32_t target) {
+    __shared__ int s_ok;
+    if (threadIdx.x == 0) {
+        int ok = 1;
+        for (long long spins = 0;; ++spins) {
+            uint32_t seen;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bar) : "memory");
+            if ((int32_t)(seen - target) >= 0) break;
+            if ((spins & 255) == 255 && *(volatile int *)a.err) ok = 0;
+            if (spins > GS_SPIN) {
+                atomicExch(a.err, 1);
+                ok = 0;
+            }
+            if (!ok) break;
+        }
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+/* One sweep: the levels in order, a grid barrier between them (one cooperative
+ * launch, one CTA per SM). A level's vertices are independent. A block-class vertex
+ * is taken by a group of 256 threads: the threads copy the in-edge values of a step
+ * into shared memory, GS_DEPTH - 1 steps ahead, and group_add adds a step. A
+ * warp-class vertex by a warp: all values in flight, then added in order from
+ * shuffles. A thread-class vertex by a thread: all loads in flight, then the adds. Block-class vertices go to the CTAs from the
+ * first on, the others from the last warp down, so that a small level's rows lie on
+ * different SMs. What does not change within a sweep (a level's vertices, row bounds
+ * and first columns) is loaded while the CTA waits for the others. */
+template <bool EDGE, bool TRACK>
+__global__ void __launch_bounds__(GS_THREADS, 1) k_gs_sweep(GsArgs a) {
+    if (TRACK && *(volatile const int *)a.done) return; /* sweeps queued after the tolerance was met */
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    const uint32_t grp = threadIdx.x / GS_GROUP, tid = threadIdx.x % GS_GROUP, lane = threadIdx.x & 31u;
+    GsGroup &g = ((GsGroup *)s_raw)[grp];
+    const uint32_t ngroups = gridDim.x * GS_GROUPS, nwarps = gridDim.x * (GS_THREADS / 32u);
+    const uint32_t gid = grp * gridDim.x + blockIdx.x;
+    const uint32_t rev = nwarps - 1u - ((threadIdx.x >> 5) * gridDim.x + blockIdx.x); /* warps from the last down */
+    const float *pr_old = a.pr_old;
+    float *pr_new = a.pr_new;
+    uint32_t par = 0;
+
+    constexpr uint32_t GQ = GS_STEP / GS_GROUP;
+    auto value = [&](uint32_t u, uint32_t v) { return __ldcg((u < v ? pr_new : pr_old) + u); };
+    auto columns = [&](uint32_t jb, uint32_t je, uint32_t b, uint32_t *u) {
+#pragma unroll
+        for (uint32_t q = 0; q < GQ; ++q) {
+            const uint64_t j = (uint64_t)jb + (uint64_t)b * GS_STEP + q * GS_GROUP + tid;
+            u[q] = j < je ? __ldg(a.col + j) : 0u;
+        }
+    };
+
+    auto row_columns = [&](uint32_t jb, uint32_t je, uint32_t *u) { /* a warp-class row, 32 at a time */
+#pragma unroll
+        for (uint32_t q = 0; q < GS_WARP_MAX / 32; ++q) {
+            const uint64_t j = (uint64_t)jb + 32u * q + lane;
+            u[q] = j < je ? __ldg(a.col + j) : 0u;
+        }
+    };
+
+    /* the first vertex that this warp takes in a level: its id, row and first columns */
+    uint32_t pv = 0, pjb = 0, pje = 0, pod = 0, pc[8];
+    auto prefetch = [&](uint4 o) {
+        const uint32_t nb = o.w - o.z, nw = o.z - o.y, nt = o.y - o.x;
+        uint32_t i = 0xFFFFFFFFu;
+        if (gid < nb) i = o.z + gid;
+        else if (rev < nw) i = o.y + rev;
+        else if ((uint64_t)(rev - nw) * 32u + lane < nt) i = o.x + (rev - nw) * 32u + lane;
+        pv = pjb = pje = 0;
+        if (i != 0xFFFFFFFFu) {
+            pv = __ldg(a.order + i);
+            pjb = __ldg(a.rowptr + pv);
+            pje = __ldg(a.rowptr + pv + 1);
+            pod = __ldg(a.outdeg + pv);
+        }
+        if (gid < nb) {
+            columns(pjb, pje, 0, pc);
+            columns(pjb, pje, 1, pc + 4);
+        } else if (rev < nw) {
+            row_columns(pjb, pje, pc);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) pc[k] = pjb + k < pje ? __ldg(a.col + pjb + k) : 0u;
+        }
+    };
+
+    uint4 o = ((const uint4 *)a.off)[0], on = a.nlev > 1 ? ((const uint4 *)a.off)[1] : o;
+    prefetch(o);
+    uint32_t target = a.meets;
+    for (uint32_t l = 0; l < a.nlev; ++l) {
+        const uint32_t nb = o.w - o.z, nw = o.z - o.y, nt = o.y - o.x;
+        bool ready = true; /* the prefetched vertex is the next one */
+        for (uint32_t k = gid; k < nb; k += ngroups) { /* block class */
+            uint32_t v = pv, jb = pjb, je = pje, od = pod, c0[GQ], c1[GQ];
+            if (!ready) {
+                v = __ldg(a.order + o.z + k);
+                jb = __ldg(a.rowptr + v);
+                je = __ldg(a.rowptr + v + 1);
+                od = __ldg(a.outdeg + v);
+                columns(jb, je, 0, pc);
+                columns(jb, je, 1, pc + 4);
+            }
+            ready = false;
 #pragma unroll
             for (uint32_t q = 0; q < GQ; ++q) {
-                const uint32_t j = jb + b * GS_STEP + q * 256 + tid;
-                u[q] = b < nstep && j < je ? __ldg(col + j) : 0u;
+                c0[q] = pc[q];
+                c1[q] = pc[4 + q];
             }
-        };
-        uint32_t cn[GQ];
-        for (uint32_t b = 0; b + 1 < GS_DEPTH; ++b) {
-            columns(b, cn);
-            issue(b, cn);
+            const uint32_t nstep = (je - jb + GS_STEP - 1) / GS_STEP;
+            auto issue = [&](uint32_t b) { /* c0 holds step b's columns; one commit group per step */
+#pragma unroll
+                for (uint32_t q = 0; q < GQ; ++q)
+                    if ((uint64_t)jb + (uint64_t)b * GS_STEP + q * GS_GROUP + tid < je)
+                        cp_async4(&g.val[b % GS_DEPTH][q * GS_GROUP + tid], (c0[q] < v ? pr_new : pr_old) + c0[q]);
+                cp_async_commit();
+#pragma unroll
+                for (uint32_t q = 0; q < GQ; ++q) c0[q] = c1[q];
+                columns(jb, je, b + 2, c1);
+            };
+            float sum = 0.0f;
+            issue(0);
+            issue(1);
+            for (uint32_t b = 0; b < nstep; ++b) {
+                cp_async_wait<1>(); /* this thread's values of step b have landed */
+                group_sync(grp);    /* everyone's; step b - 1 is added */
+                issue(b + 2);       /* into step b - 1's buffer */
+                sum = group_add(g, g.val[b % GS_DEPTH], min(GS_STEP, je - (jb + b * GS_STEP)), b ? 0u : GS_HEAD, grp,
+                                tid, sum, par);
+            }
+            cp_async_wait<0>(); /* no copy in flight when the buffers are used again */
+            if (tid == 0) gs_apply<EDGE, TRACK>(v, sum, od, pr_new, a.val, a.delta, a.reset, a.damping);
+            group_sync(grp);
         }
-        columns(GS_DEPTH - 1, cn);
-        for (uint32_t b = 0; b < nstep; ++b) {
-            cp_async_wait<GS_DEPTH - 2>(); /* this thread's values of step b have landed */
-            __syncthreads();               /* everyone's; thread 0 is done with step b - 1 */
-            issue(b + GS_DEPTH - 1, cn);   /* into step b - 1's buffer */
-            columns(b + GS_DEPTH, cn);
-            if (tid == 0) { /* in order, four values per shared-memory load */
-                const uint32_t n = min(GS_STEP, je - (jb + b * GS_STEP));
-                const float *sv = s_val[b % GS_DEPTH];
-                uint32_t k = 0;
-                for (; k + 4 <= n; k += 4) {
-                    const float4 q = *(const float4 *)(sv + k);
-                    sum += q.x;
-                    sum += q.y;
-                    sum += q.z;
-                    sum += q.w;
+        for (uint32_t k = rev; k < nw; k += nwarps) { /* warp class */
+            uint32_t v = pv, jb = pjb, je = pje, od = pod;
+            if (!ready) {
+                v = __ldg(a.order + o.y + k);
+                jb = __ldg(a.rowptr + v);
+                je = __ldg(a.rowptr + v + 1);
+                od = __ldg(a.outdeg + v);
+                row_columns(jb, je, pc);
+            }
+            ready = false;
+            float x[GS_WARP_MAX / 32], sum = 0.0f;
+#pragma unroll
+            for (uint32_t q = 0; q < GS_WARP_MAX / 32; ++q)
+                x[q] = (uint64_t)jb + 32u * q + lane < je ? value(pc[q], v) : 0.0f;
+#pragma unroll
+            for (uint32_t q = 0; q < GS_WARP_MAX / 32; ++q) {
+                const uint32_t n = je - jb > 32u * q ? je - jb - 32u * q : 0u;
+                if (n == 0u) break;
+#pragma unroll
+                for (uint32_t i = 0; i < 32u; ++i) { /* in order, in every lane */
+                    const float z = __shfl_sync(0xFFFFFFFFu, x[q], (int)i);
+                    if (i < n) sum += z;
                 }
-                for (; k < n; ++k) sum += sv[k];
             }
+            if (lane == 0) gs_apply<EDGE, TRACK>(v, sum, od, pr_new, a.val, a.delta, a.reset, a.damping);
         }
-        cp_async_wait<0>(); /* no copy in flight when the block leaves */
-        if (tid == 0) gs_apply<EDGE, TRACK>(v, sum, outdeg, pr_new, val, delta, reset, damping);
-        return;
-    }
-    if (blockIdx.x < nb + nwb) { /* warp class */
-        const uint32_t i = wb + (blockIdx.x - nb) * 8 + warp;
-        if (i >= bb) return;
-        const uint32_t v = order[i];
-        const uint32_t jb = rowptr[v], je = rowptr[v + 1];
-        float sum = 0.0f;
-        float x = jb + lane < je ? gs_in_value(__ldg(col + jb + lane), v, pr_old, pr_new) : 0.0f;
-        for (uint32_t j0 = jb; j0 < je; j0 += 32) {
-            const uint32_t nj = j0 + 32 + lane;
-            const float y = nj < je ? gs_in_value(__ldg(col + nj), v, pr_old, pr_new) : 0.0f;
-            const uint32_t n = min(32u, je - j0);
-            for (uint32_t k = 0; k < n; ++k) {
-                const float z = __shfl_sync(0xFFFFFFFFu, x, (int)k);
-                sum += z; /* every lane keeps the same running sum, in order */
+        /* thread class: warps past those of the warp class first */
+        for (uint64_t k = (uint64_t)(rev >= nw % nwarps ? rev - nw % nwarps : rev + nwarps - nw % nwarps) * 32u + lane;
+             k < nt; k += (uint64_t)nwarps * 32u) {
+            uint32_t v = pv, jb = pjb, je = pje, od = pod;
+            const bool have = ready && rev >= nw;
+            if (!have) {
+                v = __ldg(a.order + o.x + k);
+                jb = __ldg(a.rowptr + v);
+                je = __ldg(a.rowptr + v + 1);
+                od = __ldg(a.outdeg + v);
             }
-            x = y;
-        }
-        if (lane == 0) gs_apply<EDGE, TRACK>(v, sum, outdeg, pr_new, val, delta, reset, damping);
-        return;
-    }
-    /* thread class */
-    const uint32_t nth = (gridDim.x - nb - nwb) * blockDim.x;
-    for (uint32_t i = tb + (blockIdx.x - nb - nwb) * blockDim.x + tid; i < wb; i += nth) {
-        const uint32_t v = order[i];
-        const uint32_t jb = rowptr[v], je = rowptr[v + 1];
-        float sum = 0.0f;
-        for (uint32_t j0 = jb; j0 < je; j0 += 8) {
-            float x[8];
+            float x[GS_THREAD_MAX], sum = 0.0f;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) x[k] = j0 + k < je ? gs_in_value(__ldg(col + j0 + k), v, pr_old, pr_new) : 0.0f;
+            for (uint32_t i = 0; i < GS_THREAD_MAX; ++i)
+                x[i] = jb + i < je ? value(have ? pc[i] : __ldg(a.col + jb + i), v) : 0.0f;
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-                if (j0 + k < je) sum += x[k];
+            for (uint32_t i = 0; i < GS_THREAD_MAX; ++i)
+                if (jb + i < je) sum += x[i];
+            ready = false;
+            gs_apply<EDGE, TRACK>(v, sum, od, pr_new, a.val, a.delta, a.reset, a.damping);
         }
-        gs_apply<EDGE, TRACK>(v, sum, outdeg, pr_new, val, delta, reset, damping);
+        if (l + 1 == a.nlev) break;
+        gs_arrive(a);
+        o = on;
+        if (l + 2 < a.nlev) on = ((const uint4 *)a.off)[l + 2];
+        prefetch(o);
+        target += gridDim.x;
+        if (!gs_wait(a, target)) return;
     }
 }
 
@@ -393,8 +675,7 @@ inline unsigned vgrid(uint32_t n) {
  * level l, nlev levels. */
 struct GsPlan {
     uint32_t nlev = 0;
-    dbuf<uint32_t> order;
-    std::vector<uint32_t> off;
+    dbuf<uint32_t> order, off;
 };
 
 void free_gs_plan(GsPlan *p) { delete p; }
@@ -472,13 +753,12 @@ static int build_gs_plan(gcg_graph *g, GsPlan &pl) {
     uint64_t *sorted = nullptr;
     GCG_TRY(radix_sort_u64(keys.get(), tmp.get(), nv, (int)g->vbits, (int)(g->vbits + 2 + lbits), &sorted, s));
     const size_t nseg = (size_t)GS_CLASSES * pl.nlev;
-    tbuf<uint32_t> doff;
-    GCG_TRY(doff.alloc(nseg + 1, s));
+    GCG_TRY(pl.off.alloc(nseg + 1));
+    GCG_CUDA(cudaMemsetAsync(pl.off.get(), 0, (nseg + 1) * 4, s));
     GCG_TRY(pl.order.alloc(nv));
-    k_level_bounds<<<vgrid(nv), 256, 0, s>>>(sorted, nv, g->vbits, (uint32_t)nseg, doff.get(), pl.order.get());
+    k_level_bounds<<<vgrid(nv), 256, 0, s>>>(sorted, nv, g->vbits, (uint32_t)nseg, pl.off.get(),
+                                         pl.order.get());
     GCG_LAUNCH_CHECK();
-    pl.off.resize(nseg + 1);
-    GCG_CUDA(cudaMemcpyAsync(pl.off.data(), doff.get(), (nseg + 1) * 4, cudaMemcpyDeviceToHost, s));
     GCG_CUDA(cudaStreamSynchronize(s));
     return GCG_OK;
 }
@@ -507,12 +787,12 @@ int pagerank_gs_exact(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
     tbuf<float> pr, val, delta;
     tbuf<double> logs; /* delta_log[nsw], res_log[nsw] */
     tbuf<double2> part;
-    tbuf<uint32_t> ctl; /* ticket, slot, done */
+    tbuf<uint32_t> ctl; /* ticket, slot, done, error, barrier arrivals */
     GCG_TRY(pr.alloc((size_t)2 * nv, s));
-    GCG_TRY(ctl.alloc(4, s));
-    GCG_CUDA(cudaMemsetAsync(ctl.get(), 0, 4 * sizeof(uint32_t), s));
+    GCG_TRY(ctl.alloc(8, s));
+    GCG_CUDA(cudaMemsetAsync(ctl.get(), 0, 8 * sizeof(uint32_t), s));
     int *done = (int *)(ctl.get() + 2);
-    float *pr_old = pr.get(), *pr_new = pr.get() + nv;
+    float *const buf[2] = {pr.get(), pr.get() + nv}; /* sweep k reads buf[k & 1], writes the other */
     const float reset = (float)p->teleport;
     if (track) {
         GCG_TRY(val.alloc(nv, s));
@@ -521,60 +801,62 @@ int pagerank_gs_exact(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
         GCG_TRY(part.alloc(DSUM_BLOCKS, s));
         k_gs_val_init<<<vgrid(nv), 256, 0, s>>>(nv, g->outdeg.get(), reset, edge ? 1 : 0, val.get());
     }
-    if (edge) k_gs_edge_init<<<vgrid(nv), 256, 0, s>>>(nv, g->outdeg.get(), pr_old);
-    else k_gs_init<<<vgrid(nv), 256, 0, s>>>(nv, g->outdeg.get(), reset, pr_old);
+    if (edge) k_gs_edge_init<<<vgrid(nv), 256, 0, s>>>(nv, g->outdeg.get(), buf[0]);
+    else k_gs_init<<<vgrid(nv), 256, 0, s>>>(nv, g->outdeg.get(), reset, buf[0]);
     GCG_LAUNCH_CHECK();
 
     cudaEvent_t ev0, ev1;
     GCG_CUDA(cudaEventCreate(&ev0));
     GCG_CUDA(cudaEventCreate(&ev1));
-    /* one sweep = all levels in order, then pr_old <- pr_new; captured once */
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    cudaStream_t cap;
-    GCG_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-    GCG_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-    for (uint32_t l = 0; l < pl.nlev; ++l) {
-        const uint32_t *o = pl.off.data() + (size_t)GS_CLASSES * l;
-        const uint32_t tb = o[0], wb = o[1], bb = o[2], be = o[3];
-        if (tb == be) continue;
-        /* blocks: one per block-class vertex, one per 8 warp-class vertices, then
-         * the thread-class vertices (grid-strided) */
-        const uint64_t nthr = wb - tb;
-        const unsigned gr = (unsigned)((be - bb) + (bb - wb + 7) / 8 + (nthr ? vgrid((uint32_t)nthr) : 0));
-        const uint32_t *rp = g->in_rowptr.get(), *cl = g->in_col.get(), *od = g->outdeg.get();
-        if (edge)
-            k_gs_level<true, true><<<gr, 256, 0, cap>>>(pl.order.get(), tb, wb, bb, be, rp, cl, od, pr_old, pr_new,
-                                                        val.get(), delta.get(), done, p->teleport, p->damping);
-        else if (track)
-            k_gs_level<false, true><<<gr, 256, 0, cap>>>(pl.order.get(), tb, wb, bb, be, rp, cl, od, pr_old, pr_new,
-                                                         val.get(), delta.get(), done, p->teleport, p->damping);
-        else
-            k_gs_level<false, false><<<gr, 256, 0, cap>>>(pl.order.get(), tb, wb, bb, be, rp, cl, od, pr_old, pr_new,
-                                                          nullptr, nullptr, done, p->teleport, p->damping);
-    }
-    if (track)
-        k_gs_delta_sum<<<DSUM_BLOCKS, 256, 0, cap>>>(delta.get(), val.get(), nv, part.get(), ctl.get(), ctl.get() + 1,
-                                                     done, p->tol, logs.get(), logs.get() + std::max(1, nsw));
-    cudaMemcpyAsync(pr_old, pr_new, (size_t)nv * 4, cudaMemcpyDeviceToDevice, cap);
-    cudaError_t ce = cudaStreamEndCapture(cap, &graph);
-    if (ce != cudaSuccess) {
-        cudaStreamDestroy(cap);
-        return fail(GCG_ERR_CUDA, std::string("sweep capture: ") + cudaGetErrorString(ce));
-    }
-    ce = cudaGraphInstantiate(&exec, graph, 0);
-    cudaStreamDestroy(cap);
-    if (ce != cudaSuccess) {
-        cudaGraphDestroy(graph);
-        return fail(GCG_ERR_CUDA, std::string("sweep graph instantiate: ") + cudaGetErrorString(ce));
-    }
+    GsArgs a{};
+    a.order = pl.order.get();
+    a.off = pl.off.get();
+    a.nlev = pl.nlev;
+    a.rowptr = g->in_rowptr.get();
+    a.col = g->in_col.get();
+    a.outdeg = g->outdeg.get();
+    a.val = val.get();
+    a.delta = delta.get();
+    a.done = done;
+    a.err = (int *)(ctl.get() + 3);
+    a.bar = ctl.get() + 4;
+    a.reset = p->teleport;
+    a.damping = p->damping;
+    const void *kern = edge    ? (const void *)k_gs_sweep<true, true>
+                       : track ? (const void *)k_gs_sweep<false, true>
+                               : (const void *)k_gs_sweep<false, false>;
+    const size_t smem = sizeof(GsGroup) * GS_GROUPS;
+    GCG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    unsigned grid = (unsigned)num_sms();
+    int queued = 0;
+    /* one cooperative launch per sweep; where fewer SMs are to be had, a smaller grid */
+    auto launch_sweep = [&]() -> int {
+        a.pr_old = buf[queued & 1];
+        a.pr_new = buf[(queued + 1) & 1];
+        void *kargs[] = {&a};
+        cudaError_t e;
+        for (;;) {
+            a.meets = (uint32_t)queued * (pl.nlev - 1) * grid;
+            e = cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(GS_THREADS), kargs, smem, s);
+            if (e != cudaErrorCooperativeLaunchTooLarge || queued || grid == 1) break;
+            cudaGetLastError();
+            grid = (grid + 1) / 2;
+        }
+        GCG_CUDA(e);
+        if (track)
+            k_gs_delta_sum<<<DSUM_BLOCKS, 256, 0, s>>>(delta.get(), val.get(), nv, part.get(), ctl.get(),
+                                                       ctl.get() + 1, done, p->tol, logs.get(),
+                                                       logs.get() + std::max(1, nsw));
+        ++queued;
+        return GCG_OK;
+    };
     /* sweeps are queued in chunks of 8; with a tolerance the host checks the
      * sweep count after each chunk (sweeps queued past convergence return at once) */
     uint32_t h_ctl[4] = {0, 0, 0, 0};
     GCG_CUDA(cudaEventRecord(ev0, s));
     for (int sw = 0; sw < nsw;) {
         const int n = std::min(8, nsw - sw);
-        for (int k = 0; k < n; ++k) GCG_CUDA(cudaGraphLaunch(exec, s));
+        for (int k = 0; k < n; ++k) GCG_TRY(launch_sweep());
         sw += n;
         if (p->tol > 0.0 && sw < nsw) {
             GCG_CUDA(cudaMemcpyAsync(h_ctl, ctl.get(), sizeof(h_ctl), cudaMemcpyDeviceToHost, s));
@@ -584,24 +866,23 @@ int pagerank_gs_exact(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
     }
     GCG_CUDA(cudaEventRecord(ev1, s));
     GCG_CUDA(cudaMemcpyAsync(h_ctl, ctl.get(), sizeof(h_ctl), cudaMemcpyDeviceToHost, s));
+    GCG_CUDA(cudaStreamSynchronize(s));
+    if (h_ctl[3]) return fail(GCG_ERR_TIMEOUT, "pagerank: a wait between the levels of a sweep ran out");
+    const int sweeps = track ? (int)h_ctl[1] : nsw;
+    float *const pr_last = buf[sweeps & 1], *const pr_out = buf[(sweeps + 1) & 1];
     if (!edge) {
-        k_gs_final<<<vgrid(nv), 256, 0, s>>>(nv, g->outdeg.get(), pr_old, pr_new);
+        k_gs_final<<<vgrid(nv), 256, 0, s>>>(nv, g->outdeg.get(), pr_last, pr_out);
         GCG_LAUNCH_CHECK();
     }
-    GCG_CUDA(cudaEventSynchronize(ev1));
-    GCG_CUDA(cudaStreamSynchronize(s));
-    const int sweeps = track ? (int)h_ctl[1] : nsw;
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, ev0, ev1);
     cudaEventDestroy(ev0);
     cudaEventDestroy(ev1);
-    cudaGraphExecDestroy(exec);
-    cudaGraphDestroy(graph);
     double last_res = 0.0;
     if (track && sweeps > 0)
         GCG_CUDA(cudaMemcpy(&last_res, logs.get() + std::max(1, nsw) + sweeps - 1, sizeof(double),
                             cudaMemcpyDeviceToHost));
-    if (out_rank) GCG_TRY(copy_out(out_rank, edge ? val.get() : pr_new, (size_t)nv * 4, s));
+    if (out_rank) GCG_TRY(copy_out(out_rank, edge ? val.get() : pr_out, (size_t)nv * 4, s));
     if (track && p->delta_log && sweeps > 0)
         GCG_TRY(copy_out(p->delta_log, logs.get(), (size_t)sweeps * sizeof(double), s));
     if (track && p->residuals && sweeps > 0)
@@ -622,7 +903,7 @@ int pagerank_gs_exact(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
         stats->device_ms = ms;
         stats->sweep_kernel_ms = ms;
         stats->timed_sweeps = sweeps;
-        stats->kernel_launches = 1 + (track ? 1 : 0) + (edge ? 0 : 1) + ((int)pl.nlev + (track ? 1 : 0)) * sweeps;
+        stats->kernel_launches = 1 + (track ? 1 : 0) + (edge ? 0 : 1) + (track ? 2 : 1) * queued;
         stats->levels = (int)pl.nlev;
     }
     return GCG_OK;
