@@ -8,20 +8,19 @@
  * in float, r_s starting at the indicator of source_s, and each source stopping
  * after its own first sweep with normalised L1 change (FP64) <= tol.
  *
- * Layout: vertex-major matrices R[V][kp], C[V][kp] (kp = k rounded up to 32, at most
+ * Layout: vertex-major matrices R[V][kp], C[V][kp] (kp = k rounded up to 8, at most
  * 256 per group; larger k run group by group), so the contribution row of a source
- * vertex is one contiguous 4*kp-byte line: a warp gathers it with one 128-bit load
- * per lane per 32 columns (fully coalesced, 1 KiB per edge at kp = 256).
- * Work: in-edge rows are cut into segments of at most 256 edges; one warp per
- * segment broadcasts the segment's source ids with shuffles, keeps four row
- * gathers in flight, and accumulates in registers (lane = 8 columns). A row of one
+ * vertex is one contiguous 4*kp-byte line, gathered with 128-bit loads by 8 or 16
+ * lanes, a slice of at most 64 columns at a time.
+ * Work: in-edge rows are cut into segments of at most 256 edges; one group of lanes
+ * per segment broadcasts the segment's source ids with shuffles, keeps eight row
+ * gathers in flight, and accumulates in registers. A row of one
  * segment is applied at once; longer rows leave per-segment partials that a
  * fix-up pass adds in segment order. Vertices without in-edges are constant after
  * the first sweep and are written only in sweeps 0 and 1. Per-column FP64
  * residuals are reduced in a fixed order. A column that converges is copied to the
  * result at that sweep (k_ppr_retire) and keeps being swept in place; when the
- * columns still iterating fit a layout at most 3/4 as wide (widths 256, 192, 128,
- * 96, 64, 32), they are compacted into it.
+ * columns still iterating fit a layout at most 3/4 as wide, they are compacted into it.
  * Algorithmic traffic per sweep: E*(4 + 4*kp) + 3*V*4*kp bytes.
  */
 #include <math.h>
@@ -41,47 +40,44 @@ constexpr uint32_t SEG = 256;     /* edges per segment */
 constexpr int PPR_THREADS = 256;  /* 8 warps */
 constexpr uint32_t KMAX = 256;    /* columns per group */
 constexpr uint32_t NONE = 0xFFFFFFFFu;
+constexpr int SEG_BLOCKS_MAX = 8; /* per SM, of the segment kernel */
 
-template <int CPL>
-__device__ __forceinline__ void load_row(const float *p, float (&x)[CPL]) {
-    if constexpr (CPL == 8) {
-        const float4 a = __ldg((const float4 *)p), b = __ldg((const float4 *)p + 1);
-        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-    } else if constexpr (CPL == 6) {
-        const float2 a = __ldg((const float2 *)p), b = __ldg((const float2 *)p + 1), c = __ldg((const float2 *)p + 2);
-        x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y; x[4] = c.x; x[5] = c.y;
-    } else if constexpr (CPL == 4) {
-        const float4 a = __ldg((const float4 *)p);
-        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
-    } else if constexpr (CPL == 3) {
-        x[0] = __ldg(p); x[1] = __ldg(p + 1); x[2] = __ldg(p + 2);
-    } else if constexpr (CPL == 2) {
-        const float2 a = __ldg((const float2 *)p);
-        x[0] = a.x; x[1] = a.y;
-    } else {
-        x[0] = __ldg(p);
-    }
+/* A matrix row of kp columns is worked on in slices of at most SLICE columns by G lanes
+ * with one float4 each (G = 16, or 8 for up to 32 columns), so a warp has two or four rows
+ * under way. The slices of a sweep come one after another: each reads the source ids
+ * again (4 bytes an edge beside 256 gathered), but the lines gathered meanwhile are a part
+ * of the matrix only. With one row per warp and its columns spread over all lanes, a load
+ * of 64 columns asked for 256 bytes, and four in flight were bound by their latency
+ * (3.8 TB/s from L2). Per sweep, before -> now: R-MAT scale 20 with 57 of 100 columns
+ * live 1.44 -> 0.44 ms (10.6 TB/s), 143 of 256 2.40 -> 1.23; scale 22, 126 of 256
+ * 6.02 -> 4.05; uniform scale 20, 256 4.44 -> 3.18. What bounds it now is L2: 70 % of
+ * its sectors hit, 17 M of 137 M come from the other die's half. */
+constexpr uint32_t SLICE = 64;
+
+/* the lanes' float4 of a row's slice; lanes past it, and rows that are off, hold zeros */
+struct RowPart {
+    float4 v;
+};
+__device__ __forceinline__ RowPart load_row(const float *row, uint32_t lanes, uint32_t gl, bool on) {
+    RowPart x;
+    x.v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (on && gl < lanes) x.v = __ldg((const float4 *)row + gl);
+    return x;
+}
+__device__ __forceinline__ void store_row(float *row, uint32_t lanes, uint32_t gl, const RowPart &x) {
+    if (gl < lanes) ((float4 *)row)[gl] = x.v;
+}
+__device__ __forceinline__ void add_row(RowPart &s, const RowPart &x) {
+    s.v.x += x.v.x;
+    s.v.y += x.v.y;
+    s.v.z += x.v.z;
+    s.v.w += x.v.w;
 }
 
-template <int CPL>
-__device__ __forceinline__ void store_row(float *p, const float (&x)[CPL]) {
-    if constexpr (CPL == 8) {
-        ((float4 *)p)[0] = make_float4(x[0], x[1], x[2], x[3]);
-        ((float4 *)p)[1] = make_float4(x[4], x[5], x[6], x[7]);
-    } else if constexpr (CPL == 6) {
-        ((float2 *)p)[0] = make_float2(x[0], x[1]);
-        ((float2 *)p)[1] = make_float2(x[2], x[3]);
-        ((float2 *)p)[2] = make_float2(x[4], x[5]);
-    } else if constexpr (CPL == 4) {
-        ((float4 *)p)[0] = make_float4(x[0], x[1], x[2], x[3]);
-    } else if constexpr (CPL == 3) {
-        p[0] = x[0]; p[1] = x[1]; p[2] = x[2];
-    } else if constexpr (CPL == 2) {
-        ((float2 *)p)[0] = make_float2(x[0], x[1]);
-    } else {
-        p[0] = x[0];
-    }
-}
+/* A slice: columns [c0, c0 + 4 lanes) */
+struct Slice {
+    uint32_t c0, lanes;
+};
 
 struct PprArgs {
     const uint32_t *col, *outdeg;
@@ -89,6 +85,7 @@ struct PprArgs {
     const uint4 *multi;      /* (row, first slot, segment count, 0) */
     const uint32_t *zero_rows;
     uint32_t nseg, nmulti, nzero, kp, k;
+    uint32_t slice;          /* columns per slice (the last may have fewer), a multiple of 8 */
     const uint32_t *src;     /* kp source ids (NONE for padding columns) */
     const float *c_old, *r_old;
     float *c_new, *r_new, *partial;
@@ -103,174 +100,235 @@ struct PprArgs {
     double teleport, damping, tol;
 };
 
+__device__ __forceinline__ Slice slice_at(const PprArgs &a, uint32_t c0) {
+    return Slice{c0, min(a.slice, a.kp - c0) >> 2};
+}
+
+/* a lane's columns of the residual's two sums, and its columns' sources */
+struct LaneColumns {
+    double d[4], n[4];
+    uint32_t src[4];
+};
+__device__ __forceinline__ void lane_columns(const PprArgs &a, Slice sl, uint32_t gl, LaneColumns &l) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        l.d[j] = l.n[j] = 0.0;
+        l.src[j] = gl < sl.lanes ? a.src[sl.c0 + 4u * gl + j] : NONE;
+    }
+}
+
 /* apply one row: r' = tele + damping*sum, c' = r'/outdeg, residual per column */
-/* apply one row: r' = tele + damping*sum, c' = r'/outdeg, residual per column */
-template <int CPL>
-__device__ __forceinline__ void ppr_apply(const PprArgs &a, uint32_t v, const float (&sum)[CPL], const uint32_t (&srcs)[CPL],
-                                          uint32_t lane, double (&dsum)[CPL], double (&nsum)[CPL]) {
-    const size_t off = (size_t)v * a.kp + (size_t)lane * CPL;
-    float ro[CPL], rn[CPL], cn[CPL];
-    load_row<CPL>(a.r_old + off, ro);
+__device__ __forceinline__ void ppr_apply(const PprArgs &a, Slice sl, uint32_t v, const RowPart &sum, uint32_t gl,
+                                          LaneColumns &l) {
+    const size_t off = (size_t)v * a.kp + sl.c0;
+    const RowPart ro = load_row(a.r_old + off, sl.lanes, gl, true);
+    RowPart rn, cn;
     const uint32_t od = a.outdeg[v];
 #pragma unroll
-    for (int j = 0; j < CPL; ++j) {
-        const double tele = srcs[j] == v ? a.teleport : 0.0;
-        rn[j] = (float)__dadd_rn(tele, __dmul_rn(a.damping, (double)sum[j]));
-        cn[j] = od ? __fdiv_rn(rn[j], (float)od) : 0.0f;
-        dsum[j] += fabs((double)rn[j] - (double)ro[j]);
-        nsum[j] += fabs((double)rn[j]);
+    for (int j = 0; j < 4; ++j) {
+        const float s = (&sum.v.x)[j], old = (&ro.v.x)[j];
+        const double tele = l.src[j] == v ? a.teleport : 0.0;
+        const float r = (float)__dadd_rn(tele, __dmul_rn(a.damping, (double)s));
+        (&rn.v.x)[j] = r;
+        (&cn.v.x)[j] = od ? __fdiv_rn(r, (float)od) : 0.0f;
+        l.d[j] += fabs((double)r - (double)old);
+        l.n[j] += fabs((double)r);
     }
-    store_row<CPL>(a.r_new + off, rn);
-    store_row<CPL>(a.c_new + off, cn);
+    store_row(a.r_new + off, sl.lanes, gl, rn);
+    store_row(a.c_new + off, sl.lanes, gl, cn);
 }
 
-/* block-level fixed-order reduction of the per-lane column residuals */
-template <int CPL>
-__device__ __forceinline__ void block_columns(const PprArgs &a, double (&dsum)[CPL], double (&nsum)[CPL],
-                                              double2 *s_part, uint32_t out_block) {
+/* the block's sums per column of a slice, in a fixed order: the groups of a warp, then
+ * the warps, then nmore partials of earlier blocks, `stride` apart */
+template <int G>
+__device__ __forceinline__ void block_columns(const PprArgs &a, Slice sl, LaneColumns &l, double2 (*s_part)[4 * G],
+                                              double2 *out, const double2 *more, uint32_t nmore, uint32_t stride) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int j = 0; j < CPL; ++j) s_part[warp * KMAX + lane * CPL + j] = make_double2(dsum[j], nsum[j]);
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int o = G; o < 32; o <<= 1) {
+            l.d[j] += __shfl_xor_sync(0xFFFFFFFFu, l.d[j], o);
+            l.n[j] += __shfl_xor_sync(0xFFFFFFFFu, l.n[j], o);
+        }
+        if (lane < sl.lanes) s_part[warp][4u * lane + j] = make_double2(l.d[j], l.n[j]);
+    }
     __syncthreads();
-    for (uint32_t c = threadIdx.x; c < a.kp; c += blockDim.x) {
+    for (uint32_t c = threadIdx.x; c < 4u * sl.lanes; c += blockDim.x) {
         double2 t = make_double2(0.0, 0.0);
         for (uint32_t w = 0; w < blockDim.x / 32; ++w) {
-            t.x += s_part[w * KMAX + c].x;
-            t.y += s_part[w * KMAX + c].y;
+            t.x += s_part[w][c].x;
+            t.y += s_part[w][c].y;
         }
-        a.bpart[(size_t)out_block * a.kp + c] = t;
+        for (uint32_t m = 0; m < nmore; ++m) {
+            const double2 x = __ldcg(more + (size_t)m * stride * a.kp + sl.c0 + c);
+            t.x += x.x;
+            t.y += x.y;
+        }
+        out[sl.c0 + c] = t;
     }
+    __syncthreads();
 }
 
-template <int CPL>
+/* One group of lanes per segment of a slice (blockIdx.y: the slices come one after
+ * another as the blocks do). The segments are sorted by length, so the groups of a warp take about
+ * the same number of steps; a group past its end loads
+ * nothing. The loads are written as they are because the rate hangs on it: as explicitly
+ * predicated loads, all eight of a step leave at once and the sweep takes 570 us instead
+ * of 440 (same sectors, same hit rates). */
+template <int G>
 __global__ void __launch_bounds__(PPR_THREADS) k_ppr_seg(PprArgs a) {
     if (*(volatile const int *)a.done) return;
-    __shared__ double2 s_part[(PPR_THREADS / 32) * KMAX];
+    __shared__ double2 s_part[PPR_THREADS / 32][4 * G];
     const uint32_t FULL = 0xFFFFFFFFu;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-    uint32_t srcs[CPL];
+    constexpr int U = 8; /* row gathers in flight per group */
+    const uint32_t lane = threadIdx.x & 31u, gl = lane % G;
+    const uint32_t gg = (blockIdx.x * blockDim.x + threadIdx.x) / G, ng = (gridDim.x * blockDim.x) / G;
+    const uint32_t wfirst = gg - lane / G; /* the warp's first group: every lane loops alike */
+    const uint32_t c0 = blockIdx.y * a.slice;
+    const Slice sl = slice_at(a, c0);
+    LaneColumns l;
+    lane_columns(a, sl, gl, l);
+    const float *c_old = a.c_old + c0;
+    for (uint32_t k0 = wfirst; k0 < a.nseg; k0 += ng) {
+        const uint32_t k = k0 + lane / G;
+        const uint4 sg = k < a.nseg ? a.seg[k] : make_uint4(0u, 0u, 0u, 0u); /* row, eb, ee, slot */
+        const uint32_t len = sg.z - sg.y, most = __reduce_max_sync(FULL, len);
+        RowPart acc;
+        acc.v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        uint32_t mine = gl < len ? __ldg(a.col + sg.y + gl) : 0u;
+        for (uint32_t e0 = 0; e0 < most; e0 += G) {
+            const uint32_t cur = mine, nx = e0 + G + gl;
+            mine = nx < len ? __ldg(a.col + sg.y + nx) : 0u;
 #pragma unroll
-    for (int j = 0; j < CPL; ++j) srcs[j] = a.src[lane * CPL + j];
-    double dsum[CPL], nsum[CPL];
+            for (int j = 0; j < G; j += U) {
+                if (e0 + j >= most) break;
+                RowPart x[U];
 #pragma unroll
-    for (int j = 0; j < CPL; ++j) dsum[j] = nsum[j] = 0.0;
-
-    for (uint32_t k = gw; k < a.nseg; k += nw) {
-        const uint4 sg = a.seg[k]; /* row, eb, ee, slot */
-        float acc[CPL];
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t w = __shfl_sync(FULL, cur, j + u, G);
+                    x[u] = load_row(c_old + (size_t)w * a.kp, sl.lanes, gl, e0 + j + u < len);
+                }
 #pragma unroll
-        for (int j = 0; j < CPL; ++j) acc[j] = 0.0f;
-        for (uint32_t e0 = sg.y; e0 < sg.z; e0 += 32u) {
-            const uint32_t n = min(32u, sg.z - e0);
-            const uint32_t mine = lane < n ? __ldg(a.col + e0 + lane) : 0u;
-            uint32_t j = 0;
-            for (; j + 4 <= n; j += 4) { /* four row gathers in flight */
-                float x0[CPL], x1[CPL], x2[CPL], x3[CPL];
-                const uint32_t u0 = __shfl_sync(FULL, mine, j), u1 = __shfl_sync(FULL, mine, j + 1);
-                const uint32_t u2 = __shfl_sync(FULL, mine, j + 2), u3 = __shfl_sync(FULL, mine, j + 3);
-                load_row<CPL>(a.c_old + (size_t)u0 * a.kp + lane * CPL, x0);
-                load_row<CPL>(a.c_old + (size_t)u1 * a.kp + lane * CPL, x1);
-                load_row<CPL>(a.c_old + (size_t)u2 * a.kp + lane * CPL, x2);
-                load_row<CPL>(a.c_old + (size_t)u3 * a.kp + lane * CPL, x3);
-#pragma unroll
-                for (int c = 0; c < CPL; ++c) acc[c] = (((acc[c] + x0[c]) + x1[c]) + x2[c]) + x3[c];
-            }
-            for (; j < n; ++j) {
-                float x0[CPL];
-                const uint32_t u0 = __shfl_sync(FULL, mine, j);
-                load_row<CPL>(a.c_old + (size_t)u0 * a.kp + lane * CPL, x0);
-#pragma unroll
-                for (int c = 0; c < CPL; ++c) acc[c] += x0[c];
+                for (int u = 0; u < U; ++u) add_row(acc, x[u]); /* past the end: + 0 */
             }
         }
-        if (sg.w == NONE) ppr_apply<CPL>(a, sg.x, acc, srcs, lane, dsum, nsum);
-        else store_row<CPL>(a.partial + (size_t)sg.w * a.kp + lane * CPL, acc);
+        if (k < a.nseg) {
+            if (sg.w == NONE) ppr_apply(a, sl, sg.x, acc, gl, l);
+            else store_row(a.partial + (size_t)sg.w * a.kp + c0, sl.lanes, gl, acc);
+        }
     }
-    block_columns<CPL>(a, dsum, nsum, s_part, blockIdx.x);
+    block_columns<G>(a, sl, l, s_part, a.bpart + (size_t)blockIdx.x * a.kp, nullptr, 0u, 0u);
 }
 
-/* rows of more than one segment (partials in segment order), the constant
- * vertices in sweeps 0 and 1, then — in the last block — the fixed-order
- * per-column residual reduction and the stopping test */
-template <int CPL>
+/* rows of more than one segment (partials in segment order, eight in flight; the rows
+ * of most segments first), the constant vertices in sweeps 0 and 1, then, in the last
+ * block, the fixed-order per-column residual reduction and the stopping test. Each
+ * block also adds its share of the segment kernel's partials, so the last block has
+ * one per block of this kernel left to add (with all of them left to one thread per
+ * column this kernel took 204 us at R-MAT scale 20, now 41). */
+template <int G>
 __global__ void __launch_bounds__(PPR_THREADS) k_ppr_fix(PprArgs a, int sweep, int const_pass) {
     if (*(volatile const int *)a.done) return;
-    __shared__ double2 s_part[(PPR_THREADS / 32) * KMAX];
+    __shared__ double2 s_part[PPR_THREADS / 32][4 * G];
     __shared__ double s_res[KMAX];
+    __shared__ int s_act[KMAX];
     __shared__ int s_last;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-    uint32_t srcs[CPL];
-#pragma unroll
-    for (int j = 0; j < CPL; ++j) srcs[j] = a.src[lane * CPL + j];
-    double dsum[CPL], nsum[CPL];
-#pragma unroll
-    for (int j = 0; j < CPL; ++j) dsum[j] = nsum[j] = 0.0;
-    for (uint32_t k = gw; k < a.nmulti; k += nw) {
+    constexpr int U = 8;
+    const uint32_t gl = threadIdx.x % G;
+    const uint32_t gg = (blockIdx.x * blockDim.x + threadIdx.x) / G, ng = (gridDim.x * blockDim.x) / G;
+    double2 *const mypart = a.bpart + (size_t)a.nbseg * a.kp;
+    const uint32_t c0 = blockIdx.y * a.slice;
+    const Slice sl = slice_at(a, c0);
+    LaneColumns l;
+    lane_columns(a, sl, gl, l);
+    for (uint32_t k = gg; k < a.nmulti; k += ng) {
         const uint4 m = a.multi[k]; /* row, first slot, count */
-        float acc[CPL], x[CPL];
-        load_row<CPL>(a.partial + (size_t)m.y * a.kp + lane * CPL, acc);
-        for (uint32_t s = 1; s < m.z; ++s) {
-            load_row<CPL>(a.partial + (size_t)(m.y + s) * a.kp + lane * CPL, x);
+        const float *part = a.partial + (size_t)m.y * a.kp + c0;
+        RowPart acc = load_row(part, sl.lanes, gl, true);
+        for (uint32_t s = 1; s < m.z; s += U) {
+            RowPart x[U];
 #pragma unroll
-            for (int c = 0; c < CPL; ++c) acc[c] += x[c];
+            for (int u = 0; u < U; ++u) x[u] = load_row(part + (size_t)(s + u) * a.kp, sl.lanes, gl, s + u < m.z);
+#pragma unroll
+            for (int u = 0; u < U; ++u) add_row(acc, x[u]);
         }
-        ppr_apply<CPL>(a, m.x, acc, srcs, lane, dsum, nsum);
+        ppr_apply(a, sl, m.x, acc, gl, l);
     }
     if (const_pass) {
-        float zero[CPL];
-#pragma unroll
-        for (int c = 0; c < CPL; ++c) zero[c] = 0.0f;
-        for (uint32_t i = gw; i < a.nzero; i += nw)
-            ppr_apply<CPL>(a, a.zero_rows[i], zero, srcs, lane, dsum, nsum);
+        RowPart zero;
+        zero.v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (uint32_t i = gg; i < a.nzero; i += ng) ppr_apply(a, sl, a.zero_rows[i], zero, gl, l);
     }
-    block_columns<CPL>(a, dsum, nsum, s_part, a.nbseg + blockIdx.x);
+    __syncwarp();
+    block_columns<G>(a, sl, l, s_part, mypart + (size_t)blockIdx.x * a.kp, a.bpart + (size_t)blockIdx.x * a.kp,
+                     blockIdx.x < a.nbseg ? (a.nbseg - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u, gridDim.x);
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+        s_last = atomicAdd(a.ticket, 1u) == gridDim.x * gridDim.y - 1;
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    const uint32_t nb = a.nbseg + gridDim.x;
-    __shared__ int s_act[KMAX];
     /* per column: residual of this sweep; a column stops after its own first
      * sweep with residual <= tol (it keeps being swept in place until the next
-     * compaction, but its answer is taken at that sweep) */
-    for (uint32_t c = threadIdx.x; c < KMAX; c += blockDim.x) {
+     * compaction, but its answer is taken at that sweep). SPLIT threads of a column
+     * add a quarter of the blocks each, in block order */
+    constexpr uint32_t SPLIT = 4;
+    for (uint32_t c0 = 0; c0 < KMAX; c0 += PPR_THREADS / SPLIT) {
+        const uint32_t c = c0 + threadIdx.x / SPLIT, part = threadIdx.x % SPLIT;
+        const bool live = c < a.k && a.col_sweeps[c] == 0;
         double x = 0.0, y = 0.0;
-        int act = 0;
-        s_res[c] = 0.0;
-        if (c < a.k && a.col_sweeps[c] == 0) {
-            for (uint32_t b = 0; b < nb; ++b) {
-                const double2 p = __ldcg(a.bpart + (size_t)b * a.kp + c);
+        if (live) {
+            const uint32_t per = (gridDim.x + SPLIT - 1) / SPLIT, b1 = min(gridDim.x, (part + 1) * per);
+#pragma unroll 8
+            for (uint32_t b = part * per; b < b1; ++b) {
+                const double2 p = __ldcg(mypart + (size_t)b * a.kp + c);
                 x += p.x;
                 y += p.y;
             }
-            if (!const_pass) y += a.norm_const[c];
-            const double res = y > 0.0 ? x / y : 0.0;
-            s_res[c] = res;
-            a.col_res[c] = res;
-            if (a.tol > 0.0 && res <= a.tol) a.col_sweeps[c] = sweep + 1;
-            else act = 1;
         }
-        s_act[c] = act;
+#pragma unroll
+        for (int o = 1; o < (int)SPLIT; o <<= 1) {
+            x += __shfl_xor_sync(0xFFFFFFFFu, x, o);
+            y += __shfl_xor_sync(0xFFFFFFFFu, y, o);
+        }
+        if (part == 0) {
+            int act = 0;
+            double res = 0.0;
+            if (live) {
+                if (!const_pass) y += a.norm_const[c];
+                res = y > 0.0 ? x / y : 0.0;
+                a.col_res[c] = res;
+                if (a.tol > 0.0 && res <= a.tol) a.col_sweeps[c] = sweep + 1;
+                else act = 1;
+            }
+            s_res[c] = res;
+            s_act[c] = act;
+        }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32u) {
         double worst = 0.0;
         int active = 0;
-        for (uint32_t c = 0; c < a.k; ++c) {
+        for (uint32_t c = threadIdx.x; c < a.k; c += 32u) {
             worst = s_res[c] > worst ? s_res[c] : worst;
             active += s_act[c];
         }
-        a.res_log[sweep] = worst;
-        *a.last_res = worst;
-        *a.sweeps_done = sweep + 1;
-        if (active == 0) *a.done = 1;
-        *a.ticket = 0u;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double w = __shfl_xor_sync(0xFFFFFFFFu, worst, o);
+            worst = w > worst ? w : worst;
+            active += __shfl_xor_sync(0xFFFFFFFFu, active, o);
+        }
+        if (threadIdx.x == 0) {
+            a.res_log[sweep] = worst;
+            *a.last_res = worst;
+            *a.sweeps_done = sweep + 1;
+            if (active == 0) *a.done = 1;
+            *a.ticket = 0u;
+        }
     }
 }
 
@@ -282,15 +340,20 @@ __global__ void __launch_bounds__(256) k_ppr_retire(const float *__restrict__ r,
                                                     size_t dpitch) {
     __shared__ uint32_t s_l[KMAX], s_g[KMAX];
     __shared__ uint32_t s_n;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32u) { /* one warp lists them, 32 columns at a time */
         uint32_t n = 0;
-        for (uint32_t c = 0; c < k; ++c)
-            if (col_sweeps[c] == sweep_done) {
-                s_l[n] = c;
-                s_g[n] = gcol[c];
-                ++n;
+        for (uint32_t c0 = 0; c0 < k; c0 += 32u) {
+            const uint32_t c = c0 + threadIdx.x;
+            const bool is = c < k && col_sweeps[c] == sweep_done;
+            const uint32_t hit = __ballot_sync(0xFFFFFFFFu, is);
+            if (is) {
+                const uint32_t at = n + __popc(hit & ((1u << threadIdx.x) - 1u));
+                s_l[at] = c;
+                s_g[at] = gcol[c];
             }
-        s_n = n;
+            n += __popc(hit);
+        }
+        if (threadIdx.x == 0) s_n = n;
     }
     __syncthreads();
     const uint32_t n = s_n;
@@ -360,6 +423,15 @@ static int ensure_ppr_plan(gcg_graph *g) {
             slot += ns;
         }
     }
+    { /* longest first (counting sort, stable): lanes of a warp share rows of equal length */
+        std::vector<uint32_t> at(SEG + 2, 0);
+        for (const uint4 &x : seg) ++at[SEG - (x.z - x.y) + 1];
+        for (uint32_t i = 1; i < SEG + 2; ++i) at[i] += at[i - 1];
+        std::vector<uint4> sorted(seg.size());
+        for (const uint4 &x : seg) sorted[at[SEG - (x.z - x.y)]++] = x;
+        seg.swap(sorted);
+        std::stable_sort(multi.begin(), multi.end(), [](const uint4 &x, const uint4 &y) { return x.z > y.z; });
+    }
     p->nseg = (uint32_t)seg.size();
     p->nmulti = (uint32_t)multi.size();
     p->nzero = (uint32_t)zero.size();
@@ -385,15 +457,16 @@ namespace {
 
 /* rank / contribution matrices of one layout width, and its per-column state */
 struct PprLayout {
-    uint32_t cpl = 0, kp = 0, k = 0;  /* columns per lane, padded width, columns in use */
+    uint32_t kp = 0, k = 0;           /* padded width, columns in use */
     dbuf<float> r, c;                 /* 2 x V x kp each (the two sweep parities) */
     dbuf<uint32_t> src, gcol;         /* kp source ids (NONE for padding); group column of each */
     dbuf<double> norm_const, col_res; /* kp */
     dbuf<int> col_sweeps;             /* kp */
-    int alloc(uint32_t nv, uint32_t cpl_) {
-        cpl = cpl_;
-        kp = 32u * cpl_;
-        const size_t mat = (size_t)nv * kp;
+    int alloc(uint32_t nv, uint32_t width) {
+        kp = width;
+        /* room for whole 32 columns: later calls, with other numbers of columns left,
+         * find these blocks in the cache */
+        const size_t mat = (size_t)nv * ((kp + 31u) & ~31u);
         if (r.alloc(2 * mat) || c.alloc(2 * mat) || src.alloc(kp) || gcol.alloc(kp) || norm_const.alloc(kp) ||
             col_res.alloc(kp) || col_sweeps.alloc(kp))
             return GCG_ERR_NOMEM;
@@ -401,38 +474,41 @@ struct PprLayout {
     }
 };
 
-/* lanes hold 1, 2, 3, 4, 6 or 8 columns: widths 32 .. 256 */
-uint32_t cpl_for(uint32_t n) {
-    return n <= 32 ? 1u : n <= 64 ? 2u : n <= 96 ? 3u : n <= 128 ? 4u : n <= 192 ? 6u : 8u;
+/* Row width: whole 32-byte sectors; above one slice whole 128-byte lines, so that the
+ * slices of a row share none (uniform scale 20, 100 columns: 104 wide 1.86 ms a sweep,
+ * 112 1.79, 128 1.59; R-MAT scale 22, 126 live: 4.21, 4.95, 4.05). Narrow rows gain
+ * nothing from whole lines (36 live as 40 or 64: 449, 460 us). */
+uint32_t width_for(uint32_t n) { return n <= SLICE ? (n + 7u) & ~7u : (n + 31u) & ~31u; }
+
+/* blocks of the segment kernel: what the SMs hold at once */
+int seg_grid(uint32_t slice) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, slice <= 32 ? k_ppr_seg<8> : k_ppr_seg<16>, PPR_THREADS,
+                                                      0) != cudaSuccess ||
+        per_sm < 1) {
+        cudaGetLastError();
+        per_sm = 1;
+    }
+    return num_sms() * std::min(per_sm, SEG_BLOCKS_MAX);
 }
 
-template <int CPL>
-void ppr_sweep(const PprArgs &a, int nbseg, int nbfix, int sw, cudaStream_t s, std::vector<cudaEvent_t> *sev) {
+void ppr_sweep(const PprArgs &a, int nbfix, int sw, cudaStream_t s, std::vector<cudaEvent_t> *sev) {
+    cudaEvent_t e0, e1;
     if (sev) {
-        cudaEvent_t e0, e1;
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
         cudaEventRecord(e0, s);
-        k_ppr_seg<CPL><<<nbseg, PPR_THREADS, 0, s>>>(a);
+    }
+    const uint32_t ns = (a.kp + a.slice - 1) / a.slice;
+    if (a.slice <= 32) k_ppr_seg<8><<<dim3(a.nbseg, ns), PPR_THREADS, 0, s>>>(a);
+    else k_ppr_seg<16><<<dim3(a.nbseg, ns), PPR_THREADS, 0, s>>>(a);
+    if (sev) {
         cudaEventRecord(e1, s);
         sev->push_back(e0);
         sev->push_back(e1);
-    } else {
-        k_ppr_seg<CPL><<<nbseg, PPR_THREADS, 0, s>>>(a);
     }
-    k_ppr_fix<CPL><<<nbfix, PPR_THREADS, 0, s>>>(a, sw, sw < 2 ? 1 : 0);
-}
-
-void ppr_sweep_any(uint32_t cpl, const PprArgs &a, int nbseg, int nbfix, int sw, cudaStream_t s,
-                   std::vector<cudaEvent_t> *sev) {
-    switch (cpl) {
-        case 1: ppr_sweep<1>(a, nbseg, nbfix, sw, s, sev); break;
-        case 2: ppr_sweep<2>(a, nbseg, nbfix, sw, s, sev); break;
-        case 3: ppr_sweep<3>(a, nbseg, nbfix, sw, s, sev); break;
-        case 4: ppr_sweep<4>(a, nbseg, nbfix, sw, s, sev); break;
-        case 6: ppr_sweep<6>(a, nbseg, nbfix, sw, s, sev); break;
-        default: ppr_sweep<8>(a, nbseg, nbfix, sw, s, sev); break;
-    }
+    if (a.slice <= 32) k_ppr_fix<8><<<dim3(nbfix, ns), PPR_THREADS, 0, s>>>(a, sw, sw < 2 ? 1 : 0);
+    else k_ppr_fix<16><<<dim3(nbfix, ns), PPR_THREADS, 0, s>>>(a, sw, sw < 2 ? 1 : 0);
 }
 
 /* columns scol[j] of src (V x kp) -> columns dcol[j] of dst (row pitch dpitch) */
@@ -463,13 +539,13 @@ int ppr_group(gcg_graph *g, const PprPlan &pl, const uint32_t *src_host, uint32_
     cudaStream_t s = g->stream;
     const uint32_t nv = g->nv;
     const int max_sweeps = p->max_sweeps;
-    const int nbseg = num_sms() * 4, nbfix = num_sms() * 2;
+    const int nbfix = num_sms() * 2;
     dbuf<float> partial, stage;
     dbuf<double2> bpart;
     dbuf<uint32_t> ctl;
     dbuf<double> dres;
     GCG_TRY(partial.alloc((size_t)std::max<uint32_t>(pl.nslots, 1) * KMAX));
-    GCG_TRY(bpart.alloc((size_t)(nbseg + nbfix) * KMAX));
+    GCG_TRY(bpart.alloc((size_t)(num_sms() * SEG_BLOCKS_MAX + nbfix) * KMAX));
     GCG_TRY(ctl.alloc(4));
     GCG_TRY(dres.alloc((size_t)max_sweeps + 1));
     /* finished columns go straight to a device output, else to a staging matrix */
@@ -487,7 +563,7 @@ int ppr_group(gcg_graph *g, const PprPlan &pl, const uint32_t *src_host, uint32_
     std::vector<double> fin_res(k, 0.0);
 
     auto lay = std::make_unique<PprLayout>();
-    GCG_TRY(lay->alloc(nv, cpl_for(k)));
+    GCG_TRY(lay->alloc(nv, width_for(k)));
     lay->k = k;
     auto upload_state = [&](PprLayout &L) -> int {
         std::vector<uint32_t> srcv(L.kp, NONE), gc(L.kp, 0u);
@@ -524,7 +600,6 @@ int ppr_group(gcg_graph *g, const PprPlan &pl, const uint32_t *src_host, uint32_
     a.nzero = pl.nzero;
     a.partial = partial.get();
     a.bpart = bpart.get();
-    a.nbseg = (uint32_t)nbseg;
     a.ticket = ctl.get();
     a.done = (int *)(ctl.get() + 1);
     a.sweeps_done = (int *)(ctl.get() + 2);
@@ -536,6 +611,8 @@ int ppr_group(gcg_graph *g, const PprPlan &pl, const uint32_t *src_host, uint32_
     auto bind = [&](PprLayout &L) {
         a.kp = L.kp;
         a.k = L.k;
+        a.slice = std::min(L.kp, SLICE);
+        a.nbseg = (uint32_t)seg_grid(a.slice);
         a.src = L.src.get();
         a.norm_const = L.norm_const.get();
         a.col_sweeps = L.col_sweeps.get();
@@ -562,7 +639,7 @@ int ppr_group(gcg_graph *g, const PprPlan &pl, const uint32_t *src_host, uint32_
             a.c_old = lay->c.get() + (size_t)(sw & 1) * mat;
             a.r_new = lay->r.get() + (size_t)((sw + 1) & 1) * mat;
             a.c_new = lay->c.get() + (size_t)((sw + 1) & 1) * mat;
-            ppr_sweep_any(lay->cpl, a, nbseg, nbfix, sw, s, time_sweeps ? &sev : nullptr);
+            ppr_sweep(a, nbfix, sw, s, time_sweeps ? &sev : nullptr);
             if (p->tol > 0.0)
                 k_ppr_retire<<<num_sms(), 256, 0, s>>>(a.r_new, lay->kp, lay->k, nv, lay->col_sweeps.get(), sw + 1,
                                                        lay->gcol.get(), res_dst, res_pitch);
@@ -582,7 +659,7 @@ int ppr_group(gcg_graph *g, const PprPlan &pl, const uint32_t *src_host, uint32_
         }
         uint32_t nact = 0;
         for (uint32_t j = 0; j < lay->k; ++j) nact += hsw[j] == 0;
-        if (sweep >= max_sweeps || 4 * 32 * cpl_for(nact) > 3 * lay->kp) continue;
+        if (sweep >= max_sweeps || 4 * width_for(nact) > 3 * lay->kp) continue;
         /* compact the columns still iterating into a narrower layout (the others
          * are already in the result) */
         GCG_CUDA(cudaMemcpyAsync(hres.data(), lay->col_res.get(), lay->k * 8, cudaMemcpyDeviceToHost, s));
@@ -601,7 +678,7 @@ int ppr_group(gcg_graph *g, const PprPlan &pl, const uint32_t *src_host, uint32_
             }
         }
         auto nxt = std::make_unique<PprLayout>();
-        GCG_TRY(nxt->alloc(nv, cpl_for(nact)));
+        GCG_TRY(nxt->alloc(nv, width_for(nact)));
         nxt->k = nact;
         const size_t nmat = (size_t)nv * nxt->kp;
         GCG_CUDA(cudaMemsetAsync(nxt->r.get(), 0, 2 * nmat * 4, s));
