@@ -24,9 +24,9 @@
  *                  M128 x N64 x K16 MMA (8 features padded to 16), layer 2 as four
  *                  K16 steps, each layer read back with tcgen05.ld; layer 3 and exp
  *                  on the FP32 pipes
- *   k_mlp_fwd_bwd  training: one sample per thread on the FP32 pipes (forward,
- *                  backward), then per-block weight gradients as small block
- *                  GEMMs over shared-memory activation tiles, one partial slot
+ *   k_mlp_fwd_bwd  training on the FP32 pipes: tiles of 128 samples, every layer and
+ *                  every weight gradient a small block GEMM over shared-memory
+ *                  operands with its outputs in registers, one partial slot
  *                  per block (no atomics: the sum order is fixed)
  *   k_mlp_adam     fixed-order sum of the block partials, Adam on the FP32 master
  *                  weights, then the BF16-rounded copy the inference reads
@@ -53,8 +53,7 @@ constexpr int NP = GCG_MLP_NPARAMS;
 /* offsets in the flat parameter vector */
 constexpr int OW1 = 0, OB1 = OW1 + NH * NIN, OW2 = OB1 + NH, OB2 = OW2 + NH * NH, OW3 = OB2 + NH, OB3 = OW3 + NH;
 static_assert(OB3 + 1 == NP, "parameter layout");
-constexpr int TRAIN_T = 128;        /* samples per training tile (one per thread) */
-constexpr int HS = NH + 1;          /* padded row stride of the activation tiles */
+constexpr int TRAIN_T = 128;        /* samples per training tile */
 
 /* round to the nearest BF16 value (ties to even), kept as a float */
 __host__ __device__ __forceinline__ float bf16r(float x) {
@@ -511,138 +510,305 @@ struct TrainArgs {
     float dscale;           /* dL/dy = dscale * (y - t): 2 / batch size */
     float *part;            /* [gridDim.x][NP + 1] gradient partials, last = sum of squared errors */
     float *yout;            /* forward only: y per sample of the batch */
+    int x_vec;              /* x is 16-byte aligned */
 };
 
-/* shared-memory layout (floats) */
-constexpr int SM_W = 0;                       /* rounded parameters [NP] */
-constexpr int SM_H1 = (NP + 3) & ~3;          /* h1 [TRAIN_T][HS] */
-constexpr int SM_H2 = SM_H1 + TRAIN_T * HS;   /* h2 */
-constexpr int SM_D2 = SM_H2 + TRAIN_T * HS;   /* dL/da2 */
-constexpr int SM_D1 = SM_D2 + TRAIN_T * HS;   /* dL/da1 */
-constexpr int SM_X = SM_D1 + TRAIN_T * HS;    /* normalised inputs [TRAIN_T][8] */
-constexpr int SM_DY = SM_X + TRAIN_T * NIN;   /* dL/dy [TRAIN_T] */
-constexpr int SM_RED = SM_DY + TRAIN_T;       /* loss reduction [TRAIN_T] */
-constexpr int SM_TOTAL = SM_RED + TRAIN_T;
+/* shared-memory layout (floats). The activations lie feature by feature, each with the
+ * tile's samples in a row of TS floats: four consecutive samples (or weights) are one
+ * 128-bit load, and the four floats of padding put eight consecutive rows on different
+ * banks */
+constexpr int TS = TRAIN_T + 4;
+constexpr int TRAIN_THREADS = 256;
+constexpr int SM_W2 = 0;                      /* W2 [j][k] */
+constexpr int SM_W2T = SM_W2 + NH * NH;       /* W2 [k][j] */
+constexpr int SM_W1T = SM_W2T + NH * NH;      /* W1 [input][j] */
+constexpr int SM_B = SM_W1T + NIN * NH;       /* b1, b2, W3, (mean, inv_std) */
+constexpr int SM_H1 = SM_B + 3 * NH + 2 * NIN; /* h1; sign bit set where layer 1 is cut off; later dL/da1 */
+constexpr int SM_D2 = SM_H1 + NH * TS;        /* dL/da2 */
+constexpr int SM_X = SM_D2 + NH * TS;         /* normalised inputs */
+constexpr int SM_YP = SM_X + NIN * TS;        /* partial y of the four feature quarters [4][TRAIN_T] */
+constexpr int SM_DY = SM_YP + 4 * TRAIN_T;    /* dL/dy */
+constexpr int SM_TOTAL = SM_DY + TRAIN_T;
 constexpr size_t TRAIN_SMEM = (size_t)SM_TOTAL * 4;
+static_assert(SM_H1 % 4 == 0 && SM_D2 % 4 == 0 && SM_X % 4 == 0 && SM_YP % 4 == 0 && SM_DY % 4 == 0, "128-bit rows");
+static_assert(2 * TRAIN_SMEM + 2048 <= 227 * 1024, "two blocks per SM");
+static_assert(NH == 64 && NIN == 8 && TRAIN_T == 128, "the threads' tiles below");
 
-/* Forward (and, with FWD_ONLY false, backward) of one training tile per
- * iteration: thread s runs sample s through the network on the FP32 pipes; the
- * weight gradients are then accumulated as block GEMMs over the tile's
- * activations: thread p owns row j = p/2 of dW2 (32 columns), of dW1 (4 columns)
- * and one bias or W3 entry. */
+__device__ __forceinline__ float &at(float4 &v, int c) { return (&v.x)[c]; }
+
+/* two FP32 FMAs in one instruction, each rounded as fmaf */
+__device__ __forceinline__ void fma2(unsigned long long &d, unsigned long long x, unsigned long long y) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(x), "l"(y));
+}
+__device__ __forceinline__ unsigned long long pair(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpair(unsigned long long x) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+    return r;
+}
+
+/* acc[s][c] = sum over k of a[k][8 samples] * b[k][4 features], k = 0 .. K - 1 in order;
+ * pa, pb point at the thread's samples and features of row 0. Samples go in pairs, as
+ * they lie in memory, through the two-wide FMA. */
+template <int K>
+__device__ __forceinline__ void tile_gemm(float (&acc)[8][4], const float *pa, const float *pb) {
+    unsigned long long p[4][4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) p[s][c] = 0ull;
+#pragma unroll 8
+    for (int k = 0; k < K; ++k) {
+        const ulonglong2 a0 = *(const ulonglong2 *)(pa + k * TS), a1 = *(const ulonglong2 *)(pa + k * TS + 64);
+        float4 b = *(const float4 *)(pb + k * NH);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const unsigned long long bb = pair(at(b, c), at(b, c));
+            fma2(p[0][c], a0.x, bb);
+            fma2(p[1][c], a0.y, bb);
+            fma2(p[2][c], a1.x, bb);
+            fma2(p[3][c], a1.y, bb);
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float2 q = unpair(p[s][c]);
+            acc[2 * s][c] = q.x;
+            acc[2 * s + 1][c] = q.y;
+        }
+}
+
+/* Forward (and, with FWD_ONLY false, backward) of one training tile of 128 samples per
+ * iteration, FP32 throughout: every layer and every weight gradient is a small block GEMM
+ * over shared-memory operands with its outputs in registers. A thread takes 8 samples
+ * (4 sg .. and 64 + 4 sg ..) x 4 features (4 fg ..) of the activations, and 4 x 4 of dW2
+ * (rows gj + 16 i, columns gk + 16 i), which stay in registers over the block's tiles;
+ * biases and W3 are added up from the activations where they arise. 1 M samples take
+ * 0.70 ms (13.3 k FMAs a sample: 0.37 ms at the FP32 rate); what bounds it is shared
+ * memory, 3.0 k quarter-warp reads per warp and tile against 1.6 k FMA cycles. With a
+ * thread per sample and one block of 128 threads per SM, a warp per scheduler, they took
+ * 2.64 ms. */
 template <bool FWD_ONLY>
-__global__ void __launch_bounds__(TRAIN_T) k_mlp_fwd_bwd(TrainArgs a) {
-    extern __shared__ float sm[];
-    float *sw = sm + SM_W, *sH1 = sm + SM_H1, *sH2 = sm + SM_H2, *sD2 = sm + SM_D2, *sD1 = sm + SM_D1,
-          *sX = sm + SM_X, *sDy = sm + SM_DY, *sRed = sm + SM_RED;
-    for (int i = threadIdx.x; i < NP; i += TRAIN_T) sw[i] = a.wb[i];
+__global__ void __launch_bounds__(TRAIN_THREADS, 2) k_mlp_fwd_bwd(TrainArgs a) {
+    extern __shared__ __align__(16) float sm[];
+    float *sW2 = sm + SM_W2, *sW2T = sm + SM_W2T, *sW1T = sm + SM_W1T, *sB = sm + SM_B, *sH1 = sm + SM_H1,
+          *sD2 = sm + SM_D2, *sX = sm + SM_X, *sYp = sm + SM_YP, *sDy = sm + SM_DY;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t sg = (warp & 1u) * 8u + (lane & 7u), fg = (warp >> 1) * 4u + (lane >> 3);
+    for (int i = tid; i < NH * NH; i += TRAIN_THREADS) {
+        const float w = a.wb[OW2 + i];
+        sW2[i] = w;
+        sW2T[(i % NH) * NH + i / NH] = w;
+    }
+    for (int i = tid; i < NH * NIN; i += TRAIN_THREADS) sW1T[(i % NIN) * NH + i / NIN] = a.wb[OW1 + i];
+    if (tid < NH) {
+        sB[tid] = a.wb[OB1 + tid];
+        sB[NH + tid] = a.wb[OB2 + tid];
+        sB[2 * NH + tid] = a.wb[OW3 + tid];
+    }
+    if (tid < 2 * NIN) sB[3 * NH + tid] = a.norm[tid];
+    const float b3 = a.wb[OB3];
     __syncthreads();
-    const float *W1 = sw + OW1, *B1 = sw + OB1, *W2 = sw + OW2, *B2 = sw + OB2, *W3 = sw + OW3;
-    const float b3 = sw[OB3];
-    const uint32_t s = threadIdx.x, p = threadIdx.x, jj = p >> 1, half = p & 1u;
-    float gW2[32], gW1[4], gA = 0.0f, gB = 0.0f, gb3 = 0.0f, loss = 0.0f;
+    const float4 b1 = *(const float4 *)(sB + 4 * fg), b2 = *(const float4 *)(sB + NH + 4 * fg),
+                 w3 = *(const float4 *)(sB + 2 * NH + 4 * fg);
+    float bias1[4] = {b1.x, b1.y, b1.z, b1.w}, bias2[4] = {b2.x, b2.y, b2.z, b2.w}, w3v[4] = {w3.x, w3.y, w3.z, w3.w};
+
+    float gW2[4][4], gW1[2] = {0.0f, 0.0f}, gB1[4], gB2[4], gW3[4], gb3 = 0.0f, loss = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 32; ++k) gW2[k] = 0.0f;
+    for (int i = 0; i < 4; ++i) {
+        gB1[i] = gB2[i] = gW3[i] = 0.0f;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) gW1[q] = 0.0f;
+        for (int k = 0; k < 4; ++k) gW2[i][k] = 0.0f;
+    }
+    const uint32_t gj = (warp & 1u) * 8u + (lane & 7u), gk = (warp >> 1) * 4u + (lane >> 3);
+
+    /* a thread's half of a sample's inputs */
+    const uint32_t xs = tid >> 1, xh = (tid & 1u) * 4u;
     const uint64_t ntiles = (a.count + TRAIN_T - 1) / TRAIN_T;
     for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint64_t i = tile * TRAIN_T + s;
-        const bool valid = i < a.count;
-        uint64_t row = 0;
-        if (valid) row = a.idx ? a.idx[a.base + i] : a.base + i;
-        float xh[NIN];
+        {
+            const uint64_t i = tile * TRAIN_T + xs;
+            float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if (i < a.count) {
+                const uint64_t row = a.idx ? a.idx[a.base + i] : a.base + i;
+                const float *src = a.x + row * NIN + xh;
+                if (a.x_vec) {
+                    const float4 q = *(const float4 *)src;
+                    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+                } else {
 #pragma unroll
-        for (int k = 0; k < NIN; ++k)
-            xh[k] = valid ? bf16r((a.x[row * NIN + k] - a.norm[k]) * a.norm[NIN + k]) : 0.0f;
+                    for (int q = 0; q < 4; ++q) v[q] = src[q];
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    v[q] = bf16r((v[q] - sB[3 * NH + xh + q]) * sB[3 * NH + NIN + xh + q]);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) sX[(xh + q) * TS + xs] = v[q];
+        }
+        __syncthreads(); /* the inputs; the previous tile's dL/da1 has been read */
+        float acc[8][4];
+        auto store = [&](float *rows) { /* the thread's 8 x 4 values, feature rows */
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float *r = rows + (4 * fg + c) * TS + 4 * sg;
+                *(float4 *)r = make_float4(acc[0][c], acc[1][c], acc[2][c], acc[3][c]);
+                *(float4 *)(r + 64) = make_float4(acc[4][c], acc[5][c], acc[6][c], acc[7][c]);
+            }
+        };
         /* layer 1 */
-        float h[NH];
-        uint64_t m1 = 0, m2 = 0;
+        tile_gemm<NIN>(acc, sX + 4 * sg, sW1T + 4 * fg);
 #pragma unroll
-        for (int j = 0; j < NH; ++j) {
-            float acc = 0.0f;
+        for (int s = 0; s < 8; ++s)
 #pragma unroll
-            for (int k = 0; k < NIN; ++k) acc = fmaf(W1[j * NIN + k], xh[k], acc);
-            acc += B1[j];
-            if (acc > 0.0f) m1 |= 1ull << j;
-            h[j] = bf16r(fmaxf(acc, 0.0f));
-            sH1[s * HS + j] = h[j];
-        }
-        /* layers 2 and 3 */
-        float y = 0.0f;
-        for (int j = 0; j < NH; ++j) {
-            float acc = 0.0f;
-#pragma unroll
-            for (int k = 0; k < NH; ++k) acc = fmaf(W2[j * NH + k], h[k], acc);
-            acc += B2[j];
-            if (acc > 0.0f) m2 |= 1ull << j;
-            const float h2 = fmaxf(acc, 0.0f);
-            sH2[s * HS + j] = h2;
-            y = fmaf(W3[j], h2, y);
-        }
-        y += b3;
-        if (FWD_ONLY) {
-            if (valid) a.yout[i] = y;
-            continue;
-        }
-        const float err = valid ? y - a.t[row] : 0.0f;
-        loss = fmaf(err, err, loss);
-        const float dy = a.dscale * err;
-        sDy[s] = dy;
-#pragma unroll
-        for (int k = 0; k < NIN; ++k) sX[s * NIN + k] = xh[k];
-        /* backward through layers 3 and 2 (h is reused for dL/dh1) */
-#pragma unroll
-        for (int k = 0; k < NH; ++k) h[k] = 0.0f;
-        for (int j = 0; j < NH; ++j) {
-            const float d2 = ((m2 >> j) & 1ull) ? dy * W3[j] : 0.0f;
-            sD2[s * HS + j] = d2;
-#pragma unroll
-            for (int k = 0; k < NH; ++k) h[k] = fmaf(W2[j * NH + k], d2, h[k]);
-        }
-#pragma unroll
-        for (int k = 0; k < NH; ++k) sD1[s * HS + k] = ((m1 >> k) & 1ull) ? h[k] : 0.0f;
+            for (int c = 0; c < 4; ++c) {
+                const float z = acc[s][c] + bias1[c];
+                acc[s][c] = z > 0.0f ? bf16r(z) : -0.0f; /* -0: cut off, adds nothing */
+            }
+        store(sH1);
         __syncthreads();
-        /* weight gradients over the tile's samples, in sample order */
-        for (int q = 0; q < TRAIN_T; ++q) {
-            const float d2 = sD2[q * HS + jj], d1 = sD1[q * HS + jj];
-            const float *h1 = sH1 + q * HS + half * 32;
+        /* layers 2 and 3 */
+        tile_gemm<NH>(acc, sH1 + 4 * sg, sW2T + 4 * fg);
+        float yp[8];
 #pragma unroll
-            for (int k = 0; k < 32; ++k) gW2[k] = fmaf(d2, h1[k], gW2[k]);
-            const float *xq = sX + q * NIN + half * 4;
+        for (int s = 0; s < 8; ++s) {
+            yp[s] = 0.0f;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) gW1[k] = fmaf(d1, xq[k], gW1[k]);
-            if (half == 0) {
-                gA += d2;                                  /* db2[jj] */
-                gB = fmaf(sDy[q], sH2[q * HS + jj], gB);   /* dW3[jj] */
+            for (int c = 0; c < 4; ++c) {
+                acc[s][c] += bias2[c];
+                yp[s] = fmaf(w3v[c], fmaxf(acc[s][c], 0.0f), yp[s]);
+            }
+            yp[s] += __shfl_xor_sync(0xFFFFFFFFu, yp[s], 8);
+            yp[s] += __shfl_xor_sync(0xFFFFFFFFu, yp[s], 16);
+        }
+        if (lane < 8u) {
+            float *p = sYp + (warp >> 1) * TRAIN_T + 4 * sg;
+            *(float4 *)p = make_float4(yp[0], yp[1], yp[2], yp[3]);
+            *(float4 *)(p + 64) = make_float4(yp[4], yp[5], yp[6], yp[7]);
+        }
+        __syncthreads();
+        if (tid < TRAIN_T) { /* one thread per sample */
+            const uint64_t i = tile * TRAIN_T + tid;
+            const float y = (sYp[tid] + sYp[TRAIN_T + tid]) + (sYp[2 * TRAIN_T + tid] + sYp[3 * TRAIN_T + tid]) + b3;
+            if (FWD_ONLY) {
+                if (i < a.count) a.yout[i] = y;
             } else {
-                gA += d1;                                  /* db1[jj] */
-                if (p == 1) gb3 += sDy[q];
+                float err = 0.0f;
+                if (i < a.count) err = y - a.t[a.idx ? a.idx[a.base + i] : a.base + i];
+                loss = fmaf(err, err, loss);
+                const float dy = a.dscale * err;
+                gb3 += dy;
+                sDy[tid] = dy;
             }
         }
+        if (FWD_ONLY) continue; /* the next tile's inputs meet the barrier above first */
         __syncthreads();
+        /* backward through layer 3 */
+        float4 dya = *(const float4 *)(sDy + 4 * sg), dyb = *(const float4 *)(sDy + 64 + 4 * sg);
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            const float dy = s < 4 ? at(dya, s & 3) : at(dyb, s & 3);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float z = acc[s][c], d2 = z > 0.0f ? dy * w3v[c] : 0.0f;
+                gW3[c] = fmaf(dy, fmaxf(z, 0.0f), gW3[c]);
+                gB2[c] += d2;
+                acc[s][c] = d2;
+            }
+        }
+        store(sD2);
+        __syncthreads();
+        /* dL/dh1 (through layer 2), cut off where layer 1 was */
+        tile_gemm<NH>(acc, sD2 + 4 * sg, sW2 + 4 * fg);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float4 ha = *(const float4 *)(sH1 + (4 * fg + c) * TS + 4 * sg),
+                         hb = *(const float4 *)(sH1 + (4 * fg + c) * TS + 64 + 4 * sg);
+            const float h[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                if (__float_as_uint(h[s]) >> 31) acc[s][c] = 0.0f;
+                gB1[c] += acc[s][c];
+            }
+        }
+        /* dW2 over the tile's samples, in sample order */
+#pragma unroll 2
+        for (int s = 0; s < TRAIN_T; s += 4) {
+            float4 d[4], h[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                d[i] = *(const float4 *)(sD2 + (gj + 16 * i) * TS + s);
+                h[i] = *(const float4 *)(sH1 + (gk + 16 * i) * TS + s);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) gW2[i][k] = fmaf(at(d[i], q), at(h[k], q), gW2[i][k]);
+        }
+        __syncthreads(); /* h1 has been read */
+        store(sH1);      /* dL/da1 */
+        __syncthreads();
+        { /* dW1: row tid / 4, inputs 2 (tid % 4) and the next */
+            const float *d = sH1 + (tid >> 2) * TS, *x0 = sX + 2 * (tid & 3u) * TS, *x1 = x0 + TS;
+#pragma unroll 4
+            for (int s = 0; s < TRAIN_T; s += 4) {
+                float4 q = *(const float4 *)(d + s), u0 = *(const float4 *)(x0 + s), u1 = *(const float4 *)(x1 + s);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    gW1[0] = fmaf(at(q, i), at(u0, i), gW1[0]);
+                    gW1[1] = fmaf(at(q, i), at(u1, i), gW1[1]);
+                }
+            }
+        }
+        __syncthreads(); /* the inputs have been read */
     }
     if (FWD_ONLY) return;
     float *out = a.part + (size_t)blockIdx.x * (NP + 1);
 #pragma unroll
-    for (int k = 0; k < 32; ++k) out[OW2 + jj * NH + half * 32 + k] = gW2[k];
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) out[OW1 + jj * NIN + half * 4 + k] = gW1[k];
-    if (half == 0) {
-        out[OB2 + jj] = gA;
-        out[OW3 + jj] = gB;
-    } else {
-        out[OB1 + jj] = gA;
-        if (p == 1) out[OB3] = gb3;
-    }
-    /* sum of squared errors: fixed tree over the block */
-    sRed[p] = loss;
+        for (int k = 0; k < 4; ++k) out[OW2 + (gj + 16 * i) * NH + gk + 16 * k] = gW2[i][k];
+    out[OW1 + (tid >> 2) * NIN + 2 * (tid & 3u)] = gW1[0];
+    out[OW1 + (tid >> 2) * NIN + 2 * (tid & 3u) + 1] = gW1[1];
+    /* biases, W3: the 16 sample groups' parts in order; b3 and the loss over the samples */
+    float *red = sH1;
     __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        red[(0 * 16 + sg) * NH + 4 * fg + c] = gB1[c];
+        red[(1 * 16 + sg) * NH + 4 * fg + c] = gB2[c];
+        red[(2 * 16 + sg) * NH + 4 * fg + c] = gW3[c];
+    }
+    if (tid < TRAIN_T) {
+        sYp[tid] = loss;
+        sYp[TRAIN_T + tid] = gb3;
+    }
+    __syncthreads();
+    if (tid < 3 * NH) {
+        const int which = tid / NH, j = tid % NH;
+        float s = 0.0f;
+        for (int g = 0; g < 16; ++g) s += red[(which * 16 + g) * NH + j];
+        out[(which == 0 ? OB1 : which == 1 ? OB2 : OW3) + j] = s;
+    }
     for (int w = TRAIN_T / 2; w > 0; w >>= 1) {
-        if ((int)p < w) sRed[p] += sRed[p + w];
+        if ((int)tid < w) {
+            sYp[tid] += sYp[tid + w];
+            sYp[TRAIN_T + tid] += sYp[TRAIN_T + tid + w];
+        }
         __syncthreads();
     }
-    if (p == 0) out[NP] = sRed[0];
+    if (tid == 0) {
+        out[NP] = sYp[0];
+        out[OB3] = sYp[TRAIN_T];
+    }
 }
 
 struct AdamArgs {
@@ -663,6 +829,7 @@ __global__ void k_mlp_adam(AdamArgs a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < NP) {
         float gsum = 0.0f;
+#pragma unroll 16
         for (uint32_t b = 0; b < a.nblocks; ++b) gsum += a.part[(size_t)b * (NP + 1) + i];
         if (a.grad_out) a.grad_out[i] = gsum;
         if (a.apply) {
@@ -676,6 +843,7 @@ __global__ void k_mlp_adam(AdamArgs a) {
         }
     } else if (i == NP && a.loss_acc) {
         double l = 0.0;
+#pragma unroll 16
         for (uint32_t b = 0; b < a.nblocks; ++b) l += (double)a.part[(size_t)b * (NP + 1) + NP];
         *a.loss_acc += l;
     }
@@ -729,7 +897,7 @@ int stage_in(const T *user, size_t n, tbuf<T> &tmp, const T **dev, cudaStream_t 
 
 int train_grid(uint64_t count) {
     const uint64_t ntiles = (count + TRAIN_T - 1) / TRAIN_T;
-    return (int)std::max<uint64_t>(1, std::min<uint64_t>(ntiles, (uint64_t)num_sms()));
+    return (int)std::max<uint64_t>(1, std::min<uint64_t>(ntiles, 2ull * num_sms())); /* two blocks per SM */
 }
 
 int set_train_smem() {
@@ -917,11 +1085,12 @@ int gcg_mlp_forward(const gcg_mlp *m, const float *x, uint64_t n, float *y) {
     TrainArgs a;
     memset(&a, 0, sizeof(a));
     a.x = xd;
+    a.x_vec = ((uintptr_t)xd & 15u) == 0;
     a.count = n;
     a.wb = m->wb.get();
     a.norm = m->norm.get();
     a.yout = yd;
-    k_mlp_fwd_bwd<true><<<train_grid(n), TRAIN_T, TRAIN_SMEM, s>>>(a);
+    k_mlp_fwd_bwd<true><<<train_grid(n), TRAIN_THREADS, TRAIN_SMEM, s>>>(a);
     GCG_LAUNCH_CHECK();
     if (!dev) GCG_TRY(copy_out(y, yd, (size_t)n * 4, s));
     GCG_CUDA(cudaStreamSynchronize(s));
@@ -945,13 +1114,14 @@ int gcg_mlp_gradient(const gcg_mlp *m, const float *x, const float *t, uint64_t 
     TrainArgs a;
     memset(&a, 0, sizeof(a));
     a.x = xd;
+    a.x_vec = ((uintptr_t)xd & 15u) == 0;
     a.t = td;
     a.count = n;
     a.wb = m->wb.get();
     a.norm = m->norm.get();
     a.dscale = (float)(2.0 / (double)n);
     a.part = part.get();
-    k_mlp_fwd_bwd<false><<<grid, TRAIN_T, TRAIN_SMEM, s>>>(a);
+    k_mlp_fwd_bwd<false><<<grid, TRAIN_THREADS, TRAIN_SMEM, s>>>(a);
     AdamArgs d;
     memset(&d, 0, sizeof(d));
     d.part = part.get();
@@ -1020,6 +1190,7 @@ int gcg_mlp_train(gcg_mlp *m, const float *x, const float *t, uint64_t n, const 
             TrainArgs a;
             memset(&a, 0, sizeof(a));
             a.x = xd;
+            a.x_vec = ((uintptr_t)xd & 15u) == 0;
             a.t = td;
             a.idx = idx.get();
             a.base = b0;
@@ -1029,7 +1200,7 @@ int gcg_mlp_train(gcg_mlp *m, const float *x, const float *t, uint64_t n, const 
             a.dscale = (float)(2.0 / (double)cnt);
             a.part = part.get();
             const int gb = train_grid(cnt);
-            k_mlp_fwd_bwd<false><<<gb, TRAIN_T, TRAIN_SMEM, s>>>(a);
+            k_mlp_fwd_bwd<false><<<gb, TRAIN_THREADS, TRAIN_SMEM, s>>>(a);
             ++m->step;
             AdamArgs d;
             memset(&d, 0, sizeof(d));
