@@ -28,17 +28,36 @@ struct ScanInfo {
     uint32_t bad;
 };
 
-__global__ void k_scan_edges(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, uint64_t m,
-                             uint32_t nv_limit, ScanInfo *info) {
+/* Four edges per thread and step where the arrays allow 16-byte loads (a caller's
+ * device pointers need not), the block's result in three atomics: one set per
+ * warp made the atomics on the one ScanInfo what bounded it (1 M edges: 46 ->
+ * 5.5 us; 67 M: 164 -> 79). */
+__device__ __forceinline__ bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
+
+__global__ void __launch_bounds__(256) k_scan_edges(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst,
+                                                    uint64_t m, uint32_t nv_limit, ScanInfo *info) {
+    __shared__ uint32_t s_mx[8], s_bad[8];
+    __shared__ unsigned long long s_kept[8];
     uint32_t mx = 0, bad = 0;
     unsigned long long kept = 0;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t s = src[i], d = dst[i];
-        if (s == d) continue; /* sharder.hpp:428-431: self-loops never reach max_vertex_id */
+    auto edge = [&](uint32_t s, uint32_t d) {
+        if (s == d) return; /* sharder.hpp:428-431: self-loops never reach max_vertex_id */
         ++kept;
         mx = max(mx, max(s, d));
         if (nv_limit && (s >= nv_limit || d >= nv_limit)) bad = 1;
+    };
+    const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t m4 = aligned16(src) && aligned16(dst) ? m / 4 : 0;
+#pragma unroll 2
+    for (uint64_t i = i0; i < m4; i += step) {
+        const uint4 s = __ldg(reinterpret_cast<const uint4 *>(src) + i);
+        const uint4 d = __ldg(reinterpret_cast<const uint4 *>(dst) + i);
+        edge(s.x, d.x);
+        edge(s.y, d.y);
+        edge(s.z, d.z);
+        edge(s.w, d.w);
     }
+    for (uint64_t i = 4 * m4 + i0; i < m; i += step) edge(src[i], dst[i]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         mx = max(mx, __shfl_down_sync(0xFFFFFFFFu, mx, o));
@@ -46,6 +65,17 @@ __global__ void k_scan_edges(const uint32_t *__restrict__ src, const uint32_t *_
         bad |= __shfl_down_sync(0xFFFFFFFFu, bad, o);
     }
     if ((threadIdx.x & 31) == 0) {
+        s_mx[threadIdx.x >> 5] = mx;
+        s_kept[threadIdx.x >> 5] = kept;
+        s_bad[threadIdx.x >> 5] = bad;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) {
+            mx = max(mx, s_mx[w]);
+            kept += s_kept[w];
+            bad |= s_bad[w];
+        }
         if (kept) atomicAdd(&info->kept, kept);
         if (mx) atomicMax(&info->maxid, mx);
         if (bad) atomicOr(&info->bad, 1u);
@@ -66,6 +96,67 @@ __global__ void k_make_keys(const uint32_t *__restrict__ src, const uint32_t *__
         if (outcnt && !self) {
             atomicAdd(outcnt + s, 1u);
             if (sym) atomicAdd(outcnt + d, 1u);
+        }
+    }
+}
+
+/* The same with the digit counts of the sort's passes, which would otherwise cost
+ * a read of the keys (67 M edges: 204 + 184 us -> 215). */
+__global__ void __launch_bounds__(RadixCounter::THREADS) k_make_keys_count(
+    const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, uint64_t m, uint32_t vbits, int sym,
+    uint64_t *__restrict__ keys, RadixPlan pl, uint32_t *__restrict__ counts) {
+    __shared__ RadixCounter cnt;
+    cnt.clear();
+    const uint64_t sent = (vbits >= 32) ? ~0ull : ((1ull << (2 * vbits)) - 1ull);
+    constexpr int ITEMS = 4;
+    constexpr uint64_t CH = (uint64_t)RadixCounter::THREADS * ITEMS;
+    for (uint64_t c0 = blockIdx.x * CH; c0 < m; c0 += gridDim.x * CH) {
+        uint64_t s[ITEMS], d[ITEMS];
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            const uint64_t i = c0 + (uint64_t)j * RadixCounter::THREADS + threadIdx.x;
+            s[j] = i < m ? __ldg(src + i) : 0u;
+            d[j] = i < m ? __ldg(dst + i) : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            const uint64_t i = c0 + (uint64_t)j * RadixCounter::THREADS + threadIdx.x;
+            if (i >= m) break;
+            const bool self = s[j] == d[j];
+            const uint64_t k = self ? sent : ((d[j] << vbits) | s[j]);
+            keys[i] = k;
+            cnt.add(pl, k);
+            if (sym) {
+                const uint64_t r = self ? sent : ((s[j] << vbits) | d[j]);
+                keys[m + i] = r;
+                cnt.add(pl, r);
+            }
+        }
+    }
+    cnt.flush(pl, counts);
+}
+
+/* Raw out-degrees from keys in the order of their sources: a warp adds each run of
+ * one source among its 32 keys at once. Sentinels (self-loops) do not count. */
+__global__ void __launch_bounds__(256) k_src_runs(const uint64_t *__restrict__ keys, uint64_t n, uint32_t vbits,
+                                                  uint32_t *__restrict__ outdeg) {
+    constexpr int ITEMS = 8;
+    const uint64_t sent = (vbits >= 32) ? ~0ull : ((1ull << (2 * vbits)) - 1ull);
+    const uint32_t mask = (uint32_t)((1ull << vbits) - 1ull), lane = threadIdx.x & 31u;
+    const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5, i0 = w * (32 * ITEMS) + lane;
+    uint64_t k[ITEMS];
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) k[j] = i0 + j * 32 < n ? __ldg(keys + i0 + j * 32) : sent;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const uint32_t u = (uint32_t)k[j] & mask, before = __shfl_up_sync(0xFFFFFFFFu, u, 1);
+        const uint32_t heads = __ballot_sync(0xFFFFFFFFu, lane == 0 || u != before);
+        const uint32_t real = __ballot_sync(0xFFFFFFFFu, k[j] != sent);
+        if ((heads >> lane) & 1u) {
+            const uint32_t after = heads & (0xFFFFFFFEu << lane); /* the next run's first lane */
+            const uint32_t run = (after ? (after & (0u - after)) - 1u : 0xFFFFFFFFu) & (0xFFFFFFFFu << lane);
+            const uint32_t c = __popc(run & real);
+            if (c) atomicAdd(outdeg + u, c);
         }
     }
 }
@@ -130,64 +221,107 @@ __global__ void __launch_bounds__(1024) k_outdeg_hist(const uint32_t *__restrict
     extern __shared__ uint32_t s_cnt[];
     for (uint32_t i = threadIdx.x; i < win; i += blockDim.x) s_cnt[i] = 0;
     __syncthreads();
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t u = col[i];
-        if (u < win) atomicAdd(s_cnt + u, 1u);
-        else atomicAdd(outdeg + u, 1u);
+    constexpr int U = 8; /* loads in flight per thread */
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += U * step) {
+        uint32_t u[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) u[k] = i + k * step < n ? __ldg(col + i + k * step) : 0xFFFFFFFFu;
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            if (u[k] == 0xFFFFFFFFu) continue; /* past the end: ids stay below 2^32 - 2^26 */
+            if (u[k] < win) atomicAdd(s_cnt + u[k], 1u);
+            else atomicAdd(outdeg + u[k], 1u);
+        }
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < win; i += blockDim.x)
         if (s_cnt[i]) atomicAdd(outdeg + i, s_cnt[i]);
 }
 
-/* largest r in [0, nv) with rowptr[r] <= x (the non-empty row holding edge x);
- * called by a whole warp: 32 probes per step, about log32(nv) dependent loads */
-__device__ uint32_t row_of(const uint32_t *rowptr, uint32_t nv, uint32_t x) {
+/* largest r in [lo, hi) with rowptr[r] <= x, given rowptr[lo] <= x: the row that
+ * holds edge x, when it is not empty. at = rowptr[r], after = rowptr[r + 1]. Called
+ * by a whole warp: 32 probes per step until at most 31 rows are left, whose
+ * pointers the lanes load together. */
+__device__ uint32_t row_of(const uint32_t *__restrict__ rowptr, uint32_t lo, uint32_t hi, uint32_t x, uint32_t &at,
+                           uint32_t &after) {
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t lo = 0, hi = nv; /* answer in [lo, hi) */
-    while (hi - lo > 1) {
+    while (hi - lo > 31) {
         const uint32_t step = (hi - lo + 31) / 32;
         const uint32_t probe = lo + lane * step; /* probe 0 is lo itself, and rowptr[lo] <= x */
-        const bool ok = probe < hi && rowptr[probe] <= x;
+        const bool ok = probe < hi && __ldg(rowptr + probe) <= x;
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, ok) | 1u;
         const uint32_t nlo = lo + (31u - __clz(m)) * step; /* the largest probe <= x */
         hi = nlo + step < hi ? nlo + step : hi;
         lo = nlo;
     }
-    return lo;
+    const uint32_t n = hi - lo; /* rowptr ascends: the rows with rowptr <= x come first */
+    const uint32_t v = lane <= n ? __ldg(rowptr + lo + lane) : 0xFFFFFFFFu;
+    const uint32_t c = __popc(__ballot_sync(0xFFFFFFFFu, lane < n && v <= x));
+    at = __shfl_sync(0xFFFFFFFFu, v, c - 1u);
+    after = __shfl_sync(0xFFFFFFFFu, v, c);
+    return lo + c - 1u;
 }
 
-/* One warp: the k-way merge sink's interval cuts (sharder.hpp:861-892, :962).
- * Every lane follows the same cuts (the searches are warp-wide); lane 0 writes. */
-__global__ void k_intervals(const uint32_t *__restrict__ rowptr, uint32_t nv, uint32_t P, uint32_t *last,
-                            uint32_t *count) {
-    if (blockIdx.x != 0 || threadIdx.x >= 32) return;
-    const bool lead = threadIdx.x == 0;
-    const uint64_t E = rowptr[nv];
-    const uint32_t max_vid = nv - 1;
+/* One block: the k-way merge sink's interval cuts (sharder.hpp:861-892, :962).
+ * Each cut depends on the one before, so what counts is the time of one search
+ * by one warp. A table of every stride-th row pointer in shared memory, filled by
+ * the whole block, replaces most of its dependent loads, and the last load brings
+ * the cut with it (64 shards: 107 -> 55 us at 64 K vertices, 159 -> 89 at
+ * 4 M, against two searches of 4 or 5 dependent loads per cut). */
+constexpr uint32_t IV_TABLE = 16384;
+__global__ void __launch_bounds__(1024) k_intervals(const uint32_t *__restrict__ rowptr, uint32_t nv, uint32_t P,
+                                                    uint32_t *last, uint32_t *count) {
+    extern __shared__ uint32_t s_tab[];
+    const uint32_t E = rowptr[nv], max_vid = nv - 1;
     if (E == 0 || P <= 1) {
-        if (lead) {
+        if (threadIdx.x == 0) {
             last[0] = max_vid;
             *count = 1;
         }
         return;
     }
-    uint64_t eps = E / P + 1, base = 0;
+    const uint32_t stride = (uint32_t)(((uint64_t)nv + IV_TABLE - 1) / IV_TABLE), nt = (nv - 1) / stride + 1;
+#pragma unroll 8
+    for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) s_tab[i] = __ldg(rowptr + (uint64_t)i * stride);
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    auto slot = [&](uint32_t x) { /* the last table entry <= x */
+        uint32_t lo = 0, hi = nt;
+        while (hi - lo > 1) {
+            const uint32_t step = (hi - lo + 31) / 32, probe = lo + lane * step;
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, probe < hi && s_tab[probe] <= x) | 1u;
+            lo += (31u - __clz(m)) * step;
+            hi = lo + step < hi ? lo + step : hi;
+        }
+        return lo;
+    };
+    if (threadIdx.x >= 32) return;
+    /* every lane of warp 0 follows the same cuts; lane 0 writes */
+    uint32_t at, after;
+    auto find = [&](uint32_t x) {
+        const uint32_t lo = slot(x);
+        const uint64_t end = ((uint64_t)lo + 1) * stride;
+        return row_of(rowptr, lo * stride, end < nv ? (uint32_t)end : nv, x, at, after);
+    };
+    uint32_t eps = E / P + 1, base = 0;
     uint32_t shard = 0;
     while (shard < P - 1) {
-        uint64_t target = base + (eps > 0 ? eps : 1);
+        const uint64_t target = (uint64_t)base + (eps > 0 ? eps : 1);
         if (target >= E) break;
-        uint32_t r = row_of(rowptr, nv, (uint32_t)target);
-        uint64_t j = (rowptr[r] == target) ? target : (uint64_t)rowptr[r + 1];
+        const uint32_t r = find((uint32_t)target);
+        /* the cut falls before row r or, when target is inside it, after it */
+        const bool before = at == target;
+        const uint32_t j = before ? at : after;
         if (j >= E) break;
-        const uint32_t cut = row_of(rowptr, nv, (uint32_t)(j - 1));
-        if (lead) last[shard] = cut;
+        const uint32_t cut = before ? find(j - 1) : r;
+        if (lane == 0) last[shard] = cut;
         ++shard;
         eps = (E - j) / (P - shard);
         base = j;
     }
-    const uint32_t fin = (shard == P - 1) ? max_vid : row_of(rowptr, nv, (uint32_t)(E - 1));
-    if (lead) {
+    const uint32_t fin = (shard == P - 1) ? max_vid : find(E - 1);
+    if (lane == 0) {
         last[shard] = fin;
         *count = shard + 1;
     }
@@ -234,6 +368,11 @@ namespace {
 
 constexpr uint64_t PIPE_MIN_EDGES = 1ull << 24;
 constexpr int PIPE_CHUNKS = 16; /* a power of two: runs merge in equal pairs */
+
+/* one full wave of k_scan_edges (8 blocks an SM) at most, 8 edges per thread at least */
+unsigned scan_grid(uint64_t m) {
+    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((m + 2047) / 2048, (uint64_t)num_sms() * 8));
+}
 
 uint32_t id_bits(uint32_t maxid) {
     uint32_t b = 1;
@@ -310,7 +449,7 @@ int sort_host_edges(const uint32_t *src_u, const uint32_t *dst_u, uint64_t m, bo
         }
         cudaEventRecord(ev_copy[i], cs);
         cudaStreamWaitEvent(ss, ev_copy[i], 0);
-        if (cn) k_scan_edges<<<grid_for(cn), 256, 0, ss>>>(sbuf + c0, dbuf_ + c0, cn, nv_given, d_info.get() + i);
+        if (cn) k_scan_edges<<<scan_grid(cn), 256, 0, ss>>>(sbuf + c0, dbuf_ + c0, cn, nv_given, d_info.get() + i);
         cudaMemcpyAsync(h_info + i, d_info.get() + i, sizeof(ScanInfo), cudaMemcpyDeviceToHost, ss);
         cudaEventRecord(ev_scan[i], ss);
     }
@@ -432,7 +571,7 @@ int build_graph(const uint32_t *src_u, const uint32_t *dst_u, uint64_t m, uint32
         GCG_TRY(d_info.alloc(1, s));
         GCG_CUDA(cudaMemsetAsync(d_info.get(), 0, sizeof(ScanInfo), s));
         if (m > 0) {
-            k_scan_edges<<<grid_for(m), 256, 0, s>>>(src, dst, m, nv_given, d_info.get());
+            k_scan_edges<<<scan_grid(m), 256, 0, s>>>(src, dst, m, nv_given, d_info.get());
             GCG_LAUNCH_CHECK();
         }
         GCG_CUDA(cudaMemcpyAsync(&info, d_info.get(), sizeof(info), cudaMemcpyDeviceToHost, s));
@@ -466,14 +605,44 @@ int build_graph(const uint32_t *src_u, const uint32_t *dst_u, uint64_t m, uint32
     uint64_t ne = 0;
     if (g->in_rowptr.alloc((size_t)nv + 1) || g->in_col.alloc(kept) || g->indeg.alloc(nv) || g->outdeg.alloc(nv))
         return cleanup(GCG_ERR_NOMEM);
+    uint32_t *outdeg_raw = outcnt.get() && !want_out ? outcnt.get() : nullptr; /* counted already, with repeats */
     {
         int st = GCG_OK;
         if (!pipelined && nk > 0) {
             if (keys.alloc(nk, s) || tmp.alloc(nk, s)) return cleanup(GCG_ERR_NOMEM);
-            k_make_keys<<<grid_for(m), 256, 0, s>>>(src, dst, m, vbits, sym ? 1 : 0, keys.get(), nullptr);
+            /* Without an out-CSR the out-degrees are counted while the keys are in the
+             * order of their sources, if a pass may end there without adding one. The
+             * alternative, a histogram of the columns, is bound by the global atomics
+             * (64 M edges: 590 us; runs of one source: 143). */
+            RadixPlan pl = radix_plan(0, 2 * (int)vbits);
+            const RadixPlan half = radix_plan(0, (int)vbits);
+            const bool runs_of_src = !want_out && 2 * half.npass == pl.npass;
+            if (runs_of_src)
+                for (int p = 0; p < pl.npass; ++p) {
+                    pl.shift[p] = (uint8_t)(half.shift[p % half.npass] + (p < half.npass ? 0u : vbits));
+                    pl.bits[p] = half.bits[p % half.npass];
+                }
+            tbuf<uint32_t> counts;
+            if (counts.alloc(RadixPlan::MAX_PASSES * 256, s)) return cleanup(GCG_ERR_NOMEM);
+            cudaMemsetAsync(counts.get(), 0, RadixPlan::MAX_PASSES * 256 * 4, s);
+            k_make_keys_count<<<(unsigned)std::min<uint64_t>((m + 2047) / 2048, (uint64_t)num_sms() * 4),
+                                RadixCounter::THREADS, 0, s>>>(src, dst, m, vbits, sym ? 1 : 0, keys.get(), pl,
+                                                               counts.get());
             if (cudaGetLastError() != cudaSuccess) return cleanup(fail(GCG_ERR_CUDA, "k_make_keys launch"));
-            st = radix_sort_u64(keys.get(), tmp.get(), nk, 0, 2 * (int)vbits, &sorted, s);
+            const int cut = runs_of_src ? half.npass : pl.npass;
+            uint64_t *by_src = nullptr;
+            st = radix_passes(keys.get(), tmp.get(), nk, pl, 0, cut, counts.get(), &by_src, s);
             if (st) return cleanup(st);
+            sorted = by_src;
+            if (runs_of_src) {
+                cudaMemsetAsync(g->outdeg.get(), 0, (size_t)nv * 4, s);
+                k_src_runs<<<(unsigned)((nk + 2047) / 2048), 256, 0, s>>>(by_src, nk, vbits, g->outdeg.get());
+                if (cudaGetLastError() != cudaSuccess) return cleanup(fail(GCG_ERR_CUDA, "k_src_runs launch"));
+                outdeg_raw = g->outdeg.get();
+                st = radix_passes(by_src, by_src == keys.get() ? tmp.get() : keys.get(), nk, pl, cut, pl.npass,
+                                  counts.get(), &sorted, s);
+                if (st) return cleanup(st);
+            }
             runs.p[0] = sorted;
             runs.n[0] = nk;
         }
@@ -483,7 +652,7 @@ int build_graph(const uint32_t *src_u, const uint32_t *dst_u, uint64_t m, uint32
                                                                                                       : keys.get();
         st = merge_unique_csr(runs.p[0], runs.n[0], runs.p[1], runs.n[1], kept, (flags & GCG_BUILD_DEDUP) != 0,
                               kbits, nv, g->in_rowptr.get(), g->in_col.get(), kept_keys,
-                              outcnt.get() && !want_out ? outcnt.get() : nullptr, &ne, s);
+                              outdeg_raw, &ne, s);
         if (st) return cleanup(st);
         sorted = kept_keys;
     }
@@ -511,7 +680,7 @@ int build_graph(const uint32_t *src_u, const uint32_t *dst_u, uint64_t m, uint32
         const size_t have = std::min<size_t>(nv, outcnt.n);
         if (have < nv) cudaMemsetAsync(g->outdeg.get() + have, 0, (nv - have) * 4, s);
         cudaMemcpyAsync(g->outdeg.get(), outcnt.get(), have * 4, cudaMemcpyDeviceToDevice, s);
-    } else {
+    } else if (!outdeg_raw) {
         cudaMemsetAsync(g->outdeg.get(), 0, (size_t)nv * 4, s);
         if (ne > 0) {
             /* sources are the low halves of the sorted keys; take them from in_col */
@@ -528,7 +697,11 @@ int build_graph(const uint32_t *src_u, const uint32_t *dst_u, uint64_t m, uint32
     uint32_t P = nshards ? nshards : 1;
     tbuf<uint32_t> d_count;
     if (g->intervals_dev.alloc(P) || d_count.alloc(1, s)) return cleanup(GCG_ERR_NOMEM);
-    k_intervals<<<1, 32, 0, s>>>(g->in_rowptr.get(), nv, P, g->intervals_dev.get(), d_count.get());
+    const uint32_t iv_rows = P > 1 ? std::min<uint32_t>(nv, IV_TABLE) : 1;
+    if (cudaFuncSetAttribute(k_intervals, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(IV_TABLE * 4)) !=
+        cudaSuccess)
+        return cleanup(fail(GCG_ERR_CUDA, "k_intervals: shared memory"));
+    k_intervals<<<1, 1024, iv_rows * 4, s>>>(g->in_rowptr.get(), nv, P, g->intervals_dev.get(), d_count.get());
     if (cudaGetLastError() != cudaSuccess) return cleanup(fail(GCG_ERR_CUDA, "graph build kernels failed to launch"));
     uint32_t cnt = 0;
     g->intervals_host = (uint32_t *)malloc((size_t)P * 4);

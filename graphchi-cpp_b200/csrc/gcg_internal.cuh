@@ -191,6 +191,46 @@ namespace gcg {
 int radix_sort_u64(uint64_t *keys, uint64_t *tmp, uint64_t n, int begin_bit, int end_bit,
                    uint64_t **result, cudaStream_t s);
 
+/* The passes' digits: pass p takes bits [shift[p], shift[p] + bits[p]). As few
+ * passes as 8-bit digits allow, their widths within one bit of each other (a
+ * narrower digit means longer runs in the output and fewer votes). */
+struct RadixPlan {
+    static constexpr int MAX_PASSES = 8;
+    int npass;
+    uint8_t shift[MAX_PASSES], bits[MAX_PASSES];
+};
+RadixPlan radix_plan(int begin_bit, int end_bit);
+
+/* A sort's passes [first, last) alone, given the digit counts [pass][256] of all
+ * of the plan's passes (device). */
+int radix_passes(uint64_t *keys, uint64_t *tmp, uint64_t n, const RadixPlan &pl, int first, int last,
+                 const uint32_t *counts, uint64_t **result, cudaStream_t s);
+
+#ifdef __CUDACC__
+/* Digit counts of a block's keys in shared memory, one set per half block. */
+struct RadixCounter {
+    static constexpr int THREADS = 512;
+    uint32_t c[2][RadixPlan::MAX_PASSES][256];
+    __device__ __forceinline__ void clear() {
+        for (int i = threadIdx.x; i < 2 * RadixPlan::MAX_PASSES * 256; i += THREADS) (&c[0][0][0])[i] = 0;
+        __syncthreads();
+    }
+    __device__ __forceinline__ void add(const RadixPlan &pl, uint64_t key) {
+        uint32_t(*mine)[256] = c[threadIdx.x / (THREADS / 2)];
+#pragma unroll
+        for (int p = 0; p < RadixPlan::MAX_PASSES; ++p)
+            if (p < pl.npass) atomicAdd(&mine[p][(uint32_t)(key >> pl.shift[p]) & ((1u << pl.bits[p]) - 1u)], 1u);
+    }
+    __device__ __forceinline__ void flush(const RadixPlan &pl, uint32_t *counts) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < pl.npass * 256; i += THREADS) {
+            const uint32_t n = (&c[0][0][0])[i] + (&c[1][0][0])[i];
+            if (n) atomicAdd(counts + i, n);
+        }
+    }
+};
+#endif
+
 /* Exclusive scan of n uint32 values (device), returns the total through *total_dev
  * (device pointer, may be null). in and out may alias. */
 int scan_u32(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *total_dev, cudaStream_t s);

@@ -3,15 +3,11 @@
  * (stable LSD radix sort with 8-bit digits, src/util/radixSort.hpp:50-116, used by
  * shard_flushinfo::flush sharder.hpp:192 and finish_shard sharder.hpp:640).
  *
- * Design (HBM-bound integer work, no tensor cores):
- *   per 8-bit digit pass: upsweep (per-tile digit histogram, per-warp shared-memory
- *   counters) -> exclusive scan of the digit-major count table -> downsweep (each
- *   warp ranks its own contiguous 512 keys with warp-private digit counters and
- *   per-bit ballots, one digit-major scan over (digit, warp) gives every key its
- *   place in the tile, keys are regrouped by digit in shared memory and written so
- *   that each digit run of a tile is a contiguous, coalesced store).
- * Tiles are 4096 keys (256 threads x 16); each warp reads its 512 keys as 16
- * coalesced rounds of 32.
+ * Design (HBM traffic and instruction issue bound it, no tensor cores): one read
+ * of the keys counts the digits of every pass; each pass is then one kernel that
+ * reads and writes each key once. A tile's place in the output is found by a
+ * decoupled look-back over the tiles before it, one thread per digit, while the
+ * tile's keys wait in shared memory grouped by digit.
  */
 #include <algorithm>
 
@@ -21,10 +17,18 @@ namespace gcg {
 
 namespace {
 
+/* 256 threads x 22 keys, three blocks on an SM. 67 M keys build in 3.16 ms; 4
+ * blocks of 256 x 16 or 2 of 512 x 16 take 3.26: shorter runs, or fewer phases that
+ * overlap. */
 constexpr int RS_THREADS = 256;
-constexpr int RS_ITEMS = 16;
+constexpr int RS_ITEMS = 22;
+constexpr int RS_BLOCKS = 3;
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
 constexpr int RS_WARPS = RS_THREADS / 32;
+constexpr int RS_RADIX = 256;
+constexpr int RS_PASSES = RadixPlan::MAX_PASSES;
+constexpr int RS_SPIN = 1 << 14; /* polls of one tile's count before it is counted again */
+constexpr int RS_GROUP = 16;     /* tiles that share a group word */
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
@@ -32,37 +36,256 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     return m;
 }
 
-/* Warp w of a tile owns the contiguous keys [w*WSEG, (w+1)*WSEG) of the tile and
- * reads them as RS_ITEMS coalesced rounds of 32; keeping each warp's keys
- * contiguous lets the downsweep rank them with warp-private counters and stay
- * stable (tile order = warp order, then round, then lane). */
-constexpr int RS_WSEG = RS_TILE / RS_WARPS;
-
-__global__ void __launch_bounds__(RS_THREADS) rs_upsweep(const uint64_t *__restrict__ keys, uint64_t n,
-                                                         int shift, uint32_t dmask, uint32_t ntiles,
-                                                         uint32_t *__restrict__ counts) {
-    __shared__ uint32_t hist[RS_WARPS][256];
-    for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_THREADS) (&hist[0][0])[i] = 0;
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint64_t wbase = (uint64_t)blockIdx.x * RS_TILE + (uint64_t)warp * RS_WSEG;
-    uint32_t dig[RS_ITEMS];
+/* Digit counts of every pass from one read of the keys: counts[p][digit]. Bound
+ * by the shared-memory atomics (67 M keys, 6 passes: 184 us). */
+__global__ void __launch_bounds__(RadixCounter::THREADS) rs_count(const uint64_t *__restrict__ keys, uint64_t n,
+                                                                  RadixPlan pl, uint32_t *__restrict__ counts) {
+    __shared__ RadixCounter cnt;
+    cnt.clear();
+    constexpr int ITEMS = 8;
+    constexpr uint64_t CH = (uint64_t)RadixCounter::THREADS * ITEMS;
+    for (uint64_t c0 = blockIdx.x * CH; c0 < n; c0 += gridDim.x * CH) {
+        uint64_t k[ITEMS];
 #pragma unroll
-    for (int k = 0; k < RS_ITEMS; ++k) {
-        const uint64_t i = wbase + (uint64_t)k * 32 + lane;
-        dig[k] = (i < n) ? (uint32_t)((__ldg(keys + i) >> shift) & dmask) : 256u;
+        for (int j = 0; j < ITEMS; ++j) {
+            const uint64_t i = c0 + (uint64_t)j * RadixCounter::THREADS + threadIdx.x;
+            k[j] = i < n ? __ldg(keys + i) : 0ull;
+        }
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            if (c0 + (uint64_t)j * RadixCounter::THREADS + threadIdx.x >= n) break;
+            cnt.add(pl, k[j]);
+        }
     }
-#pragma unroll
-    for (int k = 0; k < RS_ITEMS; ++k)
-        if (dig[k] < 256u) atomicAdd(&hist[warp][dig[k]], 1u);
-    __syncthreads();
-    uint32_t s = 0;
-#pragma unroll
-    for (int w = 0; w < RS_WARPS; ++w) s += hist[w][threadIdx.x];
-    counts[(uint64_t)threadIdx.x * ntiles + blockIdx.x] = s;
+    cnt.flush(pl, counts);
 }
 
-/* Block-wide exclusive scan of one uint32 per thread (RS_THREADS threads). */
+/* State words: the pass that wrote it and the status in the high half, a count
+ * in the low half. The tag makes the words of an earlier pass read as absent, so
+ * they are cleared once per sort. The word is all a reader takes from the writer,
+ * so relaxed accesses do. */
+constexpr uint32_t ST_AGG = 1u, ST_INC = 2u;
+__device__ __forceinline__ void st_put(unsigned long long *p, uint32_t tag, uint32_t val) {
+    const unsigned long long w = ((unsigned long long)tag << 32) | val;
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+__device__ __forceinline__ unsigned long long st_get(const unsigned long long *p) {
+    unsigned long long w;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+    return w;
+}
+
+struct RsPass {
+    const uint64_t *in;
+    uint64_t *out;
+    uint64_t n;
+    int shift, bits;
+    uint32_t tag; /* pass number * 4, from 4 */
+    const uint32_t *counts;
+    uint32_t *ticket;
+    unsigned long long *tile;  /* [tile][digit]: keys of the digit in the tile, or up to its end */
+    unsigned long long *group; /* [group][digit]: the same of RS_GROUP tiles */
+};
+
+/* keys of digit d among in[lo, hi): what a look-back falls back on when a word
+ * does not come, so that the result needs no wait (tiles start in ticket order:
+ * it does come) */
+__device__ __noinline__ uint32_t rs_recount(const uint64_t *in, uint64_t lo, uint64_t hi, int shift, uint32_t dmask,
+                                            uint32_t d) {
+    uint32_t c = 0;
+    for (uint64_t i = lo; i < hi; ++i) c += ((uint32_t)(in[i] >> shift) & dmask) == d;
+    return c;
+}
+
+/* One pass. Warp w of a tile owns the contiguous keys [w*WSEG, (w+1)*WSEG) and
+ * reads them as RS_ITEMS coalesced rounds of 32; keeping each warp's keys
+ * contiguous lets it rank them with counters of its own and stay stable (tile
+ * order = warp order, then round, then lane).
+ *
+ * The look-back goes over the tiles of the own group, then over whole groups.
+ * All tiles of a wave count their digits at about the same time, so a look-back
+ * by single tiles would have the whole wave to walk. Bound by the shared-memory
+ * pipe (75% busy: random digits' bank conflicts), then by the votes on the integer
+ * pipe, not by HBM: 67 M keys take 0.36 ms for 1.07 GB; a pass as three steps
+ * (count per tile, scan, scatter) took 0.59. BITS >= the digit's width. */
+constexpr int RS_WSEG = RS_TILE / RS_WARPS;
+constexpr size_t RS_SMEM = (size_t)RS_TILE * 8 + (size_t)RS_WARPS * RS_RADIX * 4 + RS_RADIX * 4 + 64;
+template <int BITS>
+__global__ void __launch_bounds__(RS_THREADS, RS_BLOCKS) rs_pass(RsPass a) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    uint64_t *s_keys = reinterpret_cast<uint64_t *>(s_raw);
+    uint32_t(*s_wcnt)[RS_RADIX] = reinterpret_cast<uint32_t(*)[RS_RADIX]>(s_keys + RS_TILE);
+    uint32_t *s_gofs = &s_wcnt[RS_WARPS][0];
+    uint32_t *s_scan = s_gofs + RS_RADIX;
+    __shared__ uint32_t s_tile;
+
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t dmask = (1u << a.bits) - 1u;
+    if (tid == 0) s_tile = atomicAdd(a.ticket, 1u);
+    for (uint32_t i = tid; i < RS_WARPS * RS_RADIX; i += RS_THREADS) (&s_wcnt[0][0])[i] = 0;
+    __syncthreads();
+    const uint32_t t = s_tile;
+    const uint64_t base = (uint64_t)t * RS_TILE;
+    const uint32_t tile_n = (a.n - base) < (uint64_t)RS_TILE ? (uint32_t)(a.n - base) : (uint32_t)RS_TILE;
+    const uint32_t w0 = warp * RS_WSEG + lane; /* this lane's first key of the tile */
+    const uint64_t *in = a.in + base;
+
+    /* places past the end hold all-ones keys: last in order and of the highest
+     * digit, they rank behind every key of the tile */
+    uint64_t key[RS_ITEMS];
+    if (tile_n == (uint32_t)RS_TILE) {
+#pragma unroll
+        for (int k = 0; k < RS_ITEMS; ++k) key[k] = __ldg(in + w0 + k * 32);
+    } else {
+#pragma unroll
+        for (int k = 0; k < RS_ITEMS; ++k) key[k] = (w0 + k * 32 < tile_n) ? __ldg(in + w0 + k * 32) : ~0ull;
+    }
+
+    /* warp-private ranking over the warp's rounds, in key order */
+    uint32_t lrank[RS_ITEMS / 2]; /* two 16-bit ranks in each */
+    uint32_t *wcnt = s_wcnt[warp];
+#pragma unroll
+    for (int k = 0; k < RS_ITEMS; ++k) {
+        const uint32_t d = (uint32_t)(key[k] >> a.shift) & dmask;
+        /* lanes holding another digit, from one vote per digit bit (cheaper here
+         * than __match_any_sync, which competes with the shared-memory traffic) */
+        uint32_t others = 0;
+#pragma unroll
+        for (int b = 0; b < BITS; ++b) {
+            uint32_t vote, mine; /* written out: the compiler's form takes half as many instructions again */
+            asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\t"
+                         "and.b32 t, %2, %3;\n\tsetp.ne.u32 p, t, 0;\n\t"
+                         "vote.sync.ballot.b32 %0, p, 0xffffffff;\n\tselp.b32 %1, -1, 0, p;\n\t}"
+                         : "=r"(vote), "=r"(mine)
+                         : "r"(d), "r"(1 << b));
+            others |= vote ^ mine;
+        }
+        const uint32_t before = wcnt[d];
+        const uint32_t below = __popc(~others & lanemask_lt());
+        if (k & 1) lrank[k / 2] |= (before + below) << 16;
+        else lrank[k / 2] = before + below;
+        __syncwarp();
+        if (below == 0) wcnt[d] = before + 32u - __popc(others);
+        __syncwarp();
+    }
+    __syncthreads();
+
+    /* thread d: digit d's keys in this tile, published before anything else */
+    uint32_t total = 0, lstart = 0, excl = 0;
+    if (tid < RS_RADIX) {
+#pragma unroll
+        for (int w = 0; w < RS_WARPS; ++w) total += s_wcnt[w][tid];
+        const uint32_t held = total; /* with the places past the end */
+        if (tid == dmask) total -= (uint32_t)RS_TILE - tile_n;
+        if (t > 0) st_put(a.tile + (uint64_t)t * RS_RADIX + tid, a.tag | ST_AGG, total);
+        uint32_t v = held;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+            if (lane >= (uint32_t)o) v += y;
+        }
+        if (lane == 31) s_scan[warp] = v;
+        lstart = v - held;
+        if (t == 0) { /* keys of the digits below d in all tiles: every later tile gets it from here */
+            const uint32_t c = __ldg(a.counts + tid);
+            v = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+                if (lane >= (uint32_t)o) v += y;
+            }
+            if (lane == 31) s_scan[RS_RADIX / 32 + warp] = v;
+            excl = v - c;
+        }
+    }
+    __syncthreads();
+    if (tid < RS_RADIX) {
+#pragma unroll
+        for (uint32_t w = 0; w < RS_RADIX / 32; ++w) {
+            lstart += w < warp ? s_scan[w] : 0u;
+            if (t == 0) excl += w < warp ? s_scan[RS_RADIX / 32 + w] : 0u;
+        }
+        if (t == 0) st_put(a.tile + tid, a.tag | ST_INC, excl + total);
+        /* digit-major offsets: digit d's keys of warp w start after those of warps < w */
+        uint32_t run = lstart;
+#pragma unroll
+        for (int w = 0; w < RS_WARPS; ++w) {
+            const uint32_t c = s_wcnt[w][tid];
+            s_wcnt[w][tid] = run;
+            run += c;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < RS_ITEMS; ++k) {
+        const uint32_t d = (uint32_t)(key[k] >> a.shift) & dmask;
+        s_keys[wcnt[d] + ((k & 1) ? lrank[k / 2] >> 16 : lrank[k / 2] & 0xFFFFu)] = key[k];
+    }
+
+    /* excl: keys of digit d in the tiles before this one, and of the digits below
+     * d in all of them */
+    if (tid < RS_RADIX) {
+        const uint32_t g = t / RS_GROUP, in_g = t % RS_GROUP, pass = a.tag >> 2;
+        /* a word, waited for, or else what it would hold; true: it reaches back to the start */
+        auto take = [&](const unsigned long long *p, unsigned long long w, uint64_t lo, uint64_t hi) {
+            for (int spin = 0; (uint32_t)(w >> 34) != pass && spin < RS_SPIN; ++spin) w = st_get(p);
+            if ((uint32_t)(w >> 34) == pass) {
+                excl += (uint32_t)w;
+                return (uint32_t)(w >> 32) == (a.tag | ST_INC);
+            }
+            excl += rs_recount(a.in, lo * RS_TILE, hi * RS_TILE, a.shift, dmask, tid);
+            if (lo == 0)
+                for (uint32_t d = 0; d < tid; ++d) excl += __ldg(a.counts + d);
+            return lo == 0;
+        };
+        bool found = t == 0;
+        if (in_g) {
+            const unsigned long long *p = a.tile + (uint64_t)(g * RS_GROUP) * RS_RADIX + tid;
+            unsigned long long w[RS_GROUP - 1];
+#pragma unroll
+            for (int i = 0; i < RS_GROUP - 1; ++i) w[i] = i < (int)in_g ? st_get(p + i * RS_RADIX) : 0ull;
+#pragma unroll
+            for (int i = RS_GROUP - 2; i >= 0; --i)
+                if (i < (int)in_g && !found)
+                    found = take(p + i * RS_RADIX, w[i], (uint64_t)g * RS_GROUP + i, (uint64_t)g * RS_GROUP + i + 1);
+        }
+        unsigned long long *own = a.group + (uint64_t)g * RS_RADIX + tid;
+        const bool last = in_g == RS_GROUP - 1;
+        if (last && !found) st_put(own, a.tag | ST_AGG, excl + total);
+        constexpr int WIN = 8;
+        for (int64_t j = (int64_t)g - 1; !found; j -= WIN) { /* group 0's word reaches back to the start */
+            const unsigned long long *p = a.group + (uint64_t)j * RS_RADIX + tid;
+            unsigned long long w[WIN];
+#pragma unroll
+            for (int i = 0; i < WIN; ++i) w[i] = j >= i ? st_get(p - i * RS_RADIX) : 0ull;
+#pragma unroll
+            for (int i = 0; i < WIN; ++i)
+                if (j >= i && !found)
+                    found = take(p - i * RS_RADIX, w[i], (uint64_t)(j - i) * RS_GROUP,
+                                 (uint64_t)(j - i + 1) * RS_GROUP);
+        }
+        if (t > 0) st_put(a.tile + (uint64_t)t * RS_RADIX + tid, a.tag | ST_INC, excl + total);
+        if (last) st_put(own, a.tag | ST_INC, excl + total);
+        /* tile position i of digit d goes to excl + (i - lstart[d]); uint32
+         * wrap-around is exact: every index is below 2^32 */
+        s_gofs[tid] = excl - lstart;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t i = tid; i < tile_n; i += RS_THREADS) {
+        const uint64_t kk = s_keys[i];
+        const uint32_t d = (uint32_t)(kk >> a.shift) & dmask;
+        a.out[(uint32_t)(s_gofs[d] + i)] = kk;
+    }
+}
+
+/* ---- scan -------------------------------------------------------------- */
+
+constexpr int SC_THREADS = 256;
+constexpr int SC_ITEMS = 16;
+constexpr int SC_TILE = SC_THREADS * SC_ITEMS;
+
+/* Block-wide exclusive scan of one uint32 per thread (SC_THREADS threads). */
 __device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t *s_warp) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t v = x;
@@ -74,104 +297,18 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t *s_warp
     if (lane == 31) s_warp[warp] = v;
     __syncthreads();
     if (warp == 0) {
-        uint32_t w = (lane < RS_WARPS) ? s_warp[lane] : 0u;
+        uint32_t w = (lane < (SC_THREADS / 32)) ? s_warp[lane] : 0u;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             uint32_t y = __shfl_up_sync(0xFFFFFFFFu, w, o);
             if (lane >= o) w += y;
         }
-        if (lane < RS_WARPS) s_warp[lane] = w;
+        if (lane < (SC_THREADS / 32)) s_warp[lane] = w;
     }
     __syncthreads();
     uint32_t before = warp ? s_warp[warp - 1] : 0u;
     return before + v - x;
 }
-
-__global__ void __launch_bounds__(RS_THREADS) rs_downsweep(const uint64_t *__restrict__ keys_in,
-                                                           uint64_t *__restrict__ keys_out, uint64_t n,
-                                                           int shift, uint32_t dmask, uint32_t ntiles,
-                                                           const uint32_t *__restrict__ counts,
-                                                           const uint32_t *__restrict__ offsets) {
-    __shared__ uint64_t s_keys[RS_TILE];
-    __shared__ uint32_t s_gofs[256];
-    __shared__ uint32_t s_lstart[256];
-    __shared__ uint32_t s_wcnt[RS_WARPS][256]; /* per warp: keys of each digit (then the warp's offset) */
-    __shared__ uint32_t s_scan[RS_WARPS];
-
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint64_t base = (uint64_t)blockIdx.x * RS_TILE;
-    const uint32_t tile_n = (n - base) < (uint64_t)RS_TILE ? (uint32_t)(n - base) : (uint32_t)RS_TILE;
-    const uint64_t wbase = base + (uint64_t)warp * RS_WSEG;
-
-    uint64_t key[RS_ITEMS];
-#pragma unroll
-    for (int k = 0; k < RS_ITEMS; ++k) {
-        const uint64_t i = wbase + (uint64_t)k * 32 + lane;
-        key[k] = (i < n) ? __ldg(keys_in + i) : 0ull;
-    }
-    for (int w = 0; w < RS_WARPS; ++w) s_wcnt[w][tid] = 0;
-    const uint32_t gofs = offsets[(uint64_t)tid * ntiles + blockIdx.x];
-    const uint32_t h = counts[(uint64_t)tid * ntiles + blockIdx.x];
-    const uint32_t lstart = block_excl_scan(h, s_scan); /* synchronises: s_wcnt is clear */
-    s_lstart[tid] = lstart;
-    /* tile position i of digit d goes to gofs[d] + (i - lstart[d]); one table
-     * instead of two (uint32 wrap-around is exact: every index is below 2^32) */
-    s_gofs[tid] = gofs - lstart;
-
-    /* warp-private ranking over the warp's 16 rounds, in key order */
-    uint16_t lrank[RS_ITEMS];
-#pragma unroll
-    for (int k = 0; k < RS_ITEMS; ++k) {
-        const uint64_t i = wbase + (uint64_t)k * 32 + lane;
-        const bool valid = i < n;
-        const uint32_t d = valid ? (uint32_t)((key[k] >> shift) & dmask) : 256u;
-        /* lanes holding the same digit, from one vote per digit bit (cheaper here
-         * than __match_any_sync, which competes with the shared-memory traffic) */
-        uint32_t peers = __ballot_sync(0xFFFFFFFFu, valid);
-#pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            const uint32_t vb = __ballot_sync(0xFFFFFFFFu, (d >> b) & 1u);
-            peers &= ((d >> b) & 1u) ? vb : ~vb;
-        }
-        const uint32_t before = valid ? s_wcnt[warp][d] : 0u;
-        lrank[k] = (uint16_t)(before + __popc(peers & lanemask_lt()));
-        __syncwarp();
-        if (valid && lane == __ffs(peers) - 1) s_wcnt[warp][d] = before + __popc(peers);
-        __syncwarp();
-    }
-    __syncthreads();
-    /* digit-major offsets: digit d's keys of warp w start after those of warps < w */
-    {
-        uint32_t run = s_lstart[tid];
-#pragma unroll
-        for (int w = 0; w < RS_WARPS; ++w) {
-            const uint32_t c = s_wcnt[w][tid];
-            s_wcnt[w][tid] = run;
-            run += c;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < RS_ITEMS; ++k) {
-        const uint64_t i = wbase + (uint64_t)k * 32 + lane;
-        if (i < n) {
-            const uint32_t d = (uint32_t)((key[k] >> shift) & dmask);
-            s_keys[s_wcnt[warp][d] + lrank[k]] = key[k];
-        }
-    }
-    __syncthreads();
-    for (uint32_t i = tid; i < tile_n; i += RS_THREADS) {
-        const uint64_t kk = s_keys[i];
-        const uint32_t d = (uint32_t)((kk >> shift) & dmask);
-        keys_out[(uint32_t)(s_gofs[d] + i)] = kk;
-    }
-}
-
-/* ---- scan -------------------------------------------------------------- */
-
-constexpr int SC_THREADS = 256;
-constexpr int SC_ITEMS = 16;
-constexpr int SC_TILE = SC_THREADS * SC_ITEMS;
 
 __global__ void __launch_bounds__(SC_THREADS) sc_reduce(const uint32_t *__restrict__ in, uint64_t n,
                                                         uint32_t *__restrict__ sums) {
@@ -328,20 +465,9 @@ __global__ void __launch_bounds__(MG_THREADS) k_merge_u64(const uint64_t *__rest
  * It then writes the column of every kept key, the row pointers of the rows
  * its keys open, optionally the kept keys themselves, and takes duplicates off
  * the raw out-degree counts. */
-static_assert(MG_THREADS == RS_THREADS, "block_excl_scan is sized for RS_THREADS");
-constexpr uint32_t TS_AGG = 1u, TS_INC = 2u;
+static_assert(MG_THREADS == SC_THREADS, "block_excl_scan is sized for SC_THREADS");
 constexpr long long LB_SPIN = 1ll << 22;
-
-__device__ __forceinline__ void ts_store(unsigned long long *p, uint32_t status, uint32_t val) {
-    const unsigned long long w = ((unsigned long long)status << 32) | val;
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
-}
-
-__device__ __forceinline__ unsigned long long ts_load(const unsigned long long *p) {
-    unsigned long long w;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
-    return w;
-}
+constexpr uint32_t LB_GROUP = 32; /* tiles that share a group word */
 
 struct FinishArgs {
     const uint64_t *a, *b;
@@ -353,42 +479,50 @@ struct FinishArgs {
     uint64_t *keys_out;   /* kept keys, or null */
     uint32_t *outdeg_dup; /* raw out-degree counts to take duplicates off, or null */
     uint32_t *ticket;
-    unsigned long long *tstate;
+    unsigned long long *tstate, *gstate; /* per tile; per group of tiles */
     uint32_t *total;
     int *err;
 };
 
-/* exclusive prefix of tile t's kept keys: warp 0 walks back over the tile states,
- * 32 at a time, until it meets an inclusive prefix */
-__device__ __forceinline__ uint32_t look_back(const FinishArgs &f, uint32_t t, uint32_t lane) {
+/* Exclusive prefix of tile t's kept keys, by one warp that publishes the tile's
+ * own count and prefix: over the tiles of its group of 32 first, then over whole
+ * groups, 32 at a time. All tiles of a wave count their keys at about the same
+ * time: by single tiles the walk took a step per 32 of them. */
+__device__ __forceinline__ uint32_t look_back(const FinishArgs &f, uint32_t t, uint32_t tile_sum, uint32_t lane) {
+    const uint32_t g = t / LB_GROUP, in_g = t % LB_GROUP;
+    const bool last = in_g == LB_GROUP - 1;
     uint32_t excl = 0;
-    int64_t j = (int64_t)t - 1;
-    while (j >= 0) {
-        const int64_t idx = j - (int64_t)lane;
+    /* adds p[0], p[-1], .. p[-(n-1)] up to the first that reaches back to the start */
+    auto walk = [&](const unsigned long long *p, uint32_t n) {
         unsigned long long w = 0;
-        if (idx >= 0) {
+        if (lane < n) {
             long long spin = 0;
             do {
-                w = ts_load(f.tstate + idx);
+                w = st_get(p - lane);
             } while ((w >> 32) == 0 && ++spin < LB_SPIN);
             if ((w >> 32) == 0) atomicExch(f.err, 1);
         }
-        const uint32_t status = (uint32_t)(w >> 32);
-        const uint32_t inc = __ballot_sync(0xFFFFFFFFu, idx >= 0 && status == TS_INC);
-        const uint32_t stop = inc ? (uint32_t)(__ffs(inc) - 1) : 31u; /* nearest inclusive tile */
-        uint32_t v = (idx >= 0 && lane <= stop) ? (uint32_t)w : 0u;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-        excl += v;
-        if (inc) break;
-        j -= 32;
+        const uint32_t inc = __ballot_sync(0xFFFFFFFFu, (uint32_t)(w >> 32) == ST_INC);
+        const uint32_t stop = inc ? (uint32_t)(__ffs(inc) - 1) : 31u;
+        excl += __reduce_add_sync(0xFFFFFFFFu, lane <= stop ? (uint32_t)w : 0u);
+        return inc != 0;
+    };
+    if (lane == 0) st_put(f.tstate + t, t == 0 ? ST_INC : ST_AGG, tile_sum);
+    bool found = t == 0;
+    if (in_g) found = walk(f.tstate + t - 1, in_g);
+    if (lane == 0 && last && !found) st_put(f.gstate + g, ST_AGG, excl + tile_sum);
+    for (int64_t j = (int64_t)g - 1; !found && j >= 0; j -= 32)
+        found = walk(f.gstate + j, j + 1 < 32 ? (uint32_t)(j + 1) : 32u);
+    if (lane == 0) {
+        st_put(f.tstate + t, ST_INC, excl + tile_sum);
+        if (last) st_put(f.gstate + g, ST_INC, excl + tile_sum);
     }
     return excl;
 }
 
 __global__ void __launch_bounds__(MG_THREADS, 4) k_merge_finish(FinishArgs f) {
     __shared__ uint64_t s_in[MF_TILE + MF_TILE / MF_ITEMS];
-    __shared__ uint32_t s_warp[RS_WARPS];
+    __shared__ uint32_t s_warp[MG_THREADS / 32];
     __shared__ uint32_t s_tile, s_excl, s_sum;
     if (threadIdx.x == 0) s_tile = atomicAdd(f.ticket, 1u);
     __syncthreads();
@@ -428,20 +562,11 @@ __global__ void __launch_bounds__(MG_THREADS, 4) k_merge_finish(FinishArgs f) {
         }
     }
     const uint32_t local = block_excl_scan(cnt, s_warp);
-    if (threadIdx.x == MG_THREADS - 1) {
-        const uint32_t tile_sum = local + cnt;
-        if (t == 0) ts_store(f.tstate, TS_INC, tile_sum);
-        else ts_store(f.tstate + t, TS_AGG, tile_sum);
-        s_sum = tile_sum;
-    }
+    if (threadIdx.x == MG_THREADS - 1) s_sum = local + cnt;
     __syncthreads();
     const uint32_t tile_sum = s_sum;
     if (threadIdx.x < 32) {
-        uint32_t excl = 0;
-        if (t > 0) {
-            excl = look_back(f, t, threadIdx.x);
-            if (threadIdx.x == 0) ts_store(f.tstate + t, TS_INC, excl + tile_sum);
-        }
+        const uint32_t excl = look_back(f, t, tile_sum, threadIdx.x);
         if (threadIdx.x == 0) s_excl = excl;
     }
     __syncthreads();
@@ -481,6 +606,80 @@ __global__ void __launch_bounds__(MG_THREADS, 4) k_merge_finish(FinishArgs f) {
     }
 }
 
+/* The same from one sorted run (nothing to merge), in two passes of independent
+ * warps: the kept keys of every 512 are counted, scanned, and written at their
+ * places. The second read of the keys costs less than a look-back and merged
+ * tiles staged in shared memory (67 M keys: 540 us through the merging kernel,
+ * 568 in one pass with a look-back, 330 as two). */
+constexpr int FR_ITEMS = 16;
+constexpr int FR_WSEG = 32 * FR_ITEMS;
+
+__global__ void __launch_bounds__(256) k_run_count(const uint64_t *__restrict__ keys, uint64_t n, uint32_t nseg,
+                                                   uint32_t *__restrict__ cnt) {
+    const uint32_t w = (blockIdx.x * 256u + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    if (w >= nseg) return;
+    const uint64_t i0 = (uint64_t)w * FR_WSEG + lane;
+    uint32_t c = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint64_t key[FR_ITEMS / 2], prev[FR_ITEMS / 2];
+#pragma unroll
+        for (int k = 0; k < FR_ITEMS / 2; ++k) {
+            const uint64_t i = i0 + (h * (FR_ITEMS / 2) + k) * 32;
+            key[k] = i < n ? __ldg(keys + i) : 0ull;
+            prev[k] = i < n && i > 0 ? __ldg(keys + i - 1) : ~key[k]; /* the first key is kept */
+        }
+#pragma unroll
+        for (int k = 0; k < FR_ITEMS / 2; ++k)
+            c += i0 + (h * (FR_ITEMS / 2) + k) * 32 < n && key[k] != prev[k] ? 1u : 0u;
+    }
+    c = __reduce_add_sync(0xFFFFFFFFu, c);
+    if (lane == 0) cnt[w] = c;
+}
+
+/* first[w]: where the kept keys of segment w go; without duplicates to drop
+ * (dedup 0, first null) every key stays where it is */
+__global__ void __launch_bounds__(256, 4) k_run_write(FinishArgs f, uint32_t nseg, const uint32_t *__restrict__ first) {
+    const uint32_t w = (blockIdx.x * 256u + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    if (w >= nseg) return;
+    const uint64_t i0 = (uint64_t)w * FR_WSEG + lane;
+    const uint32_t mask = (uint32_t)((1ull << f.kbits) - 1ull);
+    uint32_t q = first ? __ldg(first + w) : w * FR_WSEG;
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        uint64_t key[FR_ITEMS / 2], prev[FR_ITEMS / 2];
+#pragma unroll
+        for (int k = 0; k < FR_ITEMS / 2; ++k) {
+            const uint64_t i = i0 + (h * (FR_ITEMS / 2) + k) * 32;
+            key[k] = i < f.kept ? __ldg(f.a + i) : 0ull;
+            prev[k] = i < f.kept && i > 0 ? __ldg(f.a + i - 1) : ~key[k];
+        }
+#pragma unroll
+        for (int k = 0; k < FR_ITEMS / 2; ++k) {
+            const uint64_t i = i0 + (h * (FR_ITEMS / 2) + k) * 32;
+            const bool kp = i < f.kept && (!f.dedup || key[k] != prev[k]);
+            const uint32_t b = __ballot_sync(0xFFFFFFFFu, kp);
+            const uint32_t at = q + __popc(b & lanemask_lt());
+            q += __popc(b);
+            const uint32_t row = (uint32_t)(key[k] >> f.kbits), prow = (uint32_t)(prev[k] >> f.kbits);
+            const uint32_t col = (uint32_t)key[k] & mask;
+            if (kp) {
+                f.col[at] = col;
+                if (f.keys_out) f.keys_out[at] = key[k];
+                if (i == 0 || row != prow)
+                    for (uint32_t r = i == 0 ? 0u : prow + 1u; r <= row; ++r) f.rowptr[r] = at;
+            } else if (f.outdeg_dup && i < f.kept) {
+                atomicSub(f.outdeg_dup + col, 1u);
+            }
+            if (i == f.kept - 1) { /* rows after the last key end at the total */
+                const uint32_t end = at + (kp ? 1u : 0u);
+                for (uint64_t r = (uint64_t)row + 1; r <= f.nv; ++r) f.rowptr[r] = end;
+                *f.total = end;
+            }
+        }
+    }
+}
+
 }  // namespace
 
 int merge_u64(const uint64_t *a, uint64_t na, const uint64_t *b, uint64_t nb, uint64_t *out, cudaStream_t s) {
@@ -511,24 +710,18 @@ int merge_unique_csr(const uint64_t *a, uint64_t na, const uint64_t *b, uint64_t
     }
     const uint64_t n = na + nb;
     if (kept > n || kept > 0xFFFFFFFFull) return fail(GCG_ERR_INVALID, "merge_unique_csr: bad key count");
-    const uint64_t ntiles = (kept + MF_TILE - 1) / MF_TILE;
+    const bool one_run = na == 0 || nb == 0;
     tbuf<uint64_t> split;
     tbuf<unsigned long long> tstate;
-    tbuf<uint32_t> ctl; /* ticket, total, err */
-    GCG_TRY(split.alloc(ntiles + 1, s));
-    GCG_TRY(tstate.alloc(ntiles, s));
+    tbuf<uint32_t> seg, ctl; /* ctl: ticket, total, err */
     GCG_TRY(ctl.alloc(3, s));
-    GCG_CUDA(cudaMemsetAsync(tstate.get(), 0, ntiles * sizeof(unsigned long long), s));
     GCG_CUDA(cudaMemsetAsync(ctl.get(), 0, 3 * sizeof(uint32_t), s));
-    k_merge_split<MF_TILE><<<(unsigned)std::min<uint64_t>((ntiles + 256) / 256, (uint64_t)num_sms() * 8), 256, 0, s>>>(
-        a, na, b ? b : a, nb, ntiles, split.get());
-    FinishArgs f;
-    f.a = a;
-    f.b = b ? b : a;
+    FinishArgs f = {};
+    f.a = na ? a : b;
+    f.b = b;
     f.na = na;
     f.nb = nb;
     f.kept = kept;
-    f.split = split.get();
     f.kbits = kbits;
     f.nv = nv;
     f.dedup = dedup ? 1 : 0;
@@ -537,10 +730,30 @@ int merge_unique_csr(const uint64_t *a, uint64_t na, const uint64_t *b, uint64_t
     f.keys_out = keys_out;
     f.outdeg_dup = outdeg_dup;
     f.ticket = ctl.get();
-    f.tstate = tstate.get();
     f.total = ctl.get() + 1;
     f.err = (int *)(ctl.get() + 2);
-    k_merge_finish<<<(unsigned)ntiles, MG_THREADS, 0, s>>>(f);
+    if (one_run) {
+        const uint32_t nseg = (uint32_t)((kept + FR_WSEG - 1) / FR_WSEG), blocks = (nseg + 7) / 8;
+        if (dedup) {
+            GCG_TRY(seg.alloc(nseg, s));
+            k_run_count<<<blocks, 256, 0, s>>>(f.a, kept, nseg, seg.get());
+            GCG_LAUNCH_CHECK();
+            GCG_TRY(scan_u32(seg.get(), seg.get(), nseg, nullptr, s));
+        }
+        k_run_write<<<blocks, 256, 0, s>>>(f, nseg, seg.get());
+    } else {
+        const uint64_t ntiles = (kept + MF_TILE - 1) / MF_TILE, nwords = ntiles + ntiles / LB_GROUP + 1;
+        GCG_TRY(split.alloc(ntiles + 1, s));
+        GCG_TRY(tstate.alloc(nwords, s));
+        GCG_CUDA(cudaMemsetAsync(tstate.get(), 0, nwords * sizeof(unsigned long long), s));
+        k_merge_split<MF_TILE>
+            <<<(unsigned)std::min<uint64_t>((ntiles + 256) / 256, (uint64_t)num_sms() * 8), 256, 0, s>>>(
+                a, na, b, nb, ntiles, split.get());
+        f.split = split.get();
+        f.tstate = tstate.get();
+        f.gstate = tstate.get() + ntiles;
+        k_merge_finish<<<(unsigned)ntiles, MG_THREADS, 0, s>>>(f);
+    }
     GCG_LAUNCH_CHECK();
     uint32_t h[2] = {0, 0};
     GCG_CUDA(cudaMemcpyAsync(h, ctl.get() + 1, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -572,28 +785,65 @@ int scan_u32(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *total_dev,
     return GCG_OK;
 }
 
-int radix_sort_u64(uint64_t *keys, uint64_t *tmp, uint64_t n, int begin_bit, int end_bit,
-                   uint64_t **result, cudaStream_t s) {
+RadixPlan radix_plan(int begin_bit, int end_bit) {
+    RadixPlan pl = {};
+    for (int left = end_bit - begin_bit, passes = (left + 7) / 8; passes > 0; --passes) {
+        const int bits = (left + passes - 1) / passes;
+        pl.shift[pl.npass] = (uint8_t)(end_bit - left);
+        pl.bits[pl.npass++] = (uint8_t)bits;
+        left -= bits;
+    }
+    return pl;
+}
+
+int radix_passes(uint64_t *keys, uint64_t *tmp, uint64_t n, const RadixPlan &pl, int first, int last,
+                 const uint32_t *counts, uint64_t **result, cudaStream_t s) {
     *result = keys;
-    if (n <= 1 || end_bit <= begin_bit) return GCG_OK;
+    if (n <= 1 || first >= last) return GCG_OK;
     if (n > 0xFFFFFFFFull) return fail(GCG_ERR_UNSUPPORTED, "radix sort: more than 2^32-1 keys");
-    uint32_t ntiles = (uint32_t)((n + RS_TILE - 1) / RS_TILE);
-    tbuf<uint32_t> counts, offsets;
-    GCG_TRY(counts.alloc((size_t)256 * ntiles, s));
-    GCG_TRY(offsets.alloc((size_t)256 * ntiles, s));
+    const uint64_t ntiles = (n + RS_TILE - 1) / RS_TILE;
+    /* state words and tickets, cleared together */
+    const uint64_t nwords = (ntiles + ntiles / RS_GROUP + 1) * RS_RADIX;
+    tbuf<unsigned long long> work;
+    GCG_TRY(work.alloc(nwords + RS_PASSES, s));
+    GCG_CUDA(cudaMemsetAsync(work.get(), 0, (nwords + RS_PASSES) * 8, s));
     uint64_t *a = keys, *b = tmp;
-    for (int shift = begin_bit; shift < end_bit; shift += 8) {
-        const int nb = end_bit - shift < 8 ? end_bit - shift : 8;
-        const uint32_t dmask = (1u << nb) - 1u;
-        rs_upsweep<<<ntiles, RS_THREADS, 0, s>>>(a, n, shift, dmask, ntiles, counts.get());
+    for (int p = first; p < last; ++p) {
+        RsPass ps;
+        ps.in = a;
+        ps.out = b;
+        ps.n = n;
+        ps.shift = pl.shift[p];
+        ps.bits = pl.bits[p];
+        ps.tag = (uint32_t)(p + 1) << 2;
+        ps.counts = counts + p * RS_RADIX;
+        ps.ticket = reinterpret_cast<uint32_t *>(work.get() + nwords + p);
+        ps.tile = work.get();
+        ps.group = work.get() + ntiles * RS_RADIX;
+        auto kern = ps.bits == 8 ? rs_pass<8> : ps.bits == 7 ? rs_pass<7> : rs_pass<6>;
+        GCG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RS_SMEM));
+        kern<<<(unsigned)ntiles, RS_THREADS, RS_SMEM, s>>>(ps);
         GCG_LAUNCH_CHECK();
-        GCG_TRY(scan_u32(counts.get(), offsets.get(), (uint64_t)256 * ntiles, nullptr, s));
-        rs_downsweep<<<ntiles, RS_THREADS, 0, s>>>(a, b, n, shift, dmask, ntiles, counts.get(), offsets.get());
-        GCG_LAUNCH_CHECK();
-        uint64_t *t = a; a = b; b = t;
+        uint64_t *x = a; a = b; b = x;
     }
     *result = a;
     return GCG_OK;
+}
+
+int radix_sort_u64(uint64_t *keys, uint64_t *tmp, uint64_t n, int begin_bit, int end_bit, uint64_t **result,
+                   cudaStream_t s) {
+    *result = keys;
+    if (n <= 1 || end_bit <= begin_bit) return GCG_OK;
+    if (end_bit - begin_bit > 8 * RS_PASSES) return fail(GCG_ERR_INVALID, "radix sort: more than 64 bits");
+    const RadixPlan pl = radix_plan(begin_bit, end_bit);
+    tbuf<uint32_t> counts;
+    GCG_TRY(counts.alloc(RS_PASSES * RS_RADIX, s));
+    GCG_CUDA(cudaMemsetAsync(counts.get(), 0, RS_PASSES * RS_RADIX * 4, s));
+    constexpr uint64_t per_block = (uint64_t)RadixCounter::THREADS * 8;
+    rs_count<<<(unsigned)std::min<uint64_t>((n + per_block - 1) / per_block, (uint64_t)num_sms() * 4),
+               RadixCounter::THREADS, 0, s>>>(keys, n, pl, counts.get());
+    GCG_LAUNCH_CHECK();
+    return radix_passes(keys, tmp, n, pl, 0, pl.npass, counts.get(), result, s);
 }
 
 }  // namespace gcg
