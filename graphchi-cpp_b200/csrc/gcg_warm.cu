@@ -9,7 +9,8 @@
  *
  * Kernels
  *   k_warm_vstat   per vertex: {log(1+indeg), indeg} packed in 8 bytes, stored at
- *                  the vertex's out-degree rank (the PageRank relabelling)
+ *                  the vertex's out-degree rank (the PageRank relabelling); the ranks
+ *                  of the vertices without in-edges
  *   k_warm_agg_edges / k_warm_agg_fix   per vertex with in-edges: sum and max of
  *                  L(u) = log(1+indeg(u)) over in-neighbours u and the sum of
  *                  indeg(u), on the PageRank chunk plan: one warp per 256 in-edges
@@ -53,6 +54,7 @@ constexpr int NP = GCG_MLP_NPARAMS;
 /* offsets in the flat parameter vector */
 constexpr int OW1 = 0, OB1 = OW1 + NH * NIN, OW2 = OB1 + NH, OB2 = OW2 + NH * NH, OW3 = OB2 + NH, OB3 = OW3 + NH;
 static_assert(OB3 + 1 == NP, "parameter layout");
+static_assert(OW2 % 4 == 0, "128-bit loads of W2");
 constexpr int TRAIN_T = 128;        /* samples per training tile */
 
 /* round to the nearest BF16 value (ties to even), kept as a float */
@@ -90,11 +92,34 @@ struct AggOut {
 };
 constexpr uint32_t AGG_HUB_MAX = 24576; /* 192 KB of {L, indeg} pairs */
 
-__global__ void k_warm_vstat(const uint32_t *__restrict__ indeg, const uint32_t *__restrict__ newid, uint32_t nv,
-                             uint2 *__restrict__ vstat) {
+/* vstat of every vertex; with out given, also the part of the result that needs no network:
+ * vertices without in-edges get exactly teleport, and part_zd[block] counts those of them
+ * that also lack out-edges. (In vertex order those stores are coalesced: as a pass over the
+ * list of such rows, which is in out-degree order, they took 19 us at R-MAT scale 22.) */
+__global__ void __launch_bounds__(256) k_warm_vstat(const uint32_t *__restrict__ indeg,
+                                                    const uint32_t *__restrict__ newid, uint32_t nv,
+                                                    uint2 *__restrict__ vstat, const uint32_t *__restrict__ outdeg,
+                                                    float teleport, float *__restrict__ out,
+                                                    uint32_t *__restrict__ part_zd) {
+    __shared__ uint32_t s_c[8];
+    uint32_t c = 0;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
         const uint32_t d = indeg[v];
         vstat[newid[v]] = make_uint2(__float_as_uint(log1pf((float)d)), d);
+        if (out && d == 0u) {
+            out[v] = teleport;
+            c += outdeg[v] == 0u;
+        }
+    }
+    if (!out) return;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
+    if ((threadIdx.x & 31u) == 0) s_c[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t tot = 0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += s_c[w];
+        part_zd[blockIdx.x] = tot;
     }
 }
 
@@ -191,6 +216,29 @@ __global__ void k_warm_features(const uint32_t *__restrict__ nz_rows, uint32_t n
     }
 }
 
+/* ---- packed FP32 arithmetic ---------------------------------------------- */
+
+/* two FP32 FMAs in one instruction, each rounded as fmaf */
+__device__ __forceinline__ void fma2(unsigned long long &d, unsigned long long x, unsigned long long y) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(x), "l"(y));
+}
+__device__ __forceinline__ unsigned long long pair(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpair(unsigned long long x) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+    return r;
+}
+/* two FP32 additions in one instruction */
+__device__ __forceinline__ float2 add2(float2 x, float2 y) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair(x.x, x.y)), "l"(pair(y.x, y.y)));
+    return unpair(r);
+}
+
 /* ---- inference on tensor cores ------------------------------------------ */
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -229,7 +277,14 @@ __global__ void k_warm_xfeat(const uint32_t *__restrict__ nz_rows, const uint32_
  * is signalled on an mbarrier by tcgen05.commit; every wait is bounded. */
 constexpr int TC_ROWS = 128;   /* M of the MMA: rows of a tile, threads of a CTA */
 constexpr int TC_COLS = 64;    /* tensor-memory columns held by a CTA (the N of both layers) */
-constexpr uint32_t TC_CTAS_PER_SM = 4;
+/* The epilogues between the MMAs are what takes the time: 64 values per row and layer
+ * through the FP32 pipes, the layers' constants from shared memory (short scoreboard is
+ * the first stall, 47 % of issue slots busy). So they add in pairs, round and pack with
+ * one conversion, read the constants 128 bits at a time, and a thread holds TC_LD
+ * accumulator columns in place of all 64, with which seven CTAs (31.6 KB of shared memory,
+ * 64 tensor-memory columns each) fit an SM. 2.2 M rows: 94 -> 69 us. */
+constexpr uint32_t TC_CTAS_PER_SM = 7;
+constexpr int TC_LD = 32;
 /* instruction descriptor of kind::f16: FP32 accumulator (bits 4-5 = 1), BF16 A
  * (bits 7-9 = 1) and B (bits 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3
  * in bits 17-22, M >> 4 in bits 24-28 */
@@ -279,23 +334,31 @@ __host__ __device__ __forceinline__ uint32_t tc_off(uint32_t row, uint32_t k, ui
     return ((row >> 3) * kcores + (k >> 3)) * 128u + (row & 7u) * 16u + (k & 7u) * 2u;
 }
 
+/* ReLU of two values, rounded to BF16 (to nearest even) and packed, the first one low */
+__device__ __forceinline__ uint32_t relu_bf16x2(float2 x) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(fmaxf(x.x, 0.0f), fmaxf(x.y, 0.0f));
+    uint32_t r;
+    memcpy(&r, &h, 4);
+    return r;
+}
+
 struct InferArgs {
-    const uint32_t *nz_rows, *od_nz;
+    const uint32_t *od_nz;
     const uint4 *xpk;              /* per nz row: 8 normalised BF16 features */
     uint32_t nnz;
     const float *wb;               /* BF16-rounded weights, FP32 biases */
     float teleport;
-    float *out;
+    float *pred;                   /* per nz row: the predicted rank, unscaled */
     double2 *part_mass;            /* per block: sum of the predicted ranks, of those without out-edges */
     int *err;                      /* set when a wait for the tensor cores ran out */
 };
 
-__global__ void __launch_bounds__(TC_ROWS) k_warm_infer(InferArgs a) {
+__global__ void __launch_bounds__(TC_ROWS, TC_CTAS_PER_SM) k_warm_infer(InferArgs a) {
     __shared__ __align__(1024) uint8_t s_a1[TC_ROWS * 16 * 2]; /* X: 128 x 16 BF16 */
     __shared__ __align__(1024) uint8_t s_b1[NH * 16 * 2];      /* W1: 64 x 16 BF16 */
     __shared__ __align__(1024) uint8_t s_a2[TC_ROWS * NH * 2]; /* H1: 128 x 64 BF16 */
     __shared__ __align__(1024) uint8_t s_b2[NH * NH * 2];      /* W2: 64 x 64 BF16 */
-    __shared__ float s_bias1[NH], s_bias2[NH], s_w3[NH];
+    __shared__ __align__(16) float s_bias1[NH], s_bias2[NH], s_w3[NH];
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
@@ -308,9 +371,12 @@ __global__ void __launch_bounds__(TC_ROWS) k_warm_infer(InferArgs a) {
         const float w = k < (uint32_t)NIN ? a.wb[OW1 + n * NIN + k] : 0.0f;
         *(uint16_t *)(s_b1 + tc_off(n, k, 2)) = (uint16_t)bf16_bits(w);
     }
-    for (uint32_t e = tid; e < (uint32_t)NH * NH; e += TC_ROWS) {
+#pragma unroll
+    for (uint32_t e = tid * 8u; e < (uint32_t)NH * NH; e += TC_ROWS * 8u) { /* one core row at a time */
         const uint32_t n = e >> 6, k = e & 63u;
-        *(uint16_t *)(s_b2 + tc_off(n, k, NH / 8)) = (uint16_t)bf16_bits(a.wb[OW2 + n * NH + k]);
+        const float4 w0 = *(const float4 *)(a.wb + OW2 + e), w1 = *(const float4 *)(a.wb + OW2 + e + 4);
+        *(uint4 *)(s_b2 + tc_off(n, k, NH / 8)) =
+            make_uint4(pack_bf16(w0.x, w0.y), pack_bf16(w0.z, w0.w), pack_bf16(w1.x, w1.y), pack_bf16(w1.z, w1.w));
     }
     for (uint32_t j = tid; j < (uint32_t)NH; j += TC_ROWS) {
         s_bias1[j] = a.wb[OB1 + j];
@@ -341,12 +407,21 @@ __global__ void __launch_bounds__(TC_ROWS) k_warm_infer(InferArgs a) {
     double msum = 0.0, mdang = 0.0;
     uint32_t phase = 0;
     const uint32_t ntiles = (a.nnz + TC_ROWS - 1) / TC_ROWS;
+    auto load = [&](uint32_t tile, uint4 &x, uint32_t &od) { /* the thread's row of a tile */
+        const uint32_t i = tile * TC_ROWS + tid;
+        const bool valid = tile < ntiles && i < a.nnz;
+        x = valid ? a.xpk[i] : make_uint4(0u, 0u, 0u, 0u);
+        od = valid ? a.od_nz[i] : 1u;
+    };
+    uint4 x;
+    uint32_t od;
+    load(blockIdx.x, x, od);
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const uint32_t i = tile * TC_ROWS + tid;
         const bool valid = i < a.nnz;
-        const uint4 x = valid ? a.xpk[i] : make_uint4(0u, 0u, 0u, 0u);
-        const uint32_t v = valid ? a.nz_rows[i] : 0u, od = valid ? a.od_nz[i] : 1u;
+        const bool dangling = od == 0u;
         *(uint4 *)(s_a1 + tc_off(tid, 0, 2)) = x;
+        load(tile + gridDim.x, x, od); /* the next tile's: its latency behind this tile's layers */
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
@@ -361,22 +436,27 @@ __global__ void __launch_bounds__(TC_ROWS) k_warm_infer(InferArgs a) {
         phase ^= 1u;
         if (!ok) s_fail = 1;
         tc_fence_after();
-        float acc[NH];
-#pragma unroll
-        for (int q = 0; q < NH / 16; ++q) tc_ld16(taddr + 16u * q, acc + 16 * q);
-        tc_wait_ld();
         /* layer-1 epilogue: bias, ReLU, BF16, into this thread's row of H1 */
 #pragma unroll
-        for (int kc = 0; kc < NH / 8; ++kc) {
-            uint32_t w[4];
+        for (int q = 0; q < NH / TC_LD; ++q) {
+            float acc[TC_LD];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const int j = kc * 8 + 2 * t;
-                const float h0 = bf16r(fmaxf(acc[j] + s_bias1[j], 0.0f));
-                const float h1 = bf16r(fmaxf(acc[j + 1] + s_bias1[j + 1], 0.0f));
-                w[t] = bf16_bits(h0) | (bf16_bits(h1) << 16);
+            for (int h = 0; h < TC_LD / 16; ++h) tc_ld16(taddr + TC_LD * q + 16u * h, acc + 16 * h);
+            tc_wait_ld();
+#pragma unroll
+            for (int kc = 0; kc < TC_LD / 8; ++kc) {
+                uint32_t w[4];
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    const int l = kc * 8 + 4 * t;
+                    const float4 b = *(const float4 *)(s_bias1 + TC_LD * q + l);
+                    const float2 u0 = add2(make_float2(acc[l], acc[l + 1]), make_float2(b.x, b.y));
+                    const float2 u1 = add2(make_float2(acc[l + 2], acc[l + 3]), make_float2(b.z, b.w));
+                    w[2 * t] = relu_bf16x2(u0);
+                    w[2 * t + 1] = relu_bf16x2(u1);
+                }
+                *(uint4 *)(s_a2 + tc_off(tid, TC_LD * q + kc * 8, NH / 8)) = make_uint4(w[0], w[1], w[2], w[3]);
             }
-            *(uint4 *)(s_a2 + tc_off(tid, kc * 8, NH / 8)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
         fence_async_smem();
         tc_fence_before();
@@ -394,19 +474,31 @@ __global__ void __launch_bounds__(TC_ROWS) k_warm_infer(InferArgs a) {
         phase ^= 1u;
         if (!ok) s_fail = 1;
         tc_fence_after();
-#pragma unroll
-        for (int q = 0; q < NH / 16; ++q) tc_ld16(taddr + 16u * q, acc + 16 * q);
-        tc_wait_ld();
         /* layer 2's bias and ReLU, layer 3 on the FP32 pipes */
         float y = 0.0f;
 #pragma unroll
-        for (int j = 0; j < NH; ++j) y = fmaf(fmaxf(acc[j] + s_bias2[j], 0.0f), s_w3[j], y);
+        for (int q = 0; q < NH / TC_LD; ++q) {
+            float acc[TC_LD];
+#pragma unroll
+            for (int h = 0; h < TC_LD / 16; ++h) tc_ld16(taddr + TC_LD * q + 16u * h, acc + 16 * h);
+            tc_wait_ld();
+#pragma unroll
+            for (int l = 0; l < TC_LD; l += 4) {
+                const float4 b = *(const float4 *)(s_bias2 + TC_LD * q + l), w = *(const float4 *)(s_w3 + TC_LD * q + l);
+                const float2 u0 = add2(make_float2(acc[l], acc[l + 1]), make_float2(b.x, b.y));
+                const float2 u1 = add2(make_float2(acc[l + 2], acc[l + 3]), make_float2(b.z, b.w));
+                y = fmaf(fmaxf(u0.x, 0.0f), w.x, y);
+                y = fmaf(fmaxf(u0.y, 0.0f), w.y, y);
+                y = fmaf(fmaxf(u1.x, 0.0f), w.z, y);
+                y = fmaf(fmaxf(u1.y, 0.0f), w.w, y);
+            }
+        }
         if (valid) {
             /* y is clamped so exp stays finite */
             const float r = a.teleport * expf(fminf(fmaxf(y + b3, -30.0f), 30.0f));
-            a.out[v] = r;
+            a.pred[i] = r;
             msum += (double)r;
-            if (od == 0) mdang += (double)r;
+            if (dangling) mdang += (double)r;
         }
         tc_fence_before(); /* this tile's tensor-memory reads precede the next tile's MMA */
     }
@@ -436,28 +528,6 @@ __global__ void __launch_bounds__(TC_ROWS) k_warm_infer(InferArgs a) {
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TC_COLS)
                      : "memory");
-}
-
-/* vertices without in-edges: exactly teleport; per block, how many also lack out-edges */
-__global__ void __launch_bounds__(256) k_warm_zero(const uint32_t *__restrict__ zero_rows, uint32_t nzero,
-                                                   const uint32_t *__restrict__ outdeg, float teleport,
-                                                   float *__restrict__ out, uint32_t *__restrict__ part_zd) {
-    __shared__ uint32_t s_c[8];
-    uint32_t c = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nzero; i += gridDim.x * blockDim.x) {
-        const uint32_t v = zero_rows[i];
-        out[v] = teleport;
-        c += outdeg[v] == 0;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
-    if ((threadIdx.x & 31u) == 0) s_c[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t tot = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += s_c[w];
-        part_zd[blockIdx.x] = tot;
-    }
 }
 
 /* Mass-stationary scale of the predicted ranks: alpha such that one Jacobi sweep
@@ -491,12 +561,10 @@ __global__ void k_warm_alpha(const double2 *__restrict__ pm, uint32_t nmass, con
 }
 
 __global__ void k_warm_scale(const uint32_t *__restrict__ nz_rows, uint32_t nnz, const double *__restrict__ alpha,
-                             float *__restrict__ out) {
+                             const float *__restrict__ pred, float *__restrict__ out) {
     const double al = *alpha;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
-        const uint32_t v = nz_rows[i];
-        out[v] = (float)((double)out[v] * al);
-    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x)
+        out[nz_rows[i]] = (float)((double)pred[i] * al);
 }
 
 /* ---- training -------------------------------------------------------------- */
@@ -535,21 +603,6 @@ static_assert(2 * TRAIN_SMEM + 2048 <= 227 * 1024, "two blocks per SM");
 static_assert(NH == 64 && NIN == 8 && TRAIN_T == 128, "the threads' tiles below");
 
 __device__ __forceinline__ float &at(float4 &v, int c) { return (&v.x)[c]; }
-
-/* two FP32 FMAs in one instruction, each rounded as fmaf */
-__device__ __forceinline__ void fma2(unsigned long long &d, unsigned long long x, unsigned long long y) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(x), "l"(y));
-}
-__device__ __forceinline__ unsigned long long pair(float lo, float hi) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 unpair(unsigned long long x) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
-    return r;
-}
 
 /* acc[s][c] = sum over k of a[k][8 samples] * b[k][4 features], k = 0 .. K - 1 in order;
  * pa, pb point at the thread's samples and features of row 0. Samples go in pairs, as
@@ -906,8 +959,15 @@ int set_train_smem() {
     return GCG_OK;
 }
 
-/* per-nz-row aggregates of the in-neighbourhood (features 2-4), on the chunk plan */
-int warm_aggregates(gcg_graph *g, tbuf<Agg3> &agg, cudaStream_t s) {
+/* blocks of the pass over all vertices */
+unsigned vstat_grid(uint32_t nv) {
+    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)nv + 255) / 256, num_sms() * 8ull));
+}
+
+/* per-nz-row aggregates of the in-neighbourhood (features 2-4), on the chunk plan; with
+ * out given, also the ranks of the vertices without in-edges (part_zd: vstat_grid entries) */
+int warm_aggregates(gcg_graph *g, tbuf<Agg3> &agg, cudaStream_t s, float teleport = 0.0f, float *out = nullptr,
+                    uint32_t *part_zd = nullptr) {
     GCG_TRY(ensure_chunk_plan(g));
     const ChunkPlan &pl = *g->cplan;
     const uint32_t nv = g->nv;
@@ -917,8 +977,8 @@ int warm_aggregates(gcg_graph *g, tbuf<Agg3> &agg, cudaStream_t s) {
     GCG_TRY(agg.alloc(std::max<uint32_t>(pl.nnz, 1), s));
     GCG_TRY(parts.alloc((size_t)2 * pl.nchunks + 2, s));
     const int sms = num_sms();
-    const unsigned b1 = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)nv + 255) / 256, sms * 8ull));
-    k_warm_vstat<<<b1, 256, 0, s>>>(g->indeg.get(), pl.newid.get(), nv, vstat.get());
+    k_warm_vstat<<<vstat_grid(nv), 256, 0, s>>>(g->indeg.get(), pl.newid.get(), nv, vstat.get(), g->outdeg.get(),
+                                               teleport, out, part_zd);
     if (pl.nchunks) {
         AggArgs a;
         a.col = pl.col_r.get();
@@ -1254,7 +1314,7 @@ int gcg_warm_start_rank(gcg_graph *g, const gcg_mlp *m, double teleport, double 
         const ChunkPlan &pl = *g->cplan;
         const int sms = num_sms();
         tbuf<Agg3> agg;
-        tbuf<float> stage;
+        tbuf<float> stage, pred;
         tbuf<double2> pmass;
         tbuf<uint32_t> pzd;
         tbuf<double> alpha;
@@ -1265,13 +1325,14 @@ int gcg_warm_start_rank(gcg_graph *g, const gcg_mlp *m, double teleport, double 
         const uint64_t tiles = ((uint64_t)pl.nnz + TC_ROWS - 1) / TC_ROWS;
         /* at most TC_CTAS_PER_SM CTAs of 64 tensor-memory columns per SM: well inside its 512 */
         const unsigned ib = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, sms * (uint64_t)TC_CTAS_PER_SM));
-        const unsigned zb = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)pl.nzero + 255) / 256, sms * 4ull));
-        rc = warm_aggregates(g, agg, s);
-        if (rc == GCG_OK && !dev) {
+        const unsigned zb = vstat_grid(nv);
+        if (!dev) {
             rc = stage.alloc(nv, s);
             dst = stage.get();
         }
-        if (rc == GCG_OK && (rc = pmass.alloc(ib, s)) == GCG_OK && (rc = pzd.alloc(zb, s)) == GCG_OK &&
+        if (rc == GCG_OK && (rc = pzd.alloc(zb, s)) == GCG_OK)
+            rc = warm_aggregates(g, agg, s, (float)teleport, dst, pzd.get());
+        if (rc == GCG_OK && (rc = pmass.alloc(ib, s)) == GCG_OK && (rc = pred.alloc(std::max<uint32_t>(pl.nnz, 1), s)) == GCG_OK &&
             (rc = alpha.alloc(1, s)) == GCG_OK && (rc = xpk.alloc(std::max<uint32_t>(pl.nnz, 1), s)) == GCG_OK &&
             (rc = ierr.alloc(1, s)) == GCG_OK && (rc = (cudaMemsetAsync(ierr.get(), 0, sizeof(int), s) == cudaSuccess
                                                             ? GCG_OK
@@ -1280,23 +1341,20 @@ int gcg_warm_start_rank(gcg_graph *g, const gcg_mlp *m, double teleport, double 
             k_warm_xfeat<<<xb, 256, 0, s>>>(pl.nz_rows.get(), pl.od_nz.get(), pl.nnz, g->indeg.get(), agg.get(),
                                             g->vbits, m->norm.get(), xpk.get());
             InferArgs a;
-            a.nz_rows = pl.nz_rows.get();
             a.od_nz = pl.od_nz.get();
             a.xpk = xpk.get();
             a.nnz = pl.nnz;
             a.wb = m->wb.get();
             a.teleport = (float)teleport;
-            a.out = dst;
+            a.pred = pred.get();
             a.part_mass = pmass.get();
             a.err = ierr.get();
             if (pl.nnz) k_warm_infer<<<ib, TC_ROWS, 0, s>>>(a);
             else cudaMemsetAsync(pmass.get(), 0, sizeof(double2), s);
-            k_warm_zero<<<zb, 256, 0, s>>>(pl.zero_rows.get(), pl.nzero, g->outdeg.get(), (float)teleport, dst,
-                                           pzd.get());
             k_warm_alpha<<<1, 32, 0, s>>>(pmass.get(), ib, pzd.get(), zb, nv, pl.nzero, teleport, damping,
                                           alpha.get());
             const unsigned sb = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)pl.nnz + 255) / 256, sms * 8ull));
-            k_warm_scale<<<sb, 256, 0, s>>>(pl.nz_rows.get(), pl.nnz, alpha.get(), dst);
+            k_warm_scale<<<sb, 256, 0, s>>>(pl.nz_rows.get(), pl.nnz, alpha.get(), pred.get(), dst);
             cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) rc = fail(GCG_ERR_CUDA, std::string("gcg_warm_start_rank: ") + cudaGetErrorString(e));
         }
