@@ -536,24 +536,38 @@ __global__ void __launch_bounds__(TC_ROWS, TC_CTAS_PER_SM) k_warm_infer(InferArg
  * and M_D = the part of M on D, the sweep's total is teleport*n +
  * damping*(total - total on D), which equals the total when
  *   alpha = teleport*(n - (1-damping)|Z| - damping|Z & D|) / ((1-damping)M + damping M_D). */
-__global__ void k_warm_alpha(const double2 *__restrict__ pm, uint32_t nmass, const uint32_t *__restrict__ pzd,
-                             uint32_t nzd, uint32_t nv, uint32_t nzero, double teleport, double damping,
-                             double *__restrict__ alpha) {
-    const uint32_t lane = threadIdx.x;
+__global__ void __launch_bounds__(256) k_warm_alpha(const double2 *__restrict__ pm, uint32_t nmass,
+                                                    const uint32_t *__restrict__ pzd, uint32_t nzd, uint32_t nv,
+                                                    uint32_t nzero, double teleport, double damping,
+                                                    double *__restrict__ alpha) {
+    __shared__ double s_m[8], s_md[8];
+    __shared__ unsigned long long s_zd[8];
+    const uint32_t tid = threadIdx.x;
     double M = 0.0, MD = 0.0;
     unsigned long long zd = 0;
-    for (uint32_t b = lane; b < nmass; b += 32u) {
+    for (uint32_t b = tid; b < nmass; b += 256u) {
         M += pm[b].x;
         MD += pm[b].y;
     }
-    for (uint32_t b = lane; b < nzd; b += 32u) zd += pzd[b];
+    for (uint32_t b = tid; b < nzd; b += 256u) zd += pzd[b];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         M += __shfl_xor_sync(0xFFFFFFFFu, M, o);
         MD += __shfl_xor_sync(0xFFFFFFFFu, MD, o);
         zd += __shfl_xor_sync(0xFFFFFFFFu, zd, o);
     }
-    if (lane == 0) {
+    if ((tid & 31u) == 0) {
+        s_m[tid >> 5] = M;
+        s_md[tid >> 5] = MD;
+        s_zd[tid >> 5] = zd;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < 8; ++w) {
+            M += s_m[w];
+            MD += s_md[w];
+            zd += s_zd[w];
+        }
         const double den = (1.0 - damping) * M + damping * MD;
         const double num = teleport * ((double)nv - (1.0 - damping) * (double)nzero - damping * (double)zd);
         *alpha = (den > 0.0 && num > 0.0) ? num / den : 1.0;
@@ -1351,7 +1365,7 @@ int gcg_warm_start_rank(gcg_graph *g, const gcg_mlp *m, double teleport, double 
             a.err = ierr.get();
             if (pl.nnz) k_warm_infer<<<ib, TC_ROWS, 0, s>>>(a);
             else cudaMemsetAsync(pmass.get(), 0, sizeof(double2), s);
-            k_warm_alpha<<<1, 32, 0, s>>>(pmass.get(), ib, pzd.get(), zb, nv, pl.nzero, teleport, damping,
+            k_warm_alpha<<<1, 256, 0, s>>>(pmass.get(), ib, pzd.get(), zb, nv, pl.nzero, teleport, damping,
                                           alpha.get());
             const unsigned sb = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)pl.nnz + 255) / 256, sms * 8ull));
             k_warm_scale<<<sb, 256, 0, s>>>(pl.nz_rows.get(), pl.nnz, alpha.get(), pred.get(), dst);
