@@ -657,7 +657,7 @@ __device__ __forceinline__ void tile_gemm(float (&acc)[8][4], const float *pa, c
  * (4 sg .. and 64 + 4 sg ..) x 4 features (4 fg ..) of the activations, and 4 x 4 of dW2
  * (rows gj + 16 i, columns gk + 16 i), which stay in registers over the block's tiles;
  * biases and W3 are added up from the activations where they arise. 1 M samples take
- * 0.70 ms (13.3 k FMAs a sample: 0.37 ms at the FP32 rate); what bounds it is shared
+ * 0.72 ms (13.3 k FMAs a sample: 0.37 ms at the FP32 rate); what bounds it is shared
  * memory, 3.0 k quarter-warp reads per warp and tile against 1.6 k FMA cycles. With a
  * thread per sample and one block of 128 threads per SM, a warp per scheduler, they took
  * 2.64 ms. */
@@ -694,6 +694,28 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 2) k_mlp_fwd_bwd(TrainArgs a) {
         for (int k = 0; k < 4; ++k) gW2[i][k] = 0.0f;
     }
     const uint32_t gj = (warp & 1u) * 8u + (lane & 7u), gk = (warp >> 1) * 4u + (lane >> 3);
+
+    /* The weights' sums go to the block's slot every FLUSH_TILES tiles: a float sum over all
+     * of a block's samples (3.4 k of 1 M) loses more than its parts do. With the blocks'
+     * slots added in FP64 the gradient over 1 M samples is 5e-8 off 64-bit arithmetic, as
+     * one float chain 1.8e-7 to 3.2e-7; the call takes 0.786 ms in place of 0.764. */
+    constexpr uint32_t FLUSH_TILES = 4;
+    float *out = FWD_ONLY ? nullptr : a.part + (size_t)blockIdx.x * (NP + 1);
+    uint32_t since = 0;
+    bool flushed = false;
+    auto flush = [&]() {
+        auto add = [&](float *p, float &g) {
+            *p = flushed ? *p + g : g;
+            g = 0.0f;
+        };
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) add(out + OW2 + (gj + 16 * i) * NH + gk + 16 * k, gW2[i][k]);
+        add(out + OW1 + (tid >> 2) * NIN + 2 * (tid & 3u), gW1[0]);
+        add(out + OW1 + (tid >> 2) * NIN + 2 * (tid & 3u) + 1, gW1[1]);
+        flushed = true;
+    };
 
     /* a thread's half of a sample's inputs */
     const uint32_t xs = tid >> 1, xh = (tid & 1u) * 4u;
@@ -835,16 +857,14 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 2) k_mlp_fwd_bwd(TrainArgs a) {
                 }
             }
         }
+        if (++since == FLUSH_TILES) {
+            flush();
+            since = 0;
+        }
         __syncthreads(); /* the inputs have been read */
     }
     if (FWD_ONLY) return;
-    float *out = a.part + (size_t)blockIdx.x * (NP + 1);
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) out[OW2 + (gj + 16 * i) * NH + gk + 16 * k] = gW2[i][k];
-    out[OW1 + (tid >> 2) * NIN + 2 * (tid & 3u)] = gW1[0];
-    out[OW1 + (tid >> 2) * NIN + 2 * (tid & 3u) + 1] = gW1[1];
+    if (since || !flushed) flush();
     /* biases, W3: the 16 sample groups' parts in order; b3 and the loss over the samples */
     float *red = sH1;
     __syncthreads();
@@ -895,9 +915,10 @@ __device__ __forceinline__ bool is_weight(int i) {
 __global__ void k_mlp_adam(AdamArgs a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < NP) {
-        float gsum = 0.0f;
+        double total = 0.0;
 #pragma unroll 16
-        for (uint32_t b = 0; b < a.nblocks; ++b) gsum += a.part[(size_t)b * (NP + 1) + i];
+        for (uint32_t b = 0; b < a.nblocks; ++b) total += (double)a.part[(size_t)b * (NP + 1) + i];
+        const float gsum = (float)total;
         if (a.grad_out) a.grad_out[i] = gsum;
         if (a.apply) {
             const float m = a.beta1 * a.m[i] + (1.0f - a.beta1) * gsum;
