@@ -361,17 +361,17 @@ def run_extras(args):
     del s, d
     bms = min(t_build[1:])
     # the LSD sort of (dst, src) keys: ceil(b/8) 8-bit digit passes per half, b = bits of a vertex id;
-    # a pass reads every key twice (histogram, scatter) and writes it once: 24 bytes per key
+    # a pass reads and writes every key once: 16 bytes per key
     vb = max(1, int(args.scale))
     passes = 2 * ((vb + 7) // 8)
-    pass_bytes = 24.0 * m * passes
+    pass_bytes = 16.0 * m * passes
     out["sharder"] = {"raw_edges": m, "ms": bms, "first_call_ms": t_build[0], "sort_bytes_16E": 16.0 * m,
                       "frac_of_16E_at_hbm_peak": 16.0 * m / peak / 1e6 / bms,
                       "radix_passes": passes, "radix_pass_bytes": pass_bytes,
                       "frac_of_radix_pass_bytes_at_hbm_peak": pass_bytes / peak / 1e6 / bms,
                       "note": "dedup + in-CSR + degrees + 64 intervals, whole build timed; 16E is the one-pass "
-                              "lower bound of a sort, radix_pass_bytes what the LSD passes move (24 B per key "
-                              "per pass); the scatter pass is bound by shared-memory bank conflicts"}
+                              "lower bound of a sort, radix_pass_bytes what the LSD passes move (16 B per key "
+                              "per pass); a pass is bound by shared-memory bank conflicts"}
 
     # ---- the vertex-API in-memory program (bit-exact Gauss-Seidel) to the tolerance ----
     s, d = dev_edges(args.scale, args.ef << args.scale, args.seed)
@@ -385,8 +385,8 @@ def run_extras(args):
                            "converged": st.converged, "residual": st.residual, "levels": st.levels,
                            "ms": st.device_ms, "GTEPS": g.num_edges * st.sweeps / st.device_ms / 1e6,
                            "note": "example_apps/pagerank.cpp in-memory program, id-ordered Gauss-Seidel, "
-                                   "bit-exact; levels of the u<v in-edge dependency schedule, one launch each "
-                                   "per sweep (CUDA graph); time excludes the level schedule's construction"}
+                                   "bit-exact; levels of the u<v in-edge dependency schedule, a grid "
+                                   "barrier between them; time excludes the level schedule's construction"}
         del o
 
     # ---- connected components (and triangles at scale 20) ----

@@ -655,7 +655,7 @@ __device__ __forceinline__ void tile_gemm(float (&acc)[8][4], const float *pa, c
  * iteration, FP32 throughout: every layer and every weight gradient is a small block GEMM
  * over shared-memory operands with its outputs in registers. A thread takes 8 samples
  * (4 sg .. and 64 + 4 sg ..) x 4 features (4 fg ..) of the activations, and 4 x 4 of dW2
- * (rows gj + 16 i, columns gk + 16 i), which stay in registers over the block's tiles;
+ * (rows gj + 16 i, columns gk + 16 i), which stay in registers for four tiles;
  * biases and W3 are added up from the activations where they arise. 1 M samples take
  * 0.72 ms (13.3 k FMAs a sample: 0.37 ms at the FP32 rate); what bounds it is shared
  * memory, 3.0 k quarter-warp reads per warp and tile against 1.6 k FMA cycles. With a
