@@ -8,14 +8,13 @@
  * teleport * exp(y) then runs to the same residual as from the uniform start.
  *
  * Kernels
- *   k_warm_vstat   per vertex: {log(1+indeg), indeg} packed in 8 bytes, stored at
- *                  the vertex's out-degree rank (the PageRank relabelling); the ranks
- *                  of the vertices without in-edges
+ *   k_warm_vstat   per vertex: its in-degree, stored at its out-degree rank (the
+ *                  PageRank relabelling); the ranks of the vertices without in-edges
  *   k_warm_agg_edges / k_warm_agg_fix   per vertex with in-edges: sum and max of
  *                  L(u) = log(1+indeg(u)) over in-neighbours u and the sum of
  *                  indeg(u), on the PageRank chunk plan: one warp per 256 in-edges
- *                  (edge-balanced whatever the degrees), one 8-byte gather per
- *                  edge (the 24576 highest out-degree sources from shared memory),
+ *                  (edge-balanced whatever the degrees), one 4-byte gather per
+ *                  edge (the 41728 highest out-degree sources from shared memory),
  *                  a warp segmented reduction of (sum, max, sum), rows crossing
  *                  chunks completed in chunk order
  *   k_warm_infer   the network on the 5th-generation tensor cores (tcgen05.mma,
@@ -85,27 +84,27 @@ struct AggArgs {
     const uint32_t *chunk_nz;
     uint64_t ne;
     uint32_t nchunks, hub;
-    const uint2 *vstat; /* {L(u) as float bits, indeg(u)} by relabelled id */
+    const uint32_t *deg; /* indeg(u) by relabelled id */
 };
 struct AggOut {
     Agg3 *nzsum, *head_part, *tail_part;
 };
-constexpr uint32_t AGG_HUB_MAX = 24576; /* 192 KB of {L, indeg} pairs */
+constexpr uint32_t AGG_HUB_MAX = 41728; /* in-degrees in shared memory: 164 KB, which leaves L1 its share */
 
-/* vstat of every vertex; with out given, also the part of the result that needs no network:
+/* deg of every vertex; with out given, also the part of the result that needs no network:
  * vertices without in-edges get exactly teleport, and part_zd[block] counts those of them
  * that also lack out-edges. (In vertex order those stores are coalesced: as a pass over the
  * list of such rows, which is in out-degree order, they took 19 us at R-MAT scale 22.) */
 __global__ void __launch_bounds__(256) k_warm_vstat(const uint32_t *__restrict__ indeg,
                                                     const uint32_t *__restrict__ newid, uint32_t nv,
-                                                    uint2 *__restrict__ vstat, const uint32_t *__restrict__ outdeg,
+                                                    uint32_t *__restrict__ deg, const uint32_t *__restrict__ outdeg,
                                                     float teleport, float *__restrict__ out,
                                                     uint32_t *__restrict__ part_zd) {
     __shared__ uint32_t s_c[8];
     uint32_t c = 0;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
         const uint32_t d = indeg[v];
-        vstat[newid[v]] = make_uint2(__float_as_uint(log1pf((float)d)), d);
+        deg[newid[v]] = d;
         if (out && d == 0u) {
             out[v] = teleport;
             c += outdeg[v] == 0u;
@@ -123,34 +122,42 @@ __global__ void __launch_bounds__(256) k_warm_vstat(const uint32_t *__restrict__
     }
 }
 
-__device__ __forceinline__ uint2 ld_keep_u2(const uint2 *p, uint64_t pol) {
-    uint2 r;
-    asm("ld.global.nc.L2::cache_hint.v2.u32 {%0,%1}, [%2], %3;" : "=r"(r.x), "=r"(r.y) : "l"(p), "l"(pol));
+__device__ __forceinline__ uint32_t ld_keep_u32(const uint32_t *p, uint64_t pol) {
+    uint32_t r;
+    asm("ld.global.nc.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(r) : "l"(p), "l"(pol));
     return r;
 }
 
+/* The edges gather the in-degree alone, 4 bytes, and form its logarithm themselves: as
+ * {L, indeg} pairs of 8 bytes half as many sources fitted the hub, and the kernel waited
+ * on the L1's requests to L2 (71 % of their rate) and on the pairs' bank conflicts with
+ * 30 % of its issue slots busy. R-MAT scale 22: 201 -> 174 us, 65 % of the slots. */
 __global__ void __launch_bounds__(EDGE_THREADS, 1) k_warm_agg_edges(AggArgs a, AggOut o) {
-    extern __shared__ uint2 s_vs[];
+    extern __shared__ uint32_t s_deg[];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint64_t pol_stream = policy_evict_first(), pol_keep = policy_evict_last();
-    for (uint32_t i = threadIdx.x; i < a.hub; i += blockDim.x) s_vs[i] = a.vstat[i];
+    for (uint32_t i = threadIdx.x; i < a.hub; i += blockDim.x) s_deg[i] = a.deg[i];
     __syncthreads();
     uint32_t ch = gwarp;
     uint32_t col[EPL], meta = 0, base = 0;
     if (ch < a.nchunks) load_chunk(a, ch, lane, pol_stream, col, meta, base);
     for (; ch < a.nchunks; ch += nwarps) {
-        Agg3 val[EPL];
+        uint32_t deg[EPL];
 #pragma unroll
         for (int j = 0; j < EPL; ++j) {
             const uint32_t x = col[j];
-            const uint2 w = x < a.hub ? s_vs[x] : ld_keep_u2(a.vstat + x, pol_keep);
-            const float L = __uint_as_float(w.x);
-            val[j] = Agg3{L, L, (float)w.y};
+            deg[j] = x < a.hub ? s_deg[x] : ld_keep_u32(a.deg + x, pol_keep);
         }
         const uint32_t cm = meta, cb = base;
         if (ch + nwarps < a.nchunks) load_chunk(a, ch + nwarps, lane, pol_stream, col, meta, base);
+        Agg3 val[EPL];
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) {
+            const float d = (float)deg[j], L = log1pf(d);
+            val[j] = Agg3{L, L, d};
+        }
         reduce_chunk_to(o, ch, lane, val, cm, cb, a.ne);
     }
 }
@@ -1006,13 +1013,13 @@ int warm_aggregates(gcg_graph *g, tbuf<Agg3> &agg, cudaStream_t s, float telepor
     GCG_TRY(ensure_chunk_plan(g));
     const ChunkPlan &pl = *g->cplan;
     const uint32_t nv = g->nv;
-    tbuf<uint2> vstat;
+    tbuf<uint32_t> deg;
     tbuf<Agg3> parts;
-    GCG_TRY(vstat.alloc(nv, s));
+    GCG_TRY(deg.alloc(nv, s));
     GCG_TRY(agg.alloc(std::max<uint32_t>(pl.nnz, 1), s));
     GCG_TRY(parts.alloc((size_t)2 * pl.nchunks + 2, s));
     const int sms = num_sms();
-    k_warm_vstat<<<vstat_grid(nv), 256, 0, s>>>(g->indeg.get(), pl.newid.get(), nv, vstat.get(), g->outdeg.get(),
+    k_warm_vstat<<<vstat_grid(nv), 256, 0, s>>>(g->indeg.get(), pl.newid.get(), nv, deg.get(), g->outdeg.get(),
                                                teleport, out, part_zd);
     if (pl.nchunks) {
         AggArgs a;
@@ -1022,16 +1029,16 @@ int warm_aggregates(gcg_graph *g, tbuf<Agg3> &agg, cudaStream_t s, float telepor
         a.ne = g->ne;
         a.nchunks = pl.nchunks;
         a.hub = std::min<uint32_t>(nv, AGG_HUB_MAX);
-        a.vstat = vstat.get();
+        a.deg = deg.get();
         AggOut o;
         o.nzsum = agg.get();
         o.head_part = parts.get();
         o.tail_part = parts.get() + pl.nchunks + 1;
-        const size_t smem = (size_t)AGG_HUB_MAX * sizeof(uint2);
+        const size_t smem = (size_t)AGG_HUB_MAX * sizeof(uint32_t);
         GCG_CUDA(cudaFuncSetAttribute(k_warm_agg_edges, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         const unsigned grid = (unsigned)std::max<uint64_t>(
             1, std::min<uint64_t>(((uint64_t)pl.nchunks * 32 + EDGE_THREADS - 1) / EDGE_THREADS, (uint64_t)sms));
-        k_warm_agg_edges<<<grid, EDGE_THREADS, (size_t)a.hub * sizeof(uint2), s>>>(a, o);
+        k_warm_agg_edges<<<grid, EDGE_THREADS, (size_t)a.hub * sizeof(uint32_t), s>>>(a, o);
         if (pl.nsplit) {
             const unsigned fb = (unsigned)std::max<uint64_t>(
                 1, std::min<uint64_t>(((uint64_t)pl.nsplit + 255) / 256, sms * 8ull));
