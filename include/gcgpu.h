@@ -243,10 +243,14 @@ int gcg_pagerank(gcg_graph *g, const gcg_pr_params *params, float *out_rank, gcg
  * that leaves the SM its 164 KB shared-memory carve-out, so L1 keeps ~92 KB) and
  * chunk_run 1, the fastest measured at R-MAT scale 24. gcg_pagerank_autotune
  * times `sweeps` fixed sweeps (the whole sweep, device time) of each candidate
- * (hub entries {0, 16384, 32768, 41724, 49152, the plan's} x runs {1, 2, 4, 16},
- * then 2..4 source tiers of the chosen hub, gcg_pagerank_set_tiers), keeps the
+ * (the one-launch solve that a graph of at most 2^25 edges gets by default; hub
+ * entries {0, 16384, 32768, 41724, 49152, the plan's} x runs {1, 2, 4, 16}; then
+ * 2..4 source tiers of the chosen hub, gcg_pagerank_set_tiers), keeps the
  * fastest for later calls on this graph and reports it (outputs may be NULL;
- * gcg_pagerank_get_tiers gives the tier count chosen). */
+ * gcg_pagerank_get_tiers gives the tier count chosen; the one-launch solve is
+ * reported as the default values). gcg_pagerank_set_config and
+ * gcg_pagerank_set_tiers select the edge kernel that they configure, whatever
+ * the values, until gcg_pagerank_autotune chooses again. */
 int gcg_pagerank_set_config(gcg_graph *g, uint32_t hub_entries, uint32_t chunk_run);
 int gcg_pagerank_get_config(gcg_graph *g, uint32_t *hub_entries, uint32_t *chunk_run);
 int gcg_pagerank_autotune(gcg_graph *g, int sweeps, uint32_t *hub_entries, uint32_t *chunk_run, double *ms_per_sweep);
