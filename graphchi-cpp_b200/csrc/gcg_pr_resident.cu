@@ -52,6 +52,11 @@ constexpr uint64_t ROW_COST = 3;
  * misses the hub ~1 cycle, and a source of out-degree d is gathered d / CTAs times
  * per CTA */
 constexpr uint32_t HUB_MIN_DEGREE = 16;
+/* Vertices without in-edges to a CTA, where the chunks alone ask for fewer CTAs: the CTAs
+ * walk them four times a solve, each step a chain of dependent loads. One to a thread: 4 M
+ * vertices with 4,096 edges, 3 sweeps: 9.7 ms by the chunks' one CTA, 0.11 by 148; 65,536
+ * with 4,096: 0.183, 0.053 (0.056 with 2,048 to a CTA, 0.059 with 4,096). */
+constexpr uint32_t ZERO_ROWS = EDGE_THREADS;
 /* polls of a wait: each takes at least an L2 round trip (~0.6 us), so seconds */
 constexpr long long RES_SPIN = 1ll << 23;
 
@@ -443,7 +448,8 @@ int pagerank_resident(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
         GCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pr_resident, EDGE_THREADS,
                                                                HUB_DEFAULT * 4u));
         if (!coop || per_sm < 1) return GCG_OK; /* the queued kernels take it */
-        const uint32_t ncta = std::max(1u, std::min((uint32_t)num_sms(), (pl.nchunks + WARPS / 2 - 1) / (WARPS / 2)));
+        const uint32_t ncta = std::min((uint32_t)num_sms(), std::max((pl.nchunks + WARPS / 2 - 1) / (WARPS / 2),
+                                                                     (pl.nzero + ZERO_ROWS - 1) / ZERO_ROWS));
         GCG_TRY(w.res_rg.alloc(ncta));
         GCG_TRY(w.res_ctl.alloc(2 + ncta));
         GCG_TRY(w.res_bres.alloc(2 * (size_t)ncta));
