@@ -109,17 +109,50 @@ __global__ void __launch_bounds__(256) k_gs_round(uint32_t r, const uint32_t *__
  * ascending source order (a float sum is not associative). A thread's and a warp's
  * row have all their loads in flight at once: with 32 in-edges per thread, eight at a
  * time, and a warp's batches one ahead, their latencies made most of a small level
- * (scale 14: 8.4 against 6.0 us a level). */
+ * (scale 14: 8.4 against 6.0 us a level).
+ *
+ * A wide level has more rows than threads wait for: there what counts is how many rows are
+ * under way. Where its rows of up to GS_WIDE_THREAD in-edges outnumber the warps they go to
+ * the threads (3 sweeps of a uniform graph of 16 in-edges, 4 M vertices: 8.8 ms by warps,
+ * 1.83 by threads; one launch per level, a full grid each, took 3.2), and where its rows of
+ * up to GS_WIDE_WARP outnumber half the warps, four a group, they go to the warps (100,000
+ * rows of 300 in-edges in one level: 2.89 -> 0.68 ms). */
 constexpr uint32_t GS_THREAD_MAX = 8, GS_WARP_MAX = 256;
-constexpr int GS_CLASSES = 4; /* segments per level: thread, warp, block, (unused) */
+constexpr uint32_t GS_WIDE_THREAD = 32, GS_WIDE_WARP = 4096;
+/* Rows that a warp of a level takes one by one, adding from shuffles: the quickest for one
+ * row. Beyond, it loads what it needs of 32 rows at once, and the next row's columns behind
+ * a row's adds, which go through shared memory: with all warps at it shuffles are bound by
+ * their rate (500,000 rows of 100 in-edges: 1.59 -> 1.12 ms). */
+constexpr uint32_t GS_FEW_ROUNDS = 4;
+constexpr int GS_CLASSES = 4; /* segments per level: thread, thread in a wide level, warp, block */
+
+/* rows of level l with up to GS_WIDE_THREAD in-edges that are beyond the thread class: mid[2 l];
+ * with up to GS_WIDE_WARP that are beyond the warp class: mid[2 l + 1] */
+__global__ void k_level_mid(const uint32_t *__restrict__ level, const uint32_t *__restrict__ rowptr, uint32_t nv,
+                            uint32_t *__restrict__ mid) {
+    const uint64_t end = ((uint64_t)nv + 31u) & ~31ull; /* whole warps: the ballot below */
+    for (uint64_t v = blockIdx.x * blockDim.x + threadIdx.x; v < end; v += gridDim.x * blockDim.x) {
+        const uint32_t d = v < nv ? rowptr[v + 1] - rowptr[v] : 0u;
+        const bool counts = (d > GS_THREAD_MAX && d <= GS_WIDE_THREAD) || (d > GS_WARP_MAX && d <= GS_WIDE_WARP);
+        const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, counts);
+        if (!counts) continue;
+        uint32_t *const at = mid + 2 * (size_t)level[v] + (d > GS_WARP_MAX);
+        const uint32_t same = __match_any_sync(lanes, (unsigned long long)at);
+        if ((threadIdx.x & 31u) == (uint32_t)__ffs((int)same) - 1u) atomicAdd(at, (uint32_t)__popc(same));
+    }
+}
 
 /* sort key: level, class, vertex id */
 __global__ void k_level_keys(const uint32_t *__restrict__ level, const uint32_t *__restrict__ rowptr, uint32_t nv,
-                             uint32_t vbits, uint64_t *keys) {
+                             const uint32_t *__restrict__ mid, uint32_t warps, uint32_t vbits, uint64_t *keys) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
-        const uint32_t d = rowptr[v + 1] - rowptr[v];
-        const uint64_t cls = d <= GS_THREAD_MAX ? 0u : d <= GS_WARP_MAX ? 1u : 2u;
-        keys[v] = ((((uint64_t)level[v] << 2) | cls) << vbits) | v;
+        const uint32_t d = rowptr[v + 1] - rowptr[v], l = level[v], *m = mid + 2 * (size_t)l;
+        const uint64_t cls = d <= GS_THREAD_MAX                       ? 0u
+                             : d <= GS_WIDE_THREAD && m[0] > warps    ? 1u
+                             : d <= GS_WARP_MAX                       ? 2u
+                             : d <= GS_WIDE_WARP && m[1] > warps / 2u ? 2u
+                                                                      : 3u;
+        keys[v] = ((((uint64_t)l << 2) | cls) << vbits) | v;
     }
 }
 
@@ -139,6 +172,13 @@ __global__ void k_level_bounds(const uint64_t *__restrict__ keys, uint32_t nv, u
     }
 }
 
+/* what a sweep reads of a level: where its thread, warp and block class begin, and its end */
+__global__ void k_level_pack(const uint32_t *__restrict__ seg, uint32_t nlev, uint4 *__restrict__ off) {
+    for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < nlev; l += gridDim.x * blockDim.x) {
+        const uint32_t *s = seg + (size_t)GS_CLASSES * l;
+        off[l] = make_uint4(s[0], s[2], s[3], s[4]);
+    }
+}
 
 /* pagerank.cpp:124,137-139: pr starts at 0.15; iteration 0 sets 1/outc when outc > 0 */
 __global__ void k_gs_init(uint32_t nv, const uint32_t *__restrict__ outdeg, float reset, float *pr) {
@@ -233,6 +273,8 @@ struct GsGroup {
         uint32_t pos;
     } told[2];
 };
+
+static_assert(sizeof(GsGroup) % 16 == 0, "the second group's 128-bit reads");
 
 __device__ __forceinline__ void group_sync(uint32_t grp) {
     asm volatile("bar.sync %0, %1;" ::"r"(grp + 1u), "n"(GS_GROUP) : "memory");
@@ -380,7 +422,8 @@ __device__ __forceinline__ float group_add(GsGroup &g, const float *sv, uint32_t
 }
 
 struct GsArgs {
-    const uint32_t *order, *off; /* off: GS_CLASSES entries per level */
+    const uint32_t *order;
+    const uint4 *off; /* per level: first vertex of the thread, warp and block class, end */
     uint32_t nlev;
     const uint32_t *rowptr, *col, *outdeg;
     const float *pr_old;
@@ -427,10 +470,10 @@ __device__ __forceinline__ bool gs_wait(const GsArgs &a, uint32_t target) {
  * launch, one CTA per SM). A level's vertices are independent. A block-class vertex
  * is taken by a group of 256 threads: the threads copy the in-edge values of a step
  * into shared memory, GS_DEPTH - 1 steps ahead, and group_add adds a step. A
- * warp-class vertex by a warp: all values in flight, then added in order from
- * shuffles. A thread-class vertex by a thread: all loads in flight, then the adds. Block-class vertices go to the CTAs from the
- * first on, the others from the last warp down, so that a small level's rows lie on
- * different SMs. What does not change within a sweep (a level's vertices, row bounds
+ * warp-class vertex by a warp: 256 values in flight, then added in order from
+ * shuffles (or shared memory, GS_FEW_ROUNDS). A thread-class vertex by a thread, eight
+ * loads in flight, then the adds. Block-class vertices go to the CTAs from the first on,
+ * the others from the last warp down, so that a small level's rows lie on different SMs. What does not change within a sweep (a level's vertices, row bounds
  * and first columns) is loaded while the CTA waits for the others. */
 template <bool EDGE, bool TRACK>
 __global__ void __launch_bounds__(GS_THREADS, 1) k_gs_sweep(GsArgs a) {
@@ -489,7 +532,30 @@ __global__ void __launch_bounds__(GS_THREADS, 1) k_gs_sweep(GsArgs a) {
         }
     };
 
-    uint4 o = ((const uint4 *)a.off)[0], on = a.nlev > 1 ? ((const uint4 *)a.off)[1] : o;
+    /* one row of many by this warp: the values through shared memory, then every lane adds them in
+     * order. pc: its first columns, then those of the warp's next row [njb, nje) */
+    float *const wv = (float *)(s_raw + GS_GROUPS * sizeof(GsGroup)) + (threadIdx.x >> 5) * GS_WARP_MAX;
+    auto warp_row = [&](uint32_t v, uint32_t jb, uint32_t je, uint32_t od, uint32_t njb, uint32_t nje) {
+        float sum = 0.0f;
+        for (uint32_t left = je - jb;;) {
+            const uint32_t n = min(left, GS_WARP_MAX);
+            float x[GS_WARP_MAX / 32];
+#pragma unroll
+            for (uint32_t q = 0; q < GS_WARP_MAX / 32; ++q) x[q] = 32u * q + lane < n ? value(pc[q], v) : 0.0f;
+            left -= n;
+            row_columns(left ? je - left : njb, left ? je : nje, pc);
+#pragma unroll
+            for (uint32_t q = 0; q < GS_WARP_MAX / 32; ++q)
+                if (32u * q < n) wv[32u * q + lane] = x[q];
+            __syncwarp();
+            sum = add_in_order(sum, wv, 0u, n);
+            __syncwarp();
+            if (!left) break;
+        }
+        if (lane == 0) gs_apply<EDGE, TRACK>(v, sum, od, pr_new, a.val, a.delta, a.reset, a.damping);
+    };
+
+    uint4 o = a.off[0], on = a.nlev > 1 ? a.off[1] : o;
     prefetch(o);
     uint32_t target = a.meets;
     for (uint32_t l = 0; l < a.nlev; ++l) {
@@ -536,10 +602,11 @@ __global__ void __launch_bounds__(GS_THREADS, 1) k_gs_sweep(GsArgs a) {
             if (tid == 0) gs_apply<EDGE, TRACK>(v, sum, od, pr_new, a.val, a.delta, a.reset, a.damping);
             group_sync(grp);
         }
-        for (uint32_t k = rev; k < nw; k += nwarps) { /* warp class */
+        uint32_t kw = rev; /* warp class */
+        for (; kw < nw && nw <= GS_FEW_ROUNDS * nwarps; kw += nwarps) {
             uint32_t v = pv, jb = pjb, je = pje, od = pod;
             if (!ready) {
-                v = __ldg(a.order + o.y + k);
+                v = __ldg(a.order + o.y + kw);
                 jb = __ldg(a.rowptr + v);
                 je = __ldg(a.rowptr + v + 1);
                 od = __ldg(a.outdeg + v);
@@ -547,20 +614,42 @@ __global__ void __launch_bounds__(GS_THREADS, 1) k_gs_sweep(GsArgs a) {
             }
             ready = false;
             float x[GS_WARP_MAX / 32], sum = 0.0f;
+            for (uint32_t left = je - jb;;) {
 #pragma unroll
-            for (uint32_t q = 0; q < GS_WARP_MAX / 32; ++q)
-                x[q] = (uint64_t)jb + 32u * q + lane < je ? value(pc[q], v) : 0.0f;
+                for (uint32_t q = 0; q < GS_WARP_MAX / 32; ++q) x[q] = 32u * q + lane < left ? value(pc[q], v) : 0.0f;
+                const bool more = left > GS_WARP_MAX;
+                if (more) row_columns(je - left + GS_WARP_MAX, je, pc);
 #pragma unroll
-            for (uint32_t q = 0; q < GS_WARP_MAX / 32; ++q) {
-                const uint32_t n = je - jb > 32u * q ? je - jb - 32u * q : 0u;
-                if (n == 0u) break;
+                for (uint32_t q = 0; q < GS_WARP_MAX / 32; ++q) {
+                    const uint32_t n = left > 32u * q ? left - 32u * q : 0u;
+                    if (n == 0u) break;
 #pragma unroll
-                for (uint32_t i = 0; i < 32u; ++i) { /* in order, in every lane */
-                    const float z = __shfl_sync(0xFFFFFFFFu, x[q], (int)i);
-                    if (i < n) sum += z;
+                    for (uint32_t i = 0; i < 32u; ++i) { /* in order, in every lane */
+                        const float z = __shfl_sync(0xFFFFFFFFu, x[q], (int)i);
+                        if (i < n) sum += z;
+                    }
                 }
+                if (!more) break;
+                left -= GS_WARP_MAX;
             }
             if (lane == 0) gs_apply<EDGE, TRACK>(v, sum, od, pr_new, a.val, a.delta, a.reset, a.damping);
+        }
+        for (; kw < nw; kw += 32u * nwarps) { /* a lane loads what the warp needs of one row in 32 */
+            uint32_t v = 0, jb = 0, je = 0, od = 0;
+            if (kw + (uint64_t)lane * nwarps < nw) {
+                v = __ldg(a.order + o.y + kw + lane * nwarps);
+                jb = __ldg(a.rowptr + v);
+                je = __ldg(a.rowptr + v + 1);
+                od = __ldg(a.outdeg + v);
+            }
+            ready = false;
+            row_columns(__shfl_sync(0xFFFFFFFFu, jb, 0), __shfl_sync(0xFFFFFFFFu, je, 0), pc);
+            for (uint32_t r = 0; r < 32u && kw + r * nwarps < nw; ++r) {
+                const uint32_t njb = __shfl_sync(0xFFFFFFFFu, jb, (int)r + 1), nje = __shfl_sync(0xFFFFFFFFu, je, (int)r + 1);
+                warp_row(__shfl_sync(0xFFFFFFFFu, v, (int)r), __shfl_sync(0xFFFFFFFFu, jb, (int)r),
+                         __shfl_sync(0xFFFFFFFFu, je, (int)r), __shfl_sync(0xFFFFFFFFu, od, (int)r),
+                         r < 31u ? njb : 0u, r < 31u ? nje : 0u);
+            }
         }
         /* thread class: warps past those of the warp class first */
         for (uint64_t k = (uint64_t)(rev >= nw % nwarps ? rev - nw % nwarps : rev + nwarps - nw % nwarps) * 32u + lane;
@@ -573,20 +662,29 @@ __global__ void __launch_bounds__(GS_THREADS, 1) k_gs_sweep(GsArgs a) {
                 je = __ldg(a.rowptr + v + 1);
                 od = __ldg(a.outdeg + v);
             }
-            float x[GS_THREAD_MAX], sum = 0.0f;
+            float sum = 0.0f;
+            if (!have) {
 #pragma unroll
-            for (uint32_t i = 0; i < GS_THREAD_MAX; ++i)
-                x[i] = jb + i < je ? value(have ? pc[i] : __ldg(a.col + jb + i), v) : 0.0f;
+                for (uint32_t i = 0; i < GS_THREAD_MAX; ++i) pc[i] = jb + i < je ? __ldg(a.col + jb + i) : 0u;
+            }
+            for (uint32_t j = jb; j < je; j += GS_THREAD_MAX) { /* the next columns with these values in flight */
+                float x[GS_THREAD_MAX];
 #pragma unroll
-            for (uint32_t i = 0; i < GS_THREAD_MAX; ++i)
-                if (jb + i < je) sum += x[i];
+                for (uint32_t i = 0; i < GS_THREAD_MAX; ++i) x[i] = j + i < je ? value(pc[i], v) : 0.0f;
+#pragma unroll
+                for (uint32_t i = 0; i < GS_THREAD_MAX; ++i)
+                    if (j + GS_THREAD_MAX + i < je) pc[i] = __ldg(a.col + j + GS_THREAD_MAX + i);
+#pragma unroll
+                for (uint32_t i = 0; i < GS_THREAD_MAX; ++i)
+                    if (j + i < je) sum += x[i];
+            }
             ready = false;
             gs_apply<EDGE, TRACK>(v, sum, od, pr_new, a.val, a.delta, a.reset, a.damping);
         }
         if (l + 1 == a.nlev) break;
         gs_arrive(a);
         o = on;
-        if (l + 2 < a.nlev) on = ((const uint4 *)a.off)[l + 2];
+        if (l + 2 < a.nlev) on = a.off[l + 2];
         prefetch(o);
         target += gridDim.x;
         if (!gs_wait(a, target)) return;
@@ -671,11 +769,11 @@ inline unsigned vgrid(uint32_t n) {
 }  // namespace
 
 /* Level schedule of the id-ordered dependency DAG: order[] (vertices by
- * (level, class, id)) and off[GS_CLASSES * l + c] = first index of class c of
- * level l, nlev levels. */
+ * (level, class, id)) and where each of the nlev levels' classes lie in it. */
 struct GsPlan {
     uint32_t nlev = 0;
-    dbuf<uint32_t> order, off;
+    dbuf<uint32_t> order;
+    dbuf<uint4> off;
 };
 
 void free_gs_plan(GsPlan *p) { delete p; }
@@ -749,15 +847,21 @@ static int build_gs_plan(gcg_graph *g, GsPlan &pl) {
     tbuf<uint64_t> keys, tmp;
     GCG_TRY(keys.alloc(nv, s));
     GCG_TRY(tmp.alloc(nv, s));
-    k_level_keys<<<vgrid(nv), 256, 0, s>>>(level.get(), g->in_rowptr.get(), nv, g->vbits, keys.get());
+    tbuf<uint32_t> mid, seg;
+    GCG_TRY(mid.alloc(2 * (size_t)pl.nlev, s));
+    GCG_CUDA(cudaMemsetAsync(mid.get(), 0, (size_t)pl.nlev * 8, s));
+    k_level_mid<<<vgrid(nv), 256, 0, s>>>(level.get(), g->in_rowptr.get(), nv, mid.get());
+    k_level_keys<<<vgrid(nv), 256, 0, s>>>(level.get(), g->in_rowptr.get(), nv, mid.get(),
+                                           (uint32_t)num_sms() * (GS_THREADS / 32), g->vbits, keys.get());
     uint64_t *sorted = nullptr;
     GCG_TRY(radix_sort_u64(keys.get(), tmp.get(), nv, (int)g->vbits, (int)(g->vbits + 2 + lbits), &sorted, s));
     const size_t nseg = (size_t)GS_CLASSES * pl.nlev;
-    GCG_TRY(pl.off.alloc(nseg + 1));
-    GCG_CUDA(cudaMemsetAsync(pl.off.get(), 0, (nseg + 1) * 4, s));
+    GCG_TRY(seg.alloc(nseg + 1, s));
+    GCG_CUDA(cudaMemsetAsync(seg.get(), 0, (nseg + 1) * 4, s));
+    GCG_TRY(pl.off.alloc(pl.nlev));
     GCG_TRY(pl.order.alloc(nv));
-    k_level_bounds<<<vgrid(nv), 256, 0, s>>>(sorted, nv, g->vbits, (uint32_t)nseg, pl.off.get(),
-                                         pl.order.get());
+    k_level_bounds<<<vgrid(nv), 256, 0, s>>>(sorted, nv, g->vbits, (uint32_t)nseg, seg.get(), pl.order.get());
+    k_level_pack<<<vgrid(pl.nlev), 256, 0, s>>>(seg.get(), pl.nlev, pl.off.get());
     GCG_LAUNCH_CHECK();
     GCG_CUDA(cudaStreamSynchronize(s));
     return GCG_OK;
@@ -825,7 +929,7 @@ int pagerank_gs_exact(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
     const void *kern = edge    ? (const void *)k_gs_sweep<true, true>
                        : track ? (const void *)k_gs_sweep<false, true>
                                : (const void *)k_gs_sweep<false, false>;
-    const size_t smem = sizeof(GsGroup) * GS_GROUPS;
+    const size_t smem = sizeof(GsGroup) * GS_GROUPS + (size_t)(GS_THREADS / 32) * GS_WARP_MAX * sizeof(float);
     GCG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     unsigned grid = (unsigned)num_sms();
     int queued = 0;
