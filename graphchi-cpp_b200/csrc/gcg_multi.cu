@@ -16,9 +16,10 @@
  *   B  rows crossing chunks: partials added in chunk order;
  *   C  vertices: every warp takes an even, contiguous share of the active graphs'
  *      tiles of 128 rows (4 rows per thread), applies them, and writes one FP64 residual
- *      partial per graph it meets (fixed slot);
- *   D  one warp per graph adds its partials in a fixed order; a graph whose
- *      residual is <= tol (or that reached max_sweeps) leaves.
+ *      partial per tile (the tile's own slot);
+ *   D  one warp per graph, or one CTA per large graph, adds its tiles' partials in an
+ *      order that depends on the graph alone, not on its companions; a graph whose residual
+ *      is <= tol (or that reached max_sweeps) leaves.
  * The kernel ends when no graph is active. A whole solve (state init, initial
  * vector, the persistent kernel, rank assembly) is captured once into a CUDA
  * graph per parameter set and replayed; gcg_batch_autotune picks the hub-cache
@@ -45,6 +46,7 @@ namespace {
 
 constexpr uint32_t VROWS = 4;       /* rows per thread in a vertex tile */
 constexpr uint32_t VT = 32 * VROWS; /* rows per vertex tile, the work of one warp */
+constexpr uint32_t LARGE_TILES = 256; /* up to so many partials a warp adds: 8 loads a lane */
 constexpr uint32_t NG_MAX = 1024;     /* graphs per batch */
 static_assert(NG_MAX <= EDGE_THREADS, "active_prefix gives each graph one thread of the CTA");
 
@@ -54,8 +56,13 @@ struct GRange {
     uint32_t ss, se;      /* split-row list entries */
     uint32_t ns, ne;      /* rows with in-edges (nz index range) */
     uint32_t zs, ze;      /* rows without in-edges (zero index range) */
+    uint32_t it_nz, it_z; /* slots of its first tiles of rows with / without in-edges */
     uint32_t gend;        /* end of the graph's edges in the union (its chunks stop there) */
 };
+
+__host__ __device__ __forceinline__ uint32_t graph_tiles(const GRange &r) {
+    return (r.ne - r.ns + VT - 1) / VT + (r.ze - r.zs + VT - 1) / VT;
+}
 
 struct MultiArgs {
     SweepArgs a;            /* union graph arguments (buffers set per sweep inside) */
@@ -63,7 +70,9 @@ struct MultiArgs {
     float *rnz[2];
     const GRange *gr;
     uint32_t ng, max_sweeps;
-    double2 *tile_part;     /* residual partials: slot (warp + graph) */
+    double2 *tile_part;     /* residual partials, per tile */
+    const uint32_t *large;  /* graphs of more than LARGE_TILES tiles */
+    uint32_t nlarge;
     const double *norm_const; /* per graph */
     int *active;            /* per graph */
     int *gsweeps;           /* per graph: sweeps run */
@@ -188,6 +197,7 @@ __global__ void __launch_bounds__(EDGE_THREADS, 1) k_multi_pagerank(MultiArgs m)
     __shared__ uint32_t s_pref[NG_MAX + 1];
     __shared__ uint32_t s_cs[NG_MAX + 1];
     __shared__ uint32_t s_item, s_grab;
+    __shared__ double2 s_red[EDGE_THREADS / 32];
     const uint32_t FULL = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -336,24 +346,24 @@ __global__ void __launch_bounds__(EDGE_THREADS, 1) k_multi_pagerank(MultiArgs m)
 
         /* ---- C: vertex tiles of the active graphs. Warp w of nw takes tiles
          *         [w T / nw, (w + 1) T / nw): rows are equal work, so no queue and no
-         *         block barrier, and its residual sums stay in registers until it meets
-         *         another graph. Warps and graphs only go up together, so w + g names
-         *         the partial. Against 4096-row tiles from a device queue with a block
-         *         reduction each (34 us of a 205 us sweep of 5.4 M rows): 64 graphs to
-         *         1e-8 16.7 -> 16.4 ms, 5 graphs of 100 K rows in all 2.70 -> 2.49. ---- */
+         *         block barrier (against 4096-row tiles from a queue: 64 graphs to 1e-8
+         *         16.6 -> 16.3 ms). A partial per tile, which a graph's companions do not
+         *         change: one per warp and graph was added in an order that hung on where the
+         *         shares fell, by one warp (one graph of 4 M rows 17.6 ms, now 15.1). ---- */
         const uint32_t totC = active_prefix(m, 2, s_pref, const_pass);
         const uint32_t nw = min(nwarps, totC); /* each has a tile */
-        if (gwarp < nw) {
-            const uint32_t end = (uint32_t)((uint64_t)(gwarp + 1) * totC / nw);
-            uint32_t item = (uint32_t)((uint64_t)gwarp * totC / nw);
+        const uint32_t cwarp = warp * gridDim.x + blockIdx.x; /* few tiles: over all SMs */
+        if (cwarp < nw) {
+            const uint32_t end = (uint32_t)((uint64_t)(cwarp + 1) * totC / nw);
+            uint32_t item = (uint32_t)((uint64_t)cwarp * totC / nw);
             while (item < end) {
                 const uint32_t g = find_graph(s_pref, m.ng, item);
                 const GRange r = m.gr[g];
                 const uint32_t first = s_pref[g], gend = min(end, s_pref[g + 1]);
                 const uint32_t ntn = (r.ne - r.ns + VT - 1) / VT;
-                double d = 0.0, n = 0.0;
                 for (; item < gend; ++item) {
                     const uint32_t t = item - first;
+                    double d = 0.0, n = 0.0;
                     if (t < ntn) {
                         /* VROWS rows per thread (coalesced per row step), all loads first */
                         const uint32_t i0 = r.ns + t * VT + lane;
@@ -394,43 +404,64 @@ __global__ void __launch_bounds__(EDGE_THREADS, 1) k_multi_pagerank(MultiArgs m)
                             }
                         }
                     }
-                }
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    d += __shfl_down_sync(FULL, d, o);
-                    n += __shfl_down_sync(FULL, n, o);
+                    for (int o = 16; o > 0; o >>= 1) {
+                        d += __shfl_down_sync(FULL, d, o);
+                        n += __shfl_down_sync(FULL, n, o);
+                    }
+                    if (lane == 0) m.tile_part[t < ntn ? r.it_nz + t : r.it_z + (t - ntn)] = make_double2(d, n);
                 }
-                if (lane == 0) m.tile_part[gwarp + g] = make_double2(d, n);
             }
         }
         if (!grid_sync(m, gen)) return;
 
         /* ---- D: per-graph residual and stop ---- */
-        for (uint32_t g = gwarp; g < m.ng; g += nwarps) {
-            if (!*(volatile int *)(m.active + g)) continue;
-            double d = 0.0, n = 0.0;
-            if (s_pref[g] < s_pref[g + 1]) { /* the warps that hold its first and its last tile (phase C's prefix) */
-                const uint32_t w0 = (uint32_t)((((uint64_t)s_pref[g] + 1) * nw - 1) / totC);
-                const uint32_t w1 = (uint32_t)(((uint64_t)s_pref[g + 1] * nw - 1) / totC);
-#pragma unroll 4
-                for (uint32_t w = w0 + lane; w <= w1; w += 32u) {
-                    const double2 p = __ldcg(m.tile_part + w + g);
-                    d += p.x;
-                    n += p.y;
-                }
+        auto add_tiles = [&](const GRange &r, uint32_t first, uint32_t step, double &d, double &n) {
+            const uint32_t nt = (r.ne - r.ns + VT - 1) / VT, nz = const_pass ? (r.ze - r.zs + VT - 1) / VT : 0u;
+#pragma unroll 8
+            for (uint32_t t = first; t < nt + nz; t += step) {
+                const double2 p = __ldcg(m.tile_part + (t < nt ? r.it_nz + t : r.it_z + (t - nt)));
+                d += p.x;
+                n += p.y;
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 d += __shfl_xor_sync(FULL, d, o);
                 n += __shfl_xor_sync(FULL, n, o);
             }
-            if (lane == 0) {
-                if (!const_pass) n += m.norm_const[g];
-                const double res = n > 0.0 ? d / n : 0.0;
-                m.gres[g] = res;
-                m.gsweeps[g] = (int)sweep + 1;
-                if ((a.tol > 0.0 && res <= a.tol) || sweep + 1 >= m.max_sweeps) m.active[g] = 0;
+        };
+        auto finish = [&](uint32_t g, double d, double n) {
+            if (!const_pass) n += m.norm_const[g];
+            const double res = n > 0.0 ? d / n : 0.0;
+            m.gres[g] = res;
+            m.gsweeps[g] = (int)sweep + 1;
+            if ((a.tol > 0.0 && res <= a.tol) || sweep + 1 >= m.max_sweeps) m.active[g] = 0;
+        };
+        for (uint32_t k = blockIdx.x; k < m.nlarge; k += gridDim.x) {
+            const uint32_t g = m.large[k];
+            if (!*(volatile int *)(m.active + g)) continue; /* the same for the CTA: cleared past the barrier below */
+            double d = 0.0, n = 0.0;
+            add_tiles(m.gr[g], threadIdx.x, EDGE_THREADS, d, n);
+            if (lane == 0) s_red[warp] = make_double2(d, n);
+            __syncthreads();
+            if (warp == 0) {
+                d = s_red[lane].x;
+                n = s_red[lane].y;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    d += __shfl_xor_sync(FULL, d, o);
+                    n += __shfl_xor_sync(FULL, n, o);
+                }
+                if (lane == 0) finish(g, d, n);
             }
+            __syncthreads();
+        }
+        for (uint32_t g = gwarp; g < m.ng; g += nwarps) {
+            const GRange r = m.gr[g];
+            if (graph_tiles(r) > LARGE_TILES || !*(volatile int *)(m.active + g)) continue;
+            double d = 0.0, n = 0.0;
+            add_tiles(r, lane, 32u, d, n);
+            if (lane == 0) finish(g, d, n);
         }
         /* the queues of the next sweep's parity were last used a sweep ago */
         if (blockIdx.x == 0 && threadIdx.x == 0) m.qctr[(sweep + 1) & 1] = 0u;
@@ -554,6 +585,8 @@ struct gcg_batch {
     std::vector<uint32_t> voff, eoff;   /* union vertex / edge offset of each graph (edges 256-aligned) */
     std::vector<uint32_t> roff;         /* offset of each graph in the callers' arrays (no padding) */
     std::vector<gcg::GRange> gr_host;
+    uint32_t ntiles = 0, nlarge = 0;
+    gcg::dbuf<uint32_t> large; /* graphs whose partials a CTA adds */
     gcg::dbuf<uint32_t> d_roff, d_voff;
     gcg::dbuf<uint32_t> long_g; /* graph of each long split row of the union (or ng: none) */
     gcg::dbuf<gcg::GRange> gr;
@@ -669,6 +702,7 @@ static int batch_build(gcg_graph *const *graphs, uint32_t ng, uint32_t flags, gc
     GCG_CUDA(cudaMemcpy(hz.data(), zb.get(), nq * 4, cudaMemcpyDeviceToHost));
     GCG_CUDA(cudaMemcpy(hs.data(), sb.get(), nq * 4, cudaMemcpyDeviceToHost));
     b->gr_host.resize(ng);
+    std::vector<uint32_t> large;
     for (uint32_t g = 0; g < ng; ++g) {
         GRange &r = b->gr_host[g];
         r.cs = b->eoff[g] / CH;
@@ -680,7 +714,14 @@ static int batch_build(gcg_graph *const *graphs, uint32_t ng, uint32_t flags, gc
         r.ze = hz[2 * g + 1];
         r.ss = hs[2 * g];
         r.se = hs[2 * g + 1];
+        r.it_nz = b->ntiles;
+        r.it_z = r.it_nz + (r.ne - r.ns + VT - 1) / VT;
+        b->ntiles += graph_tiles(r);
+        if (graph_tiles(r) > LARGE_TILES) large.push_back(g);
     }
+    b->nlarge = (uint32_t)large.size();
+    GCG_TRY(b->large.alloc(std::max<size_t>(large.size(), 1)));
+    GCG_CUDA(cudaMemcpy(b->large.get(), large.data(), large.size() * 4, cudaMemcpyHostToDevice));
     /* the graph of each long split row (the padding rows never span that far) */
     {
         std::vector<uint32_t> ls(pl.nlong), lg(std::max<uint32_t>(pl.nlong, 1), ng);
@@ -767,7 +808,7 @@ static int batch_pagerank(gcg_batch *b, const gcg_pr_params *p, float *out, int3
         GCG_TRY(b->r.alloc(nv));
         GCG_TRY(b->nzsum.alloc(std::max<uint32_t>(pl.nnz, 1)));
         GCG_TRY(b->parts.alloc((size_t)2 * pl.nchunks + 2));
-        GCG_TRY(b->tile_part.alloc((size_t)num_sms() * (EDGE_THREADS / 32) + ng));
+        GCG_TRY(b->tile_part.alloc(std::max<uint32_t>(b->ntiles, 1)));
         GCG_TRY(b->norm_const.alloc(ng));
         GCG_TRY(b->gres.alloc(ng));
         GCG_TRY(b->active.alloc(ng));
@@ -812,6 +853,8 @@ static int batch_pagerank(gcg_batch *b, const gcg_pr_params *p, float *out, int3
     m.ng = ng;
     m.max_sweeps = (uint32_t)p->max_sweeps;
     m.tile_part = b->tile_part.get();
+    m.large = b->large.get();
+    m.nlarge = b->nlarge;
     m.norm_const = b->norm_const.get();
     m.active = b->active.get();
     m.gsweeps = b->gsweeps.get();
