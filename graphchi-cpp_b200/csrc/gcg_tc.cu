@@ -15,7 +15,8 @@
  *      and streams the rest of N+(a) behind b past them for each of b's edges. A match
  *      c is a triangle (a,b,c): c's count is bumped per match, a's and b's by the match
  *      totals (counts of the top-ranked vertices gathered in shared memory first) — the
- *      per-rank incident-triangle counts of <base>_degord.4B.vout.
+ *      per-rank incident-triangle counts of <base>_degord.4B.vout. Where lists are short
+ *      (TC_SHORT) the edges are not grouped; the shorter list is searched in the longer.
  */
 #include <algorithm>
 
@@ -31,17 +32,42 @@ inline unsigned vgrid(uint64_t n) {
     return (unsigned)std::max<uint64_t>(1, std::min(b, cap));
 }
 
-__global__ void k_degree_keys(const uint32_t *__restrict__ indeg, const uint32_t *__restrict__ outdeg, uint32_t nv,
-                              uint32_t vbits, uint64_t *__restrict__ keys, uint32_t *maxdeg) {
+/* of the in + out degrees */
+struct DegreeStat {
+    double squares; /* their sum */
+    uint32_t most;
+};
+
+__global__ void __launch_bounds__(256) k_degree_keys(const uint32_t *__restrict__ indeg, const uint32_t *__restrict__ outdeg, uint32_t nv,
+                              uint32_t vbits, uint64_t *__restrict__ keys, DegreeStat *stat) {
+    __shared__ uint32_t s_m[8];
+    __shared__ double s_s[8];
     uint32_t m = 0;
+    double sq = 0.0;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
         uint64_t d = (uint64_t)indeg[v] + outdeg[v];
         keys[v] = (d << vbits) | v;
         m = max(m, d > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)d);
+        sq += (double)d * (double)d;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_down_sync(0xFFFFFFFFu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(maxdeg, m);
+    for (int o = 16; o > 0; o >>= 1) {
+        m = max(m, __shfl_down_sync(0xFFFFFFFFu, m, o));
+        sq += __shfl_down_sync(0xFFFFFFFFu, sq, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        s_m[threadIdx.x >> 5] = m;
+        s_s[threadIdx.x >> 5] = sq;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) {
+            m = max(m, s_m[w]);
+            sq += s_s[w];
+        }
+        atomicMax(&stat->most, m);
+        atomicAdd(&stat->squares, sq);
+    }
 }
 
 __global__ void k_rank_scatter(const uint64_t *__restrict__ sorted, uint32_t nv, uint32_t vbits,
@@ -154,6 +180,20 @@ constexpr uint32_t TC_FILTER = 4096;   /* bits */
 constexpr int TC_WINDOWS = 4;          /* loads of 32 candidates in flight per warp */
 constexpr uint32_t TC_TASK_MIN = 32, TC_TASK_MAX = 256; /* edges of one b that a warp takes at a time */
 constexpr uint32_t TC_WARP_WORDS = (TC_TOP + TC_FILTER) / 32 + 64; /* bits, filter, 32 lists' places and hits */
+/* Where the degrees are alike (an edge's end has less than TC_FLAT times the mean degree) the
+ * top ranks hold few of the candidates, and N+(b)'s elements below them may be many: from
+ * TC_PAIRS on, where the filter lets many candidates through, they are searched two at a
+ * time (uniform, 200 K vertices of degree 2,000: 1,078 -> 932 ms, of 500: 50.4 -> 48.1). In a
+ * kernel of its own: the same code costs R-MAT scale 20 1.6 %. */
+constexpr double TC_FLAT = 4.0;
+constexpr uint32_t TC_PAIRS = 32;
+/* Below this many neighbours of an edge's end, on average over the edges, grouping the edges
+ * costs more than it saves, and the shorter list is searched in the longer, edge by edge
+ * (k_tc_search). Uniform graphs, grouped and searched: 4 M vertices of degree 16 6.43 and
+ * 4.69 ms, 48 20.0 and 16.7; 128 K of 64 1.06 and 1.05; 200 K of 100 2.49 and 2.79; 16 K of
+ * 64 0.376 and 0.353; 1 M in communities of 50 2.11 and 1.62. R-MAT graphs of more than a few
+ * edges a vertex are above it (scale 14 with 4: 143, scale 20 with 1: 217). */
+constexpr double TC_SHORT = 96.0;
 constexpr size_t TC_SMEM = ((size_t)TC_TOP + TC_WARPS * TC_WARP_WORDS) * 4;
 
 /* Edges with candidates (b is not the last of N+(a)) grouped by b, in two passes over
@@ -249,9 +289,31 @@ __device__ __noinline__ bool low_candidate(uint32_t c, const uint32_t *__restric
     return true;
 }
 
+/* The same of two candidates at once (want: bits 0, 1), returned as bits: what a search waits
+ * for is one dependent load after another. */
+__device__ __noinline__ uint32_t low_candidates(uint32_t c0, uint32_t c1, uint32_t want,
+                                                const uint32_t *__restrict__ list, uint32_t nlow,
+                                                uint32_t *__restrict__ cnt) {
+    uint32_t at0 = 0, at1 = 0, len = nlow; /* the last element <= c */
+    while (len > 1) {
+        const uint32_t half = len >> 1;
+        const uint32_t x0 = __ldg(list + at0 + half), x1 = __ldg(list + at1 + half);
+        if (x0 <= c0) at0 += half;
+        if (x1 <= c1) at1 += half;
+        len -= half;
+    }
+    const uint32_t x0 = __ldg(list + at0), x1 = __ldg(list + at1);
+    if (x0 != c0) want &= 2u;
+    if (x1 != c1) want &= 1u;
+    if (want & 1u) atomicAdd(cnt + c0, 1u);
+    if (want & 2u) atomicAdd(cnt + c1, 1u);
+    return want;
+}
+
 /* A warp takes tasks from a device counter, those of the highest b first. Counts of the
  * top ranks are gathered in the block's shared memory and added to `cnt` at the end:
  * one global atomic per triangle on those few addresses queues at the L2. */
+template <bool FLAT>
 __global__ void __launch_bounds__(1024, 1) k_tc_count(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ cl,
                                                       uint32_t nv, uint32_t top, const uint2 *__restrict__ rev,
                                                       const uint32_t *__restrict__ rev_end,
@@ -330,6 +392,24 @@ __global__ void __launch_bounds__(1024, 1) k_tc_count(const uint32_t *__restrict
                 }
                 return m;
             };
+            /* the same of two candidates per lane, for many such elements: there the filter lets
+             * many through */
+            auto probe2 = [&](uint32_t c0, uint32_t c1, uint32_t &m0, uint32_t &m1) {
+                const uint32_t r0 = last_rank - c0, r1 = last_rank - c1;
+                bool hit0 = false, hit1 = false;
+                if (r0 < top) hit0 = (bits[r0 >> 5] >> (r0 & 31u)) & 1u;
+                if (r1 < top) hit1 = (bits[r1 >> 5] >> (r1 & 31u)) & 1u;
+                if (hit0) atomicAdd(s_top + r0, 1u);
+                if (hit1) atomicAdd(s_top + r1, 1u);
+                const uint32_t h0 = tc_hash(c0), h1 = tc_hash(c1);
+                uint32_t want = r0 - top < nv - top ? (filter[h0 >> 5] >> (h0 & 31u)) & 1u : 0u;
+                if (r1 - top < nv - top) want |= ((filter[h1 >> 5] >> (h1 & 31u)) & 1u) << 1;
+                if (want) want = low_candidates(c0, c1, want, cl + B, nlow, cnt);
+                __syncwarp();
+                m0 = __ballot_sync(FULL, hit0 || (want & 1u));
+                m1 = __ballot_sync(FULL, hit1 || (want & 2u));
+            };
+            const bool pairs = FLAT && nlow >= TC_PAIRS;
             uint32_t bsum = 0;
             for (uint32_t e0 = first; e0 < e1; e0 += 32u) {
                 const uint32_t ne = min(32u, e1 - e0);
@@ -347,6 +427,12 @@ __global__ void __launch_bounds__(1024, 1) k_tc_count(const uint32_t *__restrict
                     const uint32_t *at = cl + __shfl_sync(FULL, base, l) + lane;
                     const uint32_t n32 = __shfl_sync(FULL, nf, l);
                     uint32_t m = 0, o = 0;
+                    if (pairs)
+                        for (; o + 1u < n32; o += 2u) {
+                            uint32_t m0, m1;
+                            probe2(__ldg(at + 32u * o), __ldg(at + 32u * o + 32u), m0, m1);
+                            m += __popc(m0) + __popc(m1);
+                        }
                     for (; o + 1u < n32; o += 2u) {
                         const uint32_t x = __ldg(at + 32u * o), y = __ldg(at + 32u * o + 32u);
                         m += __popc(probe(x));
@@ -382,6 +468,17 @@ __global__ void __launch_bounds__(1024, 1) k_tc_count(const uint32_t *__restrict
                         begun += __popc(starts);
                         x[u] = w0 + lane < W ? __ldg(cl + (list_off[q[u]] + w0 + lane)) : NO_ONE;
                     }
+                    if (pairs) {
+#pragma unroll
+                        for (int u = 0; u < TC_WINDOWS; u += 2) {
+                            if (w1 + 32u * u >= W) break;
+                            uint32_t m0, m1;
+                            probe2(x[u], x[u + 1], m0, m1);
+                            if ((m0 >> lane) & 1u) atomicAdd(list_hit + q[u], 1u);
+                            if ((m1 >> lane) & 1u) atomicAdd(list_hit + q[u + 1], 1u);
+                        }
+                        continue;
+                    }
 #pragma unroll
                     for (int u = 0; u < TC_WINDOWS; ++u)
                         if (w1 + 32u * u < W && ((probe(x[u]) >> lane) & 1u)) atomicAdd(list_hit + q[u], 1u);
@@ -412,6 +509,223 @@ __global__ void __launch_bounds__(1024, 1) k_tc_count(const uint32_t *__restrict
         if (s_top[i]) atomicAdd(cnt + (last_rank - i), s_top[i]);
 }
 
+/* ---- counting where lists are short (TC_SHORT) --------------------------------- */
+
+/* One halving of the search for the last element <= x in the sorted,
+ * duplicate-free cl[base .. base + n), n >= 2: the range that still holds that
+ * element shrinks to ceil(n / 2) values. After ceil(log2 n) halvings n is 1 and
+ * x is present exactly when cl[base] equals it. */
+__device__ __forceinline__ uint32_t last_le_step(const uint32_t *__restrict__ cl, uint32_t base, uint32_t &n,
+                                                 uint32_t x) {
+    const uint32_t h = n >> 1;
+    if (__ldg(cl + base + h) <= x) base += h;
+    n -= h;
+    return base;
+}
+
+constexpr uint32_t TC_SPLIT = 64;   /* top-range vertices with more higher-ranked neighbours go batch by batch */
+
+/* Longest higher-ranked neighbour list among rows lo .. nv - 1 (atomicMax into *out). */
+__global__ void k_max_rowlen(const uint32_t *__restrict__ rp, uint32_t lo, uint32_t nv, uint32_t *out) {
+    uint32_t m = 0;
+    for (uint32_t r = lo + blockIdx.x * blockDim.x + threadIdx.x; r < nv; r += gridDim.x * blockDim.x)
+        m = max(m, rp[r + 1] - rp[r]);
+    m = __reduce_max_sync(0xFFFFFFFFu, m);
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
+}
+
+/* Triangles through vertex a, 32 of its higher-ranked neighbours b at a time (a
+ * batch). For each b the shorter of (N+(a) after b) and N+(b) is searched element
+ * by element in the longer; the searches of the batch's b's are laid end to end
+ * (a warp prefix sum of their lengths) and dealt to the lanes two at a time, so
+ * every lane runs two independent searches whatever the lengths. A match c is the
+ * triangle (a, b, c): c's count is bumped per match, b's by its match total, a's
+ * by the batch's sum. A b whose two lists are both long is not searched: the
+ * whole warp merges the two lists instead, after the searches.
+ * Work is spread two ways. Vertex a goes to warp (a mod warps), numbered block
+ * fastest, so the heavy vertices, which sit together in the upper ranks, land on
+ * every SM. Vertices among the top `nsplit` ranks with more than TC_SPLIT
+ * higher-ranked neighbours are not taken whole: their batches are dealt out one
+ * by one after the other vertices, so no warp is left with a whole heavy vertex.
+ * Ranks grow with degree, so the highest-ranked vertex of a triangle is nearly
+ * always among the top few thousand ranks: their counts are kept in the block's
+ * shared memory (dynamic, `top` entries for ranks nv - top .. nv - 1) and added
+ * to `cnt` once at the end, which keeps the per-triangle increments off a few
+ * hot global addresses. */
+__global__ void __launch_bounds__(1024, 2) k_tc_search(const uint32_t *__restrict__ rp, const uint32_t *__restrict__ cl,
+                                                       uint32_t nv, uint32_t top, uint32_t nsplit,
+                                                      const uint32_t *__restrict__ split_maxlen,
+                                                      uint32_t *__restrict__ cnt, unsigned long long *total) {
+    extern __shared__ uint32_t s_top[];
+    __shared__ uint32_t s_pre[TC_WARPS][32], s_so[TC_WARPS][32], s_lo[TC_WARPS][32], s_nl[TC_WARPS][32],
+        s_hit[TC_WARPS][32];
+    const uint32_t FULL = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t *pre = s_pre[w], *so_ = s_so[w], *lo_ = s_lo[w], *nl_ = s_nl[w], *hit = s_hit[w];
+    const uint32_t warp = w * gridDim.x + blockIdx.x;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t lo_top = nv - top, lo_split = nv - nsplit;
+    for (uint32_t i = threadIdx.x; i < top; i += blockDim.x) s_top[i] = 0;
+    __syncthreads();
+    auto bump = [&](uint32_t v, uint32_t inc) {
+        if (v >= lo_top)
+            atomicAdd(s_top + (v - lo_top), inc);
+        else
+            atomicAdd(cnt + v, inc);
+    };
+    /* the batch of a's neighbours j0 .. j0 + 31 (ab <= j0, j0 + 1 < ae); returns
+     * this lane's b's match total (0 for lanes past the list) */
+    auto batch = [&](uint32_t ab, uint32_t ae, uint32_t j0) -> uint32_t {
+        const uint32_t j = j0 + lane;
+        uint32_t ns = 0, so = 0, lo = 0, nl = 0, b = 0;
+        bool mrg = false;
+        if (j + 1 < ae) {
+            b = __ldg(cl + j);
+            const uint32_t na = ae - j - 1, bb = __ldg(rp + b), nb = __ldg(rp + b + 1) - bb;
+            if (nb) {
+                if (na <= nb) {
+                    ns = na, so = j + 1, lo = bb, nl = nb;
+                } else {
+                    ns = nb, so = bb, lo = j + 1, nl = na;
+                }
+                /* both lists long: a merge of the two (a warp walking na + nb
+                 * values, one partition search per lane) when the ns searches of
+                 * log2(nl) steps would take more than three steps per merged value
+                 * (a merge step is a dependent load; 1.5, 2, 3, 4 and 6 were
+                 * measured) */
+                const uint32_t tot = na + nb;
+                if (ns * (32 - __clz((nl - 1) | 1)) > 3 * tot + 32 * (32 - __clz((tot - 1) | 1))) {
+                    mrg = true, ns = 0;
+                }
+            }
+        }
+        uint32_t inc = ns;
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(FULL, inc, o);
+            if (lane >= o) inc += t;
+        }
+        const uint32_t W = __shfl_sync(FULL, inc, 31);
+        const uint32_t merges = __ballot_sync(FULL, mrg);
+        if (W == 0 && merges == 0) return 0u;
+        pre[lane] = inc, so_[lane] = so, lo_[lane] = lo, nl_[lane] = nl, hit[lane] = 0;
+        __syncwarp();
+        for (uint32_t t0 = 0; t0 < W; t0 += 64) {
+            uint32_t x[2], base[2], n[2], q[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const uint32_t t = t0 + 32 * u + lane;
+                n[u] = 0, x[u] = 0, base[u] = 0, q[u] = 0;
+                if (t < W) {
+                    /* owner: how many of the 32 inclusive prefix sums are <= t
+                     * (t < W = pre[31], so at most 31; indexes stay below 31) */
+                    uint32_t qq = 0;
+#pragma unroll
+                    for (uint32_t st = 16; st; st >>= 1)
+                        if (pre[qq + st - 1] <= t) qq += st;
+                    const uint32_t k = t - (qq ? pre[qq - 1] : 0);
+                    x[u] = __ldg(cl + so_[qq] + k);
+                    base[u] = lo_[qq], n[u] = nl_[qq], q[u] = qq;
+                }
+            }
+            while (n[0] > 1 || n[1] > 1) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+                    if (n[u] > 1) base[u] = last_le_step(cl, base[u], n[u], x[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (n[u] == 1 && __ldg(cl + base[u]) == x[u]) {
+                    bump(x[u], 1u);
+                    atomicAdd(hit + q[u], 1u);
+                }
+        }
+        __syncwarp();
+        /* the merged pairs, one at a time by the whole warp: A = N+(a) after b,
+         * B = N+(b); lane l walks diagonals [l per, (l + 1) per) of the merge that
+         * takes A[i] when A[i] <= B[j], so B[j] is the least B value not below
+         * A[i] and A[i] is in B exactly when they are equal */
+        for (uint32_t m = merges; m; m &= m - 1) {
+            const int l = __ffs(m) - 1;
+            const uint32_t jl = j0 + (uint32_t)l, A = jl + 1, na = ae - jl - 1;
+            const uint32_t bl = __shfl_sync(FULL, b, l), B = __ldg(rp + bl), nb = __ldg(rp + bl + 1) - B;
+            const uint32_t tot = na + nb, per = (tot + 31) / 32;
+            const uint32_t d0 = min(lane * per, tot), d1 = min(d0 + per, tot);
+            uint32_t i = d0 > nb ? d0 - nb : 0, hi = min(d0, na);
+            while (i < hi) { /* first i with A[i] > B[d0 - 1 - i] */
+                const uint32_t mid = (i + hi) >> 1;
+                if (__ldg(cl + A + mid) <= __ldg(cl + B + d0 - 1 - mid))
+                    i = mid + 1;
+                else
+                    hi = mid;
+            }
+            uint32_t k = d0 - i, found = 0;
+            uint32_t av = i < na ? __ldg(cl + A + i) : 0u, bv = k < nb ? __ldg(cl + B + k) : 0u;
+            for (uint32_t d = d0; d < d1; ++d) {
+                if (i < na && (k >= nb || av <= bv)) {
+                    if (k < nb && av == bv) {
+                        bump(av, 1u);
+                        ++found;
+                    }
+                    ++i;
+                    if (i < na) av = __ldg(cl + A + i);
+                } else {
+                    ++k;
+                    if (k < nb) bv = __ldg(cl + B + k);
+                }
+            }
+            found = __reduce_add_sync(FULL, found);
+            if (lane == 0 && found) hit[l] += found;
+            __syncwarp();
+        }
+        const uint32_t h = hit[lane];
+        if (h) bump(b, h);
+        __syncwarp(); /* the tables are rewritten by the next batch */
+        return h;
+    };
+    unsigned long long mine = 0;
+    auto finish = [&](uint32_t a, uint32_t acc) {
+        const uint32_t A = __reduce_add_sync(FULL, acc);
+        if (A && lane == 0) {
+            bump(a, A);
+            mine += A;
+        }
+    };
+    for (uint32_t a = warp; a < nv; a += nwarps) {
+        const uint32_t ab = __ldg(rp + a), ae = __ldg(rp + a + 1);
+        if (ae - ab < 2) continue; /* a triangle needs two higher-ranked neighbours */
+        if (a >= lo_split && ae - ab > TC_SPLIT) continue; /* dealt out batch by batch below */
+        uint32_t acc = 0;
+        for (uint32_t j0 = ab; j0 + 1 < ae; j0 += 32) acc += batch(ab, ae, j0);
+        finish(a, acc);
+    }
+    /* the split vertices' batches: item t is batch t / nsplit of vertex
+     * lo_split + t % nsplit, and goes to warp t mod warps (neighbouring vertices'
+     * batches to different warps); each lane checks one of its warp's items, the
+     * warp runs the real ones */
+    const uint64_t items = (uint64_t)nsplit * ((*split_maxlen + 31) / 32);
+    for (uint64_t k0 = 0; warp + (uint64_t)nwarps * k0 < items; k0 += 32) {
+        const uint64_t t = warp + (uint64_t)nwarps * (k0 + lane);
+        uint32_t a = 0, ab = 0, ae = 0, j0 = 0;
+        bool real = false;
+        if (t < items) {
+            a = lo_split + (uint32_t)(t % nsplit);
+            ab = __ldg(rp + a), ae = __ldg(rp + a + 1);
+            j0 = ab + 32u * (uint32_t)(t / nsplit);
+            real = ae - ab > TC_SPLIT && j0 + 1 < ae;
+        }
+        for (uint32_t m = __ballot_sync(FULL, real); m; m &= m - 1) {
+            const int l = __ffs(m) - 1;
+            const uint32_t va = __shfl_sync(FULL, a, l), vab = __shfl_sync(FULL, ab, l),
+                           vae = __shfl_sync(FULL, ae, l), vj0 = __shfl_sync(FULL, j0, l);
+            finish(va, batch(vab, vae, vj0));
+        }
+    }
+    if (lane == 0 && mine) atomicAdd(total, mine);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < top; i += blockDim.x)
+        if (s_top[i]) atomicAdd(cnt + lo_top + i, s_top[i]);
+}
+
 }  // namespace
 }  // namespace gcg
 
@@ -433,18 +747,23 @@ extern "C" int gcg_triangle_count(gcg_graph *g, uint64_t *total, uint32_t *per_r
 
     /* 1. degree ranking */
     tbuf<uint64_t> keys, tmp;
-    tbuf<uint32_t> rank, dmax;
+    tbuf<uint32_t> rank;
+    tbuf<DegreeStat> dstat;
     GCG_TRY(keys.alloc(std::max<uint64_t>(nv, ne), s));
     GCG_TRY(tmp.alloc(std::max<uint64_t>(nv, ne), s));
     GCG_TRY(rank.alloc(nv, s));
-    GCG_TRY(dmax.alloc(1, s));
-    GCG_CUDA(cudaMemsetAsync(dmax.get(), 0, 4, s));
-    k_degree_keys<<<vgrid(nv), 256, 0, s>>>(g->indeg.get(), g->outdeg.get(), nv, vbits, keys.get(), dmax.get());
-    uint32_t maxdeg = 0;
-    GCG_CUDA(cudaMemcpyAsync(&maxdeg, dmax.get(), 4, cudaMemcpyDeviceToHost, s));
+    GCG_TRY(dstat.alloc(1, s));
+    GCG_CUDA(cudaMemsetAsync(dstat.get(), 0, sizeof(DegreeStat), s));
+    k_degree_keys<<<vgrid(nv), 256, 0, s>>>(g->indeg.get(), g->outdeg.get(), nv, vbits, keys.get(), dstat.get());
+    DegreeStat deg = {};
+    GCG_CUDA(cudaMemcpyAsync(&deg, dstat.get(), sizeof(deg), cudaMemcpyDeviceToHost, s));
     GCG_CUDA(cudaStreamSynchronize(s));
     uint32_t dbits = 1;
-    while (dbits < 33 && (1ull << dbits) <= maxdeg) ++dbits;
+    while (dbits < 33 && (1ull << dbits) <= deg.most) ++dbits;
+    /* neighbours of an edge's end, on average over the edges (a symmetric graph counts each twice) */
+    const double twice = g->symmetric ? 2.0 : 1.0;
+    const double edge_degree = ne ? deg.squares / (2.0 * (double)ne) / twice : 0.0;
+    const double mean_degree = 2.0 * (double)ne / (double)nv / twice;
     if (vbits + dbits > 64) return fail(GCG_ERR_UNSUPPORTED, "gcg_triangle_count: degree and id do not fit 64 bits");
     uint64_t *sorted = nullptr;
     GCG_TRY(radix_sort_u64(keys.get(), tmp.get(), nv, 0, (int)(vbits + dbits), &sorted, s));
@@ -513,7 +832,21 @@ extern "C" int gcg_triangle_count(gcg_graph *g, uint64_t *total, uint32_t *per_r
     GCG_TRY(d_total.alloc(1, s));
     GCG_CUDA(cudaMemsetAsync(cnt_ptr, 0, (size_t)nv * 4, s));
     GCG_CUDA(cudaMemsetAsync(d_total.get(), 0, 8, s));
-    if (m_or > 0) {
+    const uint32_t top = std::min(nv, TC_TOP);
+    const unsigned sms = (unsigned)num_sms();
+    if (m_or > 0 && edge_degree < TC_SHORT) {
+        const uint32_t nsplit = std::min(nv, std::max<uint32_t>(65536u, nv / 16));
+        tbuf<uint32_t> split_maxlen;
+        GCG_TRY(split_maxlen.alloc(1, s));
+        GCG_CUDA(cudaMemsetAsync(split_maxlen.get(), 0, 4, s));
+        k_max_rowlen<<<vgrid(nsplit), 256, 0, s>>>(rp.get(), nv - nsplit, nv, split_maxlen.get());
+        GCG_CUDA(cudaFuncSetAttribute(k_tc_search, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TC_TOP * 4)));
+        /* two blocks per SM, each with its own top-rank counters */
+        const unsigned cb = (unsigned)std::min<uint64_t>(((uint64_t)nv + TC_WARPS - 1) / TC_WARPS, 2ull * sms);
+        k_tc_search<<<cb, TC_WARPS * 32, (size_t)top * 4, s>>>(rp.get(), cl.get(), nv, top, nsplit,
+                                                               split_maxlen.get(), cnt_ptr, d_total.get());
+        GCG_LAUNCH_CHECK();
+    } else if (m_or > 0) {
         /* the edges grouped by b, cut into tasks */
         tbuf<uint32_t> in_cnt, ntask, ctl, part;
         tbuf<uint2> task;
@@ -529,8 +862,6 @@ extern "C" int gcg_triangle_count(gcg_graph *g, uint64_t *total, uint32_t *per_r
         GCG_TRY(task.alloc(most, s));
         GCG_CUDA(cudaMemsetAsync(in_cnt.get(), 0, (size_t)nv * 4, s));
         GCG_CUDA(cudaMemsetAsync(ctl.get(), 0, 8, s));
-        const uint32_t top = std::min(nv, TC_TOP);
-        const unsigned sms = (unsigned)num_sms();
         GCG_TRY(part.alloc((size_t)sms * top, s));
         GCG_CUDA(cudaFuncSetAttribute(k_tc_group<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TC_TOP * 4)));
         GCG_CUDA(cudaFuncSetAttribute(k_tc_group<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TC_TOP * 4)));
@@ -541,8 +872,9 @@ extern "C" int gcg_triangle_count(gcg_graph *g, uint64_t *total, uint32_t *per_r
         GCG_TRY(scan_u32(in_cnt.get(), in_cnt.get(), nv, nullptr, s));
         k_tc_group<true><<<sms, 1024, top * 4, s>>>(okeys, m_or, vbits, rp.get(), nv, top, in_cnt.get(), part.get(), rev);
         k_tc_tasks<<<vgrid(nv), 256, 0, s>>>(in_cnt.get(), ntask.get(), rp.get(), nv, size, task.get());
-        GCG_CUDA(cudaFuncSetAttribute(k_tc_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
-        k_tc_count<<<sms, TC_WARPS * 32, TC_SMEM, s>>>(rp.get(), cl.get(), nv, top, rev, in_cnt.get(),
+        auto kern = edge_degree < TC_FLAT * mean_degree ? k_tc_count<true> : k_tc_count<false>;
+        GCG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
+        kern<<<sms, TC_WARPS * 32, TC_SMEM, s>>>(rp.get(), cl.get(), nv, top, rev, in_cnt.get(),
                                                              task.get(), ctl.get(), size, full, ctl.get() + 1,
                                                              cnt_ptr, d_total.get());
         GCG_LAUNCH_CHECK();
