@@ -304,6 +304,26 @@ int pagerank_delta(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg_pr
 int cc_label_propagation(gcg_graph *g, int scheduler, int max_iters, uint32_t *labels, gcg_cc_stats *stats,
                          int32_t *frontier_log);
 
+/* polls of a wait that GCG_PR_TEST_BARRIER_TIMEOUT lets run out */
+constexpr long long GCG_TEST_SPIN = 1ll << 14;
+
+/* the two events around what a call times, destroyed on every way out of it */
+struct EventPair {
+    cudaEvent_t first = nullptr, last = nullptr;
+    EventPair() = default;
+    EventPair(const EventPair &) = delete;
+    EventPair &operator=(const EventPair &) = delete;
+    ~EventPair() {
+        if (first) cudaEventDestroy(first);
+        if (last) cudaEventDestroy(last);
+    }
+    int create() {
+        GCG_CUDA(cudaEventCreate(&first));
+        GCG_CUDA(cudaEventCreate(&last));
+        return GCG_OK;
+    }
+};
+
 constexpr int MP_THREADS = 256;
 constexpr int MP_ITEMS = 8;
 constexpr int MP_TILE = MP_THREADS * MP_ITEMS;

@@ -432,6 +432,7 @@ struct GsArgs {
     uint32_t *bar; /* arrivals at the grid barrier, counted up over the call */
     uint32_t meets; /* arrivals before this sweep */
     int *err;
+    long long spin_limit;
     double reset, damping;
 };
 
@@ -454,7 +455,7 @@ __device__ __forceinline__ bool gs_wait(const GsArgs &a, uint32_t target) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bar) : "memory");
             if ((int32_t)(seen - target) >= 0) break;
             if ((spins & 255) == 255 && *(volatile int *)a.err) ok = 0;
-            if (spins > GS_SPIN) {
+            if (spins > a.spin_limit) {
                 atomicExch(a.err, 1);
                 ok = 0;
             }
@@ -909,9 +910,8 @@ int pagerank_gs_exact(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
     else k_gs_init<<<vgrid(nv), 256, 0, s>>>(nv, g->outdeg.get(), reset, buf[0]);
     GCG_LAUNCH_CHECK();
 
-    cudaEvent_t ev0, ev1;
-    GCG_CUDA(cudaEventCreate(&ev0));
-    GCG_CUDA(cudaEventCreate(&ev1));
+    EventPair ev;
+    GCG_TRY(ev.create());
     GsArgs a{};
     a.order = pl.order.get();
     a.off = pl.off.get();
@@ -924,6 +924,11 @@ int pagerank_gs_exact(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
     a.done = done;
     a.err = (int *)(ctl.get() + 3);
     a.bar = ctl.get() + 4;
+    a.spin_limit = GS_SPIN;
+    if (p->flags & GCG_PR_TEST_BARRIER_TIMEOUT) { /* one arrival short */
+        a.spin_limit = GCG_TEST_SPIN;
+        GCG_CUDA(cudaMemsetAsync(a.bar, 0xFF, 4, s));
+    }
     a.reset = p->teleport;
     a.damping = p->damping;
     const void *kern = edge    ? (const void *)k_gs_sweep<true, true>
@@ -957,7 +962,7 @@ int pagerank_gs_exact(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
     /* sweeps are queued in chunks of 8; with a tolerance the host checks the
      * sweep count after each chunk (sweeps queued past convergence return at once) */
     uint32_t h_ctl[4] = {0, 0, 0, 0};
-    GCG_CUDA(cudaEventRecord(ev0, s));
+    GCG_CUDA(cudaEventRecord(ev.first, s));
     for (int sw = 0; sw < nsw;) {
         const int n = std::min(8, nsw - sw);
         for (int k = 0; k < n; ++k) GCG_TRY(launch_sweep());
@@ -968,7 +973,7 @@ int pagerank_gs_exact(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
             if (h_ctl[2]) break;
         }
     }
-    GCG_CUDA(cudaEventRecord(ev1, s));
+    GCG_CUDA(cudaEventRecord(ev.last, s));
     GCG_CUDA(cudaMemcpyAsync(h_ctl, ctl.get(), sizeof(h_ctl), cudaMemcpyDeviceToHost, s));
     GCG_CUDA(cudaStreamSynchronize(s));
     if (h_ctl[3]) return fail(GCG_ERR_TIMEOUT, "pagerank: a wait between the levels of a sweep ran out");
@@ -979,9 +984,7 @@ int pagerank_gs_exact(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
         GCG_LAUNCH_CHECK();
     }
     float ms = 0.0f;
-    cudaEventElapsedTime(&ms, ev0, ev1);
-    cudaEventDestroy(ev0);
-    cudaEventDestroy(ev1);
+    cudaEventElapsedTime(&ms, ev.first, ev.last);
     double last_res = 0.0;
     if (track && sweeps > 0)
         GCG_CUDA(cudaMemcpy(&last_res, logs.get() + std::max(1, nsw) + sweeps - 1, sizeof(double),

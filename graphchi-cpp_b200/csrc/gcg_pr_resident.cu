@@ -72,6 +72,7 @@ struct ResArgs {
     const float *init_rank;
     float *out;       /* result by vertex id, or null */
     ResStatus *status; /* pinned host memory */
+    long long spin_limit; /* polls of a wait */
     uint32_t max_sweeps;
 };
 
@@ -161,7 +162,7 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
 __device__ __forceinline__ bool wait_reach(const ResArgs &m, const uint32_t *p, uint32_t target) {
     for (long long spins = 0; (int32_t)(ld_acq(p) - target) < 0; ++spins) {
         if ((spins & 255) == 255 && *(volatile int *)m.err) return false;
-        if (spins > RES_SPIN) {
+        if (spins > m.spin_limit) {
             atomicExch(m.err, 1);
             m.status->err = 1;
             __threadfence_system();
@@ -525,6 +526,11 @@ int pagerank_resident(gcg_graph *g, const gcg_pr_params *p, float *out_rank, gcg
     memset(w.h_flags, 0, sizeof(ResStatus));
 
     GCG_CUDA(cudaMemsetAsync(w.res_ctl.get(), 0, (2 + (size_t)w.res_ctas) * 4, s));
+    m.spin_limit = RES_SPIN;
+    if (p->flags & GCG_PR_TEST_BARRIER_TIMEOUT) { /* one arrival short */
+        m.spin_limit = GCG_TEST_SPIN;
+        GCG_CUDA(cudaMemsetAsync(m.bar, 0xFF, 4, s));
+    }
     GCG_CUDA(cudaEventRecord(w.ev[0], s));
     void *kargs[] = {&m};
     const cudaError_t launched = cudaLaunchCooperativeKernel(

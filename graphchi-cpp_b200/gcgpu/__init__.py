@@ -318,7 +318,7 @@ class Graph:
 
     def pagerank(self, mode=PR_JACOBI, max_sweeps=3, teleport=0.15, damping=0.85, tol=0.0, init=1.0,
                  init_rank=None, out=None, residuals=None, time_sweeps=False, source=None, delta_log=None,
-                 work_log=None, delta_threshold=0.0):
+                 work_log=None, delta_threshold=0.0, flags=0):
         """Returns (ranks, PrStats). out/init_rank/residuals/delta_log/work_log: numpy or device tensors."""
         p = PrParams()
         _pr_default(C.byref(p))
@@ -329,7 +329,7 @@ class Graph:
             p.delta_log = ptr(delta_log)
         if work_log is not None:
             p.work_log = ptr(work_log)
-        p.flags = PR_TIME_SWEEPS if time_sweeps else 0
+        p.flags = flags | (PR_TIME_SWEEPS if time_sweeps else 0)
         p.source = NO_SOURCE if source is None else int(source)
         if init_rank is not None:
             init_rank = init_rank if not isinstance(init_rank, np.ndarray) else \

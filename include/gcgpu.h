@@ -204,9 +204,11 @@ typedef struct {
 } gcg_pr_params;
 
 #define GCG_PR_TIME_SWEEPS 0x1u
-/* Test hook of gcg_batch_pagerank: the persistent kernel's grid barrier waits for
- * one CTA that does not exist, so its bounded wait runs out and the call returns
- * GCG_ERR_TIMEOUT (exercises the failure path without faulting the GPU). */
+/* Test hook of gcg_batch_pagerank, and of gcg_pagerank where it runs as cooperative
+ * launches (the one-launch Jacobi solve, the GS modes with more than one level): the
+ * kernel's grid barrier waits for one CTA that does not exist, so its bounded wait runs
+ * out and the call returns GCG_ERR_TIMEOUT (exercises the failure path without faulting
+ * the GPU). */
 #define GCG_PR_TEST_BARRIER_TIMEOUT 0x2u
 #define GCG_NO_SOURCE 0xFFFFFFFFu
 
