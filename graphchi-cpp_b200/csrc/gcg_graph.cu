@@ -627,7 +627,8 @@ int build_graph(const uint32_t *src_u, const uint32_t *dst_u, uint64_t m, uint32
             if (cudaGetLastError() != cudaSuccess) return cleanup(fail(GCG_ERR_CUDA, "k_make_keys launch"));
             const int cut = runs_of_src ? half.npass : pl.npass;
             uint64_t *by_src = nullptr;
-            st = radix_passes(keys.get(), tmp.get(), nk, pl, 0, cut, counts.get(), &by_src, s);
+            const bool recount = (flags & GCG_BUILD_TEST_RECOUNT) != 0;
+            st = radix_passes(keys.get(), tmp.get(), nk, pl, 0, cut, counts.get(), &by_src, s, recount);
             if (st) return cleanup(st);
             sorted = by_src;
             if (runs_of_src) {
@@ -636,7 +637,7 @@ int build_graph(const uint32_t *src_u, const uint32_t *dst_u, uint64_t m, uint32
                 if (cudaGetLastError() != cudaSuccess) return cleanup(fail(GCG_ERR_CUDA, "k_src_runs launch"));
                 outdeg_raw = g->outdeg.get();
                 st = radix_passes(by_src, by_src == keys.get() ? tmp.get() : keys.get(), nk, pl, cut, pl.npass,
-                                  counts.get(), &sorted, s);
+                                  counts.get(), &sorted, s, recount);
                 if (st) return cleanup(st);
             }
             runs.p[0] = sorted;

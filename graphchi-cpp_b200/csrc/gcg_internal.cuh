@@ -202,9 +202,9 @@ struct RadixPlan {
 RadixPlan radix_plan(int begin_bit, int end_bit);
 
 /* A sort's passes [first, last) alone, given the digit counts [pass][256] of all
- * of the plan's passes (device). */
+ * of the plan's passes (device). recount: no tile takes another's word for its counts. */
 int radix_passes(uint64_t *keys, uint64_t *tmp, uint64_t n, const RadixPlan &pl, int first, int last,
-                 const uint32_t *counts, uint64_t **result, cudaStream_t s);
+                 const uint32_t *counts, uint64_t **result, cudaStream_t s, bool recount = false);
 
 #ifdef __CUDACC__
 /* Digit counts of a block's keys in shared memory, one set per half block. */

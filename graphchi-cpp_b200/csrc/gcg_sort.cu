@@ -27,7 +27,8 @@ constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
 constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_RADIX = 256;
 constexpr int RS_PASSES = RadixPlan::MAX_PASSES;
-constexpr int RS_SPIN = 1 << 14; /* polls of one tile's count before it is counted again */
+constexpr int RS_SPIN = 1 << 14;   /* polls of one tile's count before it is counted again */
+constexpr int RS_RECOUNT = -1;     /* in their place: every count is taken again (a test's) */
 constexpr int RS_GROUP = 16;     /* tiles that share a group word */
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
@@ -81,6 +82,7 @@ struct RsPass {
     uint64_t n;
     int shift, bits;
     uint32_t tag; /* pass number * 4, from 4 */
+    int spin;     /* RS_SPIN or RS_RECOUNT */
     const uint32_t *counts;
     uint32_t *ticket;
     unsigned long long *tile;  /* [tile][digit]: keys of the digit in the tile, or up to its end */
@@ -228,8 +230,8 @@ __global__ void __launch_bounds__(RS_THREADS, RS_BLOCKS) rs_pass(RsPass a) {
         const uint32_t g = t / RS_GROUP, in_g = t % RS_GROUP, pass = a.tag >> 2;
         /* a word, waited for, or else what it would hold; true: it reaches back to the start */
         auto take = [&](const unsigned long long *p, unsigned long long w, uint64_t lo, uint64_t hi) {
-            for (int spin = 0; (uint32_t)(w >> 34) != pass && spin < RS_SPIN; ++spin) w = st_get(p);
-            if ((uint32_t)(w >> 34) == pass) {
+            for (int spin = 0; (uint32_t)(w >> 34) != pass && spin < a.spin; ++spin) w = st_get(p);
+            if ((uint32_t)(w >> 34) == pass && a.spin >= 0) {
                 excl += (uint32_t)w;
                 return (uint32_t)(w >> 32) == (a.tag | ST_INC);
             }
@@ -820,7 +822,7 @@ RadixPlan radix_plan(int begin_bit, int end_bit) {
 }
 
 int radix_passes(uint64_t *keys, uint64_t *tmp, uint64_t n, const RadixPlan &pl, int first, int last,
-                 const uint32_t *counts, uint64_t **result, cudaStream_t s) {
+                 const uint32_t *counts, uint64_t **result, cudaStream_t s, bool recount) {
     *result = keys;
     if (n <= 1 || first >= last) return GCG_OK;
     if (n > 0xFFFFFFFFull) return fail(GCG_ERR_UNSUPPORTED, "radix sort: more than 2^32-1 keys");
@@ -839,6 +841,7 @@ int radix_passes(uint64_t *keys, uint64_t *tmp, uint64_t n, const RadixPlan &pl,
         ps.shift = pl.shift[p];
         ps.bits = pl.bits[p];
         ps.tag = (uint32_t)(p + 1) << 2;
+        ps.spin = recount ? RS_RECOUNT : RS_SPIN;
         ps.counts = counts + p * RS_RADIX;
         ps.ticket = reinterpret_cast<uint32_t *>(work.get() + nwords + p);
         ps.tile = work.get();

@@ -32,6 +32,7 @@ STATUS_NAMES = {0: "GCG_OK", -1: "GCG_ERR_INVALID", -2: "GCG_ERR_CUDA", -3: "GCG
 BUILD_DEDUP = 0x1
 BUILD_SYMMETRISE = 0x2
 BUILD_NO_OUT_CSR = 0x4
+BUILD_TEST_RECOUNT = 0x100
 CSR_IN = 0
 CSR_OUT = 1
 PR_JACOBI = 0

@@ -44,6 +44,9 @@ typedef struct gcg_graph gcg_graph;
 #define GCG_BUILD_DEDUP 0x1u      /* keep one copy of repeated (src,dst) */
 #define GCG_BUILD_SYMMETRISE 0x2u /* add (dst,src) for every (src,dst) before dedup */
 #define GCG_BUILD_NO_OUT_CSR 0x4u /* skip the src-grouped (out-edge) CSR */
+/* Test hook: the radix sort of a device edge list counts again what it otherwise takes from
+ * the tiles before (its way out when such a count does not come); the graph is the same. */
+#define GCG_BUILD_TEST_RECOUNT 0x100u
 
 /* Replaces sharder<ET>::preprocessing_add_edge + execute_sharding
  * (src/preprocessing/sharder.hpp:427-446, :535-548, :861-1008) for an edge list
