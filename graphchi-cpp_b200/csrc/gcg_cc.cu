@@ -231,13 +231,24 @@ __global__ void __launch_bounds__(256) k_cc_second(Nbrs n, uint32_t nv, const ui
 /* The most frequent root among 1024 sampled vertices (ties: the smaller id), by one block
  * of 256 threads once every parent is a root: counted in a hash table in shared memory of
  * twice as many slots, the equal roots of a warp at once. cnt[1] = that root, cnt[2] =
- * fewer than half of the sampled vertices that hang below some root hang below it. */
+ * fewer than half of the sampled vertices that hang below some root hang below it. With the
+ * lists given (n.rin) cnt[2] also wants those of them that have neighbours to have more than
+ * CC_GIANT / 8 on average: of fewer (1.58 in a uniform graph of one neighbour a vertex) no
+ * giant component is made that a second round could find (uniform, 1 M vertices with 512 K
+ * edges: 135 us with the round, 123 without; a core of 130,000 vertices with 1 M edges among
+ * 4 M keeps it: 164 us, without 722). */
+constexpr int CC_GIANT = 13;
+__device__ __noinline__ int cc_dense(const Nbrs &n, uint32_t x) {
+    const uint32_t d = nbr_count(n, x);
+    return d ? 8 * (int)min(d, 4096u) - CC_GIANT : 0;
+}
 constexpr uint32_t CC_SLOTS = 2048;
 static_assert(CC_SLOTS == 1u << 11, "the hash's shift");
-__device__ void cc_sample(const uint32_t *parent, uint32_t nv, uint32_t *cnt) {
+__device__ void cc_sample(const Nbrs &n, const uint32_t *parent, uint32_t nv, uint32_t *cnt) {
     __shared__ uint32_t s_key[CC_SLOTS], s_cnt[CC_SLOTS];
     __shared__ unsigned long long s_best;
     __shared__ uint32_t s_below;
+    __shared__ int s_dense;
     const uint32_t t = threadIdx.x;
     for (uint32_t k = t; k < CC_SLOTS; k += 256u) {
         s_key[k] = GCG_NO_SOURCE; /* no vertex */
@@ -246,6 +257,7 @@ __device__ void cc_sample(const uint32_t *parent, uint32_t nv, uint32_t *cnt) {
     if (t == 0) {
         s_best = ~0ull;
         s_below = 0u;
+        s_dense = n.rin ? 0 : 1;
     }
     uint32_t x[4], r[4];
 #pragma unroll
@@ -274,6 +286,7 @@ __device__ void cc_sample(const uint32_t *parent, uint32_t nv, uint32_t *cnt) {
         }
         const uint32_t nb = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, r[q] != x[q]));
         if ((t & 31u) == 0u) atomicAdd(&s_below, nb);
+        if (n.rin) atomicAdd(&s_dense, cc_dense(n, x[q]));
     }
     __syncthreads();
     for (uint32_t k = t; k < CC_SLOTS; k += 256u)
@@ -281,7 +294,7 @@ __device__ void cc_sample(const uint32_t *parent, uint32_t nv, uint32_t *cnt) {
     __syncthreads();
     if (t == 0) {
         cnt[1] = (uint32_t)(s_best & 0xFFFFFFFFull);
-        cnt[2] = 2u * (1024u - (uint32_t)(s_best >> 32)) < s_below;
+        cnt[2] = 2u * (1024u - (uint32_t)(s_best >> 32)) < s_below && s_dense > 0;
     }
 }
 
@@ -357,7 +370,8 @@ __global__ void __launch_bounds__(256) k_cc_rest(Nbrs n, uint32_t nv, const uint
  * R-MAT scale 24). AGAIN: the same after the second round, if there
  * was one. The last block to finish takes the sample. */
 template <bool SAMPLE, bool AGAIN>
-__global__ void __launch_bounds__(256) k_cc_compress(uint32_t nv, uint32_t *parent, uint32_t *cnt) {
+__global__ void __launch_bounds__(256) k_cc_compress(const __grid_constant__ Nbrs n, uint32_t nv, uint32_t *parent,
+                                                     uint32_t *cnt) {
     if (AGAIN && cnt[2] == 0u) return;
     uint32_t roots = 0;
     const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
@@ -393,7 +407,7 @@ __global__ void __launch_bounds__(256) k_cc_compress(uint32_t nv, uint32_t *pare
         if (!s_last) return;
         __threadfence();
         if (threadIdx.x == 0) cnt[3] = 0u;
-        cc_sample(parent, nv, cnt);
+        cc_sample(n, parent, nv, cnt);
     } else {
         __shared__ uint32_t s_roots[8];
 #pragma unroll
@@ -448,9 +462,11 @@ extern "C" int gcg_connected_components(gcg_graph *g, uint32_t *labels, gcg_cc_s
         nb.cout = g->symmetric ? nullptr : g->out_col.get();
         k_cc_first<<<vb, 256, 0, s>>>(nb, nv, parent, minima.get(), cnt.get());
         k_cc_minima<<<vb, 256, 0, s>>>(nb, nv, minima.get(), parent);
-        k_cc_compress<true, false><<<vb, 256, 0, s>>>(nv, parent, cnt.get());
+        /* fewer neighbours than vertices: the sample looks whether those that have any have enough */
+        const Nbrs lists = (g->symmetric ? 1u : 2u) * g->ne > nv ? Nbrs{} : nb;
+        k_cc_compress<true, false><<<vb, 256, 0, s>>>(lists, nv, parent, cnt.get());
         k_cc_second<<<vb, 256, 0, s>>>(nb, nv, cnt.get(), parent);
-        k_cc_compress<true, true><<<vb, 256, 0, s>>>(nv, parent, cnt.get());
+        k_cc_compress<true, true><<<vb, 256, 0, s>>>(Nbrs{}, nv, parent, cnt.get());
         k_cc_rest<<<vb, 256, 0, s>>>(nb, nv, cnt.get(), parent);
     } else {
         const PrPlan &pl = *g->plan;
@@ -464,7 +480,7 @@ extern "C" int gcg_connected_components(gcg_graph *g, uint32_t *labels, gcg_cc_s
         k_cc_hook<<<tb, MP_THREADS, 0, s>>>(g->in_rowptr.get(), g->in_col.get(), pl.tile_row.get(),
                                            pl.tile_edge.get(), pl.ntiles, parent);
     }
-    k_cc_compress<false, false><<<vb, 256, 0, s>>>(nv, parent, cnt.get());
+    k_cc_compress<false, false><<<vb, 256, 0, s>>>(Nbrs{}, nv, parent, cnt.get());
     GCG_LAUNCH_CHECK();
     GCG_CUDA(cudaEventRecord(ev1, s));
     uint32_t nroots = 0;
