@@ -10,9 +10,11 @@
  * gcg_batch_pagerank runs every sweep of every graph inside ONE cooperative
  * persistent kernel (one 1024-thread CTA per SM). Per sweep, four phases split by
  * a grid barrier:
- *   A  edges: warps stride over the 256-edge chunks of the still-active graphs
- *      (their concatenated chunk ranges; equal-sized chunks need no queue) and run
- *      the same pipelined gather / warp reduction as the single-graph kernel;
+ *   A  edges: CTAs take ranges of the still-active graphs' concatenated 256-edge
+ *      chunks from a device cursor, large ones first, and their warps stride over
+ *      them with the same pipelined gather / warp reduction as the single-graph
+ *      kernel (one hub over the union: warps stride over all chunks, or take runs
+ *      from the queue);
  *   B  rows crossing chunks: partials added in chunk order;
  *   C  vertices: every warp takes an even, contiguous share of the active graphs'
  *      tiles of 128 rows (4 rows per thread), applies them, and writes one FP64 residual

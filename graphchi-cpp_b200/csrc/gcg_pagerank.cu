@@ -11,10 +11,10 @@
  *                two 128-bit column loads per lane (streamed: no L1 allocation,
  *                L2 evict-first), eight independent gathers of contrib[src]
  *                (L2 evict-last, so the contrib vector stays resident while the
- *                columns stream past), row starts read from a word per lane, in-lane segment sums, and a warp segmented scan
- *                (shuffles) to join rows across lanes. Rows inside the chunk get
- *                their sum written; a row crossing chunk boundaries leaves one
- *                partial per chunk.
+ *                columns stream past), row starts read from a word per lane,
+ *                in-lane segment sums, and a warp segmented scan (shuffles) to join
+ *                rows across lanes. Rows inside the chunk get their sum written; a
+ *                row crossing chunk boundaries leaves one partial per chunk.
  *   k_pr_fix     rows that cross chunks: partials added in chunk order.
  *   k_pr_vertex  apply for every vertex with in-edges:
  *                r' = (float)(teleport + damping*(double)sum), c' = r'/outdeg

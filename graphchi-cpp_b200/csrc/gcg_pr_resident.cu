@@ -420,12 +420,12 @@ __global__ void __launch_bounds__(EDGE_THREADS, 1) k_pr_resident(ResArgs m) {
 
 }  // namespace
 
-/* Where the line lies (solves to 1e-8, one B200, this launch against the queued
- * kernels): 1.0 M edges 0.65 against 1.41 ms (3 sweeps: 54 against 110 us), 2.4 M
- * uniform 1.19 against 2.16, 4.2 M 1.44 against 2.26, 16 M 4.00 against 5.32, 33 M
- * 7.65 against 8.20, 67 M 16.7 against 13.8: there the CTAs' fixed ranges, cut by
- * edges and rows alone, are less even than chunks dealt one by one, and the scattered
- * gathers want the texture path. Explicit launch configurations, source tiers and
+/* Where the line lies (host time of solves to 1e-8, this launch against the queued
+ * kernels): 1.0 M edges 0.63 against 1.43 ms (3 sweeps: 60 against 125 us), 2.4 M
+ * uniform 1.06 against 2.08, R-MAT of 3.9 M 1.13 against 2.16, 16 M 3.07 against 4.62,
+ * 32 M 6.31 against 6.89; 67 M, with the limit lifted, 16.7 against 13.8: there the
+ * CTAs' fixed ranges, cut by edges and rows alone, are less even than chunks dealt one
+ * by one, and the scattered gathers want the texture path. Explicit launch configurations, source tiers and
  * per-sweep timing belong to the queued kernels. */
 bool resident_applies(const gcg_graph *g, const gcg_pr_params *p) {
     const ChunkPlan &pl = *g->cplan;

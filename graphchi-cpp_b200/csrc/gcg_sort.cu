@@ -17,9 +17,8 @@ namespace gcg {
 
 namespace {
 
-/* 256 threads x 22 keys, three blocks on an SM. 67 M keys build in 3.16 ms; 4
- * blocks of 256 x 16 or 2 of 512 x 16 take 3.26: shorter runs, or fewer phases that
- * overlap. */
+/* 256 threads x 22 keys, three blocks on an SM: 3 % faster over a build of 67 M edges than 4
+ * blocks of 256 x 16 or 2 of 512 x 16 (shorter runs, or fewer phases that overlap). */
 constexpr int RS_THREADS = 256;
 constexpr int RS_ITEMS = 22;
 constexpr int RS_BLOCKS = 3;

@@ -243,15 +243,15 @@ __global__ void __launch_bounds__(1024, 1) k_tc_group(const uint64_t *__restrict
         }
         return;
     } else {
-    for (uint32_t r = threadIdx.x; r < top; r += blockDim.x) { /* where this block's part of each list begins */
-        const uint32_t c = mine[r];
-        if (c) s_cnt[r] = atomicAdd(at + (nv - 1u - r), c);
-    }
-    __syncthreads();
-    each([&](uint32_t j, uint32_t a, uint32_t b) {
-        const uint32_t r = nv - 1u - b;
-        rev[r < top ? atomicAdd(s_cnt + r, 1u) : atomicAdd(at + b, 1u)] = make_uint2(j, a);
-    });
+        for (uint32_t r = threadIdx.x; r < top; r += blockDim.x) { /* where this block's part of each list begins */
+            const uint32_t c = mine[r];
+            if (c) s_cnt[r] = atomicAdd(at + (nv - 1u - r), c);
+        }
+        __syncthreads();
+        each([&](uint32_t j, uint32_t a, uint32_t b) {
+            const uint32_t r = nv - 1u - b;
+            rev[r < top ? atomicAdd(s_cnt + r, 1u) : atomicAdd(at + b, 1u)] = make_uint2(j, a);
+        });
     }
 }
 

@@ -75,8 +75,8 @@ __host__ __device__ __forceinline__ uint32_t bf16_bits(float x_rounded) {
 /* ---- features ------------------------------------------------------------ */
 
 /* The in-neighbourhood aggregates run on the PageRank chunk plan: 256-edge warp
- * chunks over the in-CSR with sources relabelled by out-degree, head bits for
- * row starts, split rows completed in chunk order. Each edge contributes
+ * chunks over the in-CSR with sources relabelled by out-degree, the plan's words
+ * per lane for row starts, split rows completed in chunk order. Each edge contributes
  * {L(u), L(u), indeg(u)} to its row's (sum, max, sum). */
 struct AggArgs {
     const uint32_t *col; /* relabelled sources */
@@ -664,10 +664,10 @@ __device__ __forceinline__ void tile_gemm(float (&acc)[8][4], const float *pa, c
  * (4 sg .. and 64 + 4 sg ..) x 4 features (4 fg ..) of the activations, and 4 x 4 of dW2
  * (rows gj + 16 i, columns gk + 16 i), which stay in registers for four tiles;
  * biases and W3 are added up from the activations where they arise. 1 M samples take
- * 0.72 ms (13.3 k FMAs a sample: 0.37 ms at the FP32 rate); what bounds it is shared
- * memory, 3.0 k quarter-warp reads per warp and tile against 1.6 k FMA cycles. With a
- * thread per sample and one block of 128 threads per SM, a warp per scheduler, they took
- * 2.64 ms. */
+ * 0.75 ms (13.3 k FMAs a sample: 0.37 ms at the FP32 rate), the whole call 0.79; what
+ * bounds it is shared memory, 3.0 k quarter-warp reads per warp and tile against 1.6 k FMA
+ * cycles (84 % of its rate). With a thread per sample and one block of 128 threads per SM,
+ * a warp per scheduler, the call took 2.69 ms. */
 template <bool FWD_ONLY>
 __global__ void __launch_bounds__(TRAIN_THREADS, 2) k_mlp_fwd_bwd(TrainArgs a) {
     extern __shared__ __align__(16) float sm[];
@@ -704,8 +704,9 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 2) k_mlp_fwd_bwd(TrainArgs a) {
 
     /* The weights' sums go to the block's slot every FLUSH_TILES tiles: a float sum over all
      * of a block's samples (3.4 k of 1 M) loses more than its parts do. With the blocks'
-     * slots added in FP64 the gradient over 1 M samples is 5e-8 off 64-bit arithmetic, as
-     * one float chain 1.8e-7 to 3.2e-7; the call takes 0.786 ms in place of 0.764. */
+     * slots added in FP64 the gradient over 1 M samples is 3e-8 off 64-bit arithmetic, as
+     * one float chain 1.8e-7 to 3.2e-7 (where no sample falls on the other side of a ReLU: one
+     * that does makes up to 5e-7); the call takes 0.79 ms in place of 0.76. */
     constexpr uint32_t FLUSH_TILES = 4;
     float *out = FWD_ONLY ? nullptr : a.part + (size_t)blockIdx.x * (NP + 1);
     uint32_t since = 0;

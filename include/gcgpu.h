@@ -306,8 +306,9 @@ int gcg_batch_create(gcg_graph *const *graphs, uint32_t ngraphs, gcg_batch **out
  * hottest sources, rows kept in id order) instead of within each graph's id
  * range (a hub per graph, rows in relabelled order; the default, and the only
  * layout whose ranks are bit-identical to each graph's own gcg_pagerank solve).
- * Without the flag the one-hub layout is taken only when the union's ids are too
- * wide for per-graph relabelling (more than 64 sort-key bits). */
+ * Without the flag the one-hub layout is taken only for a batch of one graph, and
+ * when the union's ids are too wide for per-graph relabelling (more than 64
+ * sort-key bits). */
 #define GCG_BATCH_ONE_HUB 1u
 int gcg_batch_create_ex(gcg_graph *const *graphs, uint32_t ngraphs, uint32_t flags, gcg_batch **out);
 /* First union vertex id of each graph (ngraphs+1 entries, last = total). */
